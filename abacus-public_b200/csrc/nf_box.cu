@@ -936,9 +936,9 @@ static KParams params_from(nf_ctx *ctx, const EngineLaunch &L) {
         double ie2 = (double)eps;  // eps_int^-2
         kp.pc.near_thr = (float)(1.0 / ie2);
         kp.pc.inv_eps3 = (float)pow(ie2, 1.5);
-        kp.pc.c1 = (float)(-15.0 * ie2 * ie2);
-        kp.pc.c2 = (float)(6.0 * pow(ie2, 2.5));
-        kp.pc.c3 = (float)(10.0 * pow(ie2, 1.5));
+        kp.pc.c1 = (float)(-15.0 * ie2 * ie2 * NEWTON_UNIT);
+        kp.pc.c2 = (float)(6.0 * pow(ie2, 2.5) * NEWTON_UNIT);
+        kp.pc.c3 = (float)(10.0 * pow(ie2, 1.5) * NEWTON_UNIT);
     }
     {
         // margin of the near test: eps (+1% and a rounding allowance)
@@ -974,12 +974,14 @@ static KParams make_params(nf_ctx *ctx, nf_box *box, const Plan &pl) {
 }
 
 // Output scale of the co-add, formed in double on the host and rounded once
-// to float (single spline: eps_int^3, the raw kernel's units; otherwise 1).
+// to float: out of the pair sums' unit, and for the single spline times
+// eps_int^3 (the raw kernel's units).
 // eps: the softening parameter in use (0: the context's).
 static float output_scale(const nf_config &cfg, float eps = 0.f) {
     if (eps <= 0.f) eps = cfg.eps;
-    if (cfg.softening == SOFT_SINGLE_SPLINE) return (float)pow((double)eps, -1.5);  // eps_int^3
-    return 1.0f;
+    const double eps3 =
+        cfg.softening == SOFT_SINGLE_SPLINE ? pow((double)eps, -1.5) : 1.0;  // eps_int^3
+    return (float)(eps3 / pair_unit(cfg.softening));
 }
 
 int engine_variant_smax(int variant) { return VARIANTS[variant].smax; }
