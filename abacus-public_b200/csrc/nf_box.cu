@@ -1,5 +1,9 @@
 // nf_box.cu -- batched near-field form: positions resident in HBM, one
-// persistent launch per slab range, deterministic co-add.
+// persistent launch per slab range, deterministic co-add; and the one-sided
+// pencil engine.  Boxes are swept by the mutual engine (nf_mutual.cu) except
+// with plain accumulation or a softening below its fixed-point range; the
+// one-sided engine below serves those, the plain drop-in and the
+// allocation-free entry point.
 //
 // Work decomposition (the reference's pencil-on-pencil scheme,
 // singlestep/Direct/SetInteractionCollection.hh:4-35 and
@@ -162,8 +166,8 @@ __device__ __forceinline__ float4 load_src(const KParams &kp, const WarpSmem &ws
 
 // One staged chunk (m_pad sources, a multiple of UNR) against the lane's
 // sinks, accumulated straight into the running partials.  Separations are
-// taken sink - source, so a += g * d.  NEAR selects the both-branch single
-// spline evaluation.  Scalar form: one sink per lane.
+// taken sink - source, so a += g * d.  NEAR selects the splines' full
+// formula.  Scalar form: one sink per lane.
 template <int SOFT, bool DENS, bool NEAR, int UNR>
 __device__ __forceinline__ void chunk_scalar(const float4 *bxy, const float2 *bz, int m_pad,
                                              float sx, float sy, float sz, float &px, float &py,
@@ -175,13 +179,8 @@ __device__ __forceinline__ void chunk_scalar(const float4 *bxy, const float2 *bz
             float4 t = bxy[j + u];
             float tz = bz[j + u].x;
             float dx = sx + t.x, dy = sy + t.z, dz = sz + tz;
-            float g;
-            if (NEAR) {
-                g = spline_g_both(dx, dy, dz, pc);
-            } else {
-                float r2;
-                g = pair_g_fast<SOFT>(dx, dy, dz, pc, r2);
-            }
+            const float r2 = fmaf(dz, dz, fmaf(dy, dy, fmaf(dx, dx, r2_add<SOFT>(pc))));
+            const float g = pair_g<SOFT, NEAR>(r2, pc);
             px = fmaf(g, dx, px);
             py = fmaf(g, dy, py);
             pz = fmaf(g, dz, pz);
@@ -207,15 +206,7 @@ __device__ __forceinline__ void chunk_paired(const float4 *bxy, const float2 *bz
 #pragma unroll
             for (int q = 0; q < SP; q++) {
                 float2 dx = add2(sx[q], tx), dy = add2(sy[q], ty), dz = add2(sz[q], tz);
-                float2 g;
-                if (SOFT == SOFT_PLUMMER || SOFT == SOFT_SINGLE_SPLINE) {
-                    float2 r2 = r2_x2(dx, dy, dz, SOFT == SOFT_PLUMMER ? pc.eps : 1e-25f);
-                    g = NEAR ? spline_g_both_x2(r2, pc) : inv_r3_x2(r2);
-                } else {  // the cubic kernels: component-wise scalar evaluation
-                    float r2;
-                    g.x = pair_g_fast<SOFT>(dx.x, dy.x, dz.x, pc, r2);
-                    g.y = pair_g_fast<SOFT>(dx.y, dy.y, dz.y, pc, r2);
-                }
+                const float2 g = pair_g_x2<SOFT, NEAR>(r2_x2(dx, dy, dz, r2_add<SOFT>(pc)), pc);
                 px[q] = fma2(g, dx, px[q]);
                 py[q] = fma2(g, dy, py[q]);
                 pz[q] = fma2(g, dz, pz[q]);
@@ -247,38 +238,6 @@ __device__ __forceinline__ int64_t sink_particle(const WarpSmem &ws, int i, int 
     a = 0;
     while (i >= ws.spre[a + 1]) a++;
     return ws.sstart[a] + (i - ws.spre[a]);
-}
-
-// Fold a partial p into the running compensated sum (h, l) and clear it
-// (plain: one FP32 running sum).  Kahan's compensated summation with the
-// correction kept as the low part to add (the sum is h + l):
-//   y = p + l;  t = h + y;  l = y - (t - h);  h = t
-// four paired instructions per component and sink pair.  Scalar and paired
-// (two sinks) forms; a - b is formed as fma(b, -1, a), which rounds exactly
-// like a subtraction.
-__device__ __forceinline__ void fold1(float &h, float &l, float &p, bool plain) {
-    if (plain) {
-        h += p;
-    } else {
-        float y = p + l;
-        float t = h + y;
-        l = y - (t - h);
-        h = t;
-    }
-    p = 0.f;
-}
-
-__device__ __forceinline__ void fold2(float2 &h, float2 &l, float2 &p, bool plain) {
-    if (plain) {
-        h = add2(h, p);
-    } else {
-        const float2 m1 = dup2(-1.0f);
-        float2 y = add2(p, l);
-        float2 t = add2(h, y);
-        l = fma2(fma2(h, m1, t), m1, y);  // y - (t - h)
-        h = t;
-    }
-    p = make_float2(0.f, 0.f);
 }
 
 // FP32 partials are folded into the compensated (h, l) sums every FOLD_CHUNKS chunks.
@@ -319,7 +278,7 @@ __device__ void run_tile(const KParams &kp, WarpSmem &ws, const Item &it, int la
         px[q] = py[q] = pz[q] = pw[q] = make_float2(0.f, 0.f);
         hx[q] = hy[q] = hz[q] = lx[q] = ly[q] = lz[q] = make_float2(0.f, 0.f);
     }
-    constexpr bool FLAG = SOFT == SOFT_SINGLE_SPLINE;
+    constexpr bool FLAG = has_near(SOFT);
     const bool plain = kp.plain;
     // the tile's sink bounding box (pencil frame), widened by eps: sources
     // outside it cannot be near any of the tile's sinks
@@ -504,33 +463,53 @@ __global__ void __launch_bounds__(WARPS_PER_CTA * 32, MINB) pencil_kernel(KParam
     }
 }
 
-// Sum the 2R+1 pencil partials of every particle in a fixed order, apply the
-// output scale (single spline: eps^3) and write accstruct records.
+// Where a sweep left the sums of the particles of a range: pencil partials
+// (one-sided) or fixed point (mutual, acc != nullptr).
+struct SumsView {
+    const Partial *__restrict__ part;
+    const unsigned long long *__restrict__ acc;
+    const unsigned char *__restrict__ bad;
+    int64_t n;
+    int W, nc;
+    float scale;   // of x, y, z (mutual: out of the fixed-point unit as well)
+    float wscale;  // of w (mutual)
+};
+
+// The sums of particle p of the range.  One-sided: its 2R+1 partials summed
+// in compensated FP32 in pencil-slot order; x, y, z times the output scale
+// (one rounding: the correction is scaled and added inside the FMA), w
+// unscaled.
+__device__ __forceinline__ void coadd_sink(const SumsView &v, int64_t p, float r[4]) {
+    if (v.acc) {
+        const bool bad = v.bad[p];
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            r[c] = 0.f;
+            if (c < v.nc) r[c] = __ll2float_rn((long long)v.acc[c * v.n + p]) * (c < 3 ? v.scale : v.wscale);
+            if (bad && c < 3) r[c] = __int_as_float(0x7fffffff);
+        }
+        return;
+    }
+    float s[4] = {0.f, 0.f, 0.f, 0.f}, e[4] = {0.f, 0.f, 0.f, 0.f};
+    for (int a = 0; a < v.W; a++)
+#pragma unroll
+        for (int c = 0; c < 4; c++)
+            if (c < v.nc) add_partial(s[c], e[c], v.part[((int64_t)a * v.nc + c) * v.n + p]);
+#pragma unroll
+    for (int c = 0; c < 3; c++) r[c] = fmaf(s[c], v.scale, e[c] * v.scale);
+    r[3] = v.nc == 4 ? s[3] + e[3] : 0.f;
+}
+
+// The record of every particle of a range, as accstruct.
 // perm (optional): the caller's particle index of each packed slot; the
 // record of slot p0 + p goes to perm[p0 + p] - p0 (a permutation of the
 // range, since the in-cell ordering never moves a particle out of its cell).
-// The 2R+1 partials of particle p of the range, summed in compensated FP32
-// in pencil-slot order; x, y, z times the output scale (one rounding: the
-// correction is scaled and added inside the FMA), w unscaled.
-__device__ __forceinline__ void coadd_sink(const Partial *__restrict__ part, int64_t n, int W,
-                                           int nc, int64_t p, float scale, float r[4]) {
-    float s[4] = {0.f, 0.f, 0.f, 0.f}, e[4] = {0.f, 0.f, 0.f, 0.f};
-    for (int a = 0; a < W; a++)
-#pragma unroll
-        for (int c = 0; c < 4; c++)
-            if (c < nc) add_partial(s[c], e[c], part[((int64_t)a * nc + c) * n + p]);
-#pragma unroll
-    for (int c = 0; c < 3; c++) r[c] = fmaf(s[c], scale, e[c] * scale);
-    r[3] = nc == 4 ? s[3] + e[3] : 0.f;
-}
-
-__global__ void coadd_kernel(const Partial *__restrict__ part, int64_t n, int W, int nc,
-                             float scale, int out_kind, void *out,
+__global__ void coadd_kernel(SumsView v, int out_kind, void *out,
                              const uint32_t *__restrict__ perm, int64_t p0) {
     int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < n; p += stride) {
+    for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < v.n; p += stride) {
         float r[4];
-        coadd_sink(part, n, W, nc, p, scale, r);
+        coadd_sink(v, p, r);
         const float x = r[0], y = r[1], z = r[2];
         const int64_t o_i = perm ? (int64_t)perm[p0 + p] - p0 : p;
         if (out_kind == NF_OUT_FLOAT4) {
@@ -621,8 +600,7 @@ struct KickConst {
     float near_scale, rescale, kick1, kick2, b2;
 };
 
-__global__ void kick_kernel(const Partial *__restrict__ part, int64_t n, int W, int nc,
-                            float scale, const int64_t *__restrict__ cs, int64_t c0,
+__global__ void kick_kernel(SumsView v, const int64_t *__restrict__ cs, int64_t c0,
                             int64_t ncells, int64_t p0, const uint32_t *__restrict__ perm,
                             KickConst k, const float *__restrict__ far, float *vel, void *acc_out,
                             int out_kind, float *stats) {
@@ -635,7 +613,7 @@ __global__ void kick_kernel(const Partial *__restrict__ part, int64_t n, int W, 
         for (int64_t slot = s0 + lane; slot < s1; slot += 32) {
             const int64_t i = slot - p0;
             float r[4];
-            coadd_sink(part, n, W, nc, i, scale, r);
+            coadd_sink(v, i, r);
             const float nx = r[0], ny = r[1], nz = r[2], nw = r[3];
             const int64_t o = perm ? (int64_t)perm[slot] - p0 : i;
             const float fx = far ? far[3 * o] : 0.f, fy = far ? far[3 * o + 1] : 0.f,
@@ -687,31 +665,18 @@ __global__ void kick_kernel(const Partial *__restrict__ part, int64_t n, int W, 
 
 typedef void (*KernelFn)(KParams);
 
-// Kernel shapes the autotuner chooses among (tunable for the Plummer and
-// single-spline kernels without the density channel; the other kernels run
-// shape 0).
+// Shapes of the one-sided kernel: 128-sink tiles, or the plain drop-in's 64.
+// (The autotuner's shapes are those of the mutual sweep, nf_mutual.cu; boxes
+// that take the one-sided sweep run shape 0 whatever it picks.)
 struct Variant {
     int smax, unr, minb;
-    const char *name;
 };
-static const Variant VARIANTS[] = {
-    {4, 8, 2, "sinks/lane<=4 unroll 8, 2 CTAs/SM"},
-    {4, 16, 2, "sinks/lane<=4 unroll 16, 2 CTAs/SM"},
-    {8, 4, 1, "sinks/lane<=8 unroll 4, 1 CTA/SM"},
-    {2, 4, 3, "sinks/lane<=2 unroll 4, 3 CTAs/SM"},
-    {2, 2, 4, "sinks/lane<=2 unroll 2, 4 CTAs/SM"},
-};
-static constexpr int NVARIANTS = sizeof(VARIANTS) / sizeof(VARIANTS[0]);
+static const Variant VARIANTS[] = {{4, 8, 2}, {2, 4, 3}};
+static constexpr int BOX_VARIANT = 0, PLAIN_VARIANT = 1;
 
 template <int SOFT, bool DENS>
 static KernelFn variant_kernel(int v) {
-    switch (v) {
-    case 1: return pencil_kernel<SOFT, DENS, 4, 16, 2>;
-    case 2: return pencil_kernel<SOFT, DENS, 8, 4, 1>;
-    case 3: return pencil_kernel<SOFT, DENS, 2, 4, 3>;
-    case 4: return pencil_kernel<SOFT, DENS, 2, 2, 4>;
-    default: return pencil_kernel<SOFT, DENS, 4, 8, 2>;
-    }
+    return v == PLAIN_VARIANT ? pencil_kernel<SOFT, DENS, 2, 4, 3> : pencil_kernel<SOFT, DENS, 4, 8, 2>;
 }
 
 static bool tunable(int soft, bool dens) {
@@ -770,7 +735,7 @@ struct HostTile {
 };
 
 static nf_status build_plan(nf_ctx *ctx, nf_box *box, int lo, int hi, int variant, Plan &pl) {
-    const int cpd = box->cpd, R = ctx->cfg.near_field_radius, W = 2 * R + 1;
+    const int cpd = box->cpd, R = ctx->cfg.near_field_radius;
     const auto &cs = box->cell_start;
     auto count = [&](int x, int y, int z) -> int64_t {
         int64_t c = ((int64_t)wrap_h(x, cpd) * cpd + wrap_h(y, cpd)) * cpd + wrap_h(z, cpd);
@@ -779,10 +744,16 @@ static nf_status build_plan(nf_ctx *ctx, nf_box *box, int lo, int hi, int varian
     pl.lo = lo;
     pl.hi = hi;
     pl.variant = variant;
-    const int smax = VARIANTS[variant].smax;
-    const int unr = VARIANTS[variant].unr;
+    const int smax = VARIANTS[BOX_VARIANT].smax;
+    const int unr = VARIANTS[BOX_VARIANT].unr;
     pl.p0 = cs[(int64_t)lo * cpd * cpd];
     pl.n_range = cs[(int64_t)hi * cpd * cpd] - pl.p0;
+    const int rec = ctx->cfg.out_kind == NF_OUT_FLOAT4 ? 16 : 12;
+    pl.out_bytes = (size_t)pl.n_range * rec;
+    NF_CUDA(cudaMalloc(&pl.d_out, pl.out_bytes ? pl.out_bytes : 16));
+    NF_CUDA(cudaMalloc(&pl.d_counters, 2 * sizeof(int)));
+    nf_status mst = mutual_plan(ctx, box, lo, hi, variant, pl, ctx->stream);
+    if (mst != NF_OK || pl.mutual) return mst;
     std::vector<HostTile> tiles;
     tiles.reserve((size_t)(hi - lo) * cpd * cpd + 1024);
     uint64_t pairs = 0, padded = 0;
@@ -828,7 +799,7 @@ static nf_status build_plan(nf_ctx *ctx, nf_box *box, int lo, int hi, int varian
     pl.pairs = pairs;
     pl.padded_pairs = padded;
     // occupancy-derived persistent grid
-    KernelFn fn = pick_kernel(ctx->cfg.softening, ctx->cfg.b2 > 0.f, variant);
+    KernelFn fn = pick_kernel(ctx->cfg.softening, ctx->cfg.b2 > 0.f, BOX_VARIANT);
     int per_sm = 0;
     NF_CUDA(cudaFuncSetAttribute((const void *)fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)kernel_smem()));
@@ -885,7 +856,6 @@ static nf_status build_plan(nf_ctx *ctx, nf_box *box, int lo, int hi, int varian
     for (auto &t : light) lv.push_back(t.it);
     pl.n_heavy_groups = (int)heavy.size();
     pl.n_light = (int)lv.size();
-    NF_CUDA(cudaMalloc(&pl.d_counters, 2 * sizeof(int)));
     if (!hv.empty()) {
         NF_CUDA(cudaMalloc(&pl.d_heavy, hv.size() * sizeof(Item)));
         NF_CUDA(cudaMemcpy(pl.d_heavy, hv.data(), hv.size() * sizeof(Item), cudaMemcpyHostToDevice));
@@ -894,10 +864,6 @@ static nf_status build_plan(nf_ctx *ctx, nf_box *box, int lo, int hi, int varian
         NF_CUDA(cudaMalloc(&pl.d_light, lv.size() * sizeof(Item)));
         NF_CUDA(cudaMemcpy(pl.d_light, lv.data(), lv.size() * sizeof(Item), cudaMemcpyHostToDevice));
     }
-    int rec = ctx->cfg.out_kind == NF_OUT_FLOAT4 ? 16 : 12;
-    pl.out_bytes = (size_t)pl.n_range * rec;
-    NF_CUDA(cudaMalloc(&pl.d_out, pl.out_bytes ? pl.out_bytes : 16));
-    (void)W;
     return NF_OK;
 }
 
@@ -905,6 +871,7 @@ static void free_plan(Plan &pl) {
     if (pl.graph) cudaGraphExecDestroy(pl.graph);
     cudaFree(pl.d_heavy);
     cudaFree(pl.d_light);
+    cudaFree(pl.d_mutual);
     cudaFree(pl.d_counters);
     cudaFree(pl.d_out);
     pl = Plan{};
@@ -929,23 +896,8 @@ static KParams params_from(nf_ctx *ctx, const EngineLaunch &L) {
     kp.n_range = L.n_range;
     kp.nc = cfg.b2 > 0.f ? 4 : 3;
     kp.plain = cfg.accumulation == NF_ACC_PLAIN;
-    const float eps = L.eps > 0.f ? L.eps : cfg.eps;
-    kp.pc.eps = eps;
-    kp.pc.b2 = cfg.b2;
-    if (cfg.softening == SOFT_SINGLE_SPLINE) {
-        double ie2 = (double)eps;  // eps_int^-2
-        kp.pc.near_thr = (float)(1.0 / ie2);
-        kp.pc.inv_eps3 = (float)pow(ie2, 1.5);
-        kp.pc.c1 = (float)(-15.0 * ie2 * ie2 * NEWTON_UNIT);
-        kp.pc.c2 = (float)(6.0 * pow(ie2, 2.5) * NEWTON_UNIT);
-        kp.pc.c3 = (float)(10.0 * pow(ie2, 1.5) * NEWTON_UNIT);
-    }
-    {
-        // margin of the near test: eps (+1% and a rounding allowance)
-        double h = 1.0 / (double)L.cpd;
-        double e = cfg.softening == SOFT_SINGLE_SPLINE ? 1.0 / sqrt((double)eps) : 0.0;
-        kp.near_w = (float)(e * 1.01 + 1e-6 * h);
-    }
+    kp.pc = pair_const(cfg, L.eps);
+    kp.near_w = near_width(cfg, L.eps, L.cpd);
     double h = 1.0 / (double)L.cpd;
     for (int a = 0; a < 2 * R + 1; a++) {
         kp.zshift[a] = (float)((a - R) * h);
@@ -968,7 +920,7 @@ static KParams make_params(nf_ctx *ctx, nf_box *box, const Plan &pl) {
     L.part = box->d_part;
     L.p0 = pl.p0;
     L.n_range = pl.n_range;
-    L.variant = pl.variant;
+    L.variant = BOX_VARIANT;
     L.eps = box->eps;
     return params_from(ctx, L);
 }
@@ -977,16 +929,39 @@ static KParams make_params(nf_ctx *ctx, nf_box *box, const Plan &pl) {
 // to float: out of the pair sums' unit, and for the single spline times
 // eps_int^3 (the raw kernel's units).
 // eps: the softening parameter in use (0: the context's).
-static float output_scale(const nf_config &cfg, float eps = 0.f) {
+static double output_scale_exact(const nf_config &cfg, float eps) {
     if (eps <= 0.f) eps = cfg.eps;
     const double eps3 =
         cfg.softening == SOFT_SINGLE_SPLINE ? pow((double)eps, -1.5) : 1.0;  // eps_int^3
-    return (float)(eps3 / pair_unit(cfg.softening));
+    return eps3 / pair_unit(cfg.softening);
+}
+static float output_scale(const nf_config &cfg, float eps = 0.f) {
+    return (float)output_scale_exact(cfg, eps);
 }
 
-int engine_variant_smax(int variant) { return VARIANTS[variant].smax; }
+static SumsView sums_view(const nf_config &cfg, const Partial *part, int64_t n, float eps) {
+    SumsView v{};
+    v.part = part;
+    v.n = n;
+    v.W = 2 * cfg.near_field_radius + 1;
+    v.nc = cfg.b2 > 0.f ? 4 : 3;
+    v.scale = output_scale(cfg, eps);
+    return v;
+}
+
+static SumsView sums_view(const nf_config &cfg, const Plan &pl, const void *scratch, float eps) {
+    if (!pl.mutual) return sums_view(cfg, (const Partial *)scratch, pl.n_range, eps);
+    SumsView v = sums_view(cfg, nullptr, pl.n_range, eps);
+    v.acc = (const unsigned long long *)scratch;
+    v.bad = (const unsigned char *)scratch + (size_t)pl.n_range * 8 * v.nc;
+    v.scale = (float)std::ldexp(output_scale_exact(cfg, eps), -pl.fbits);
+    v.wscale = (float)std::ldexp(1.0, -pl.wbits);
+    return v;
+}
+
 // The plain drop-in runs the reference's block shape: 64-sink tiles.
-int engine_plain_variant() { return 3; }
+int engine_plain_variant() { return PLAIN_VARIANT; }
+int engine_box_variant() { return BOX_VARIANT; }
 
 int engine_grid(nf_ctx *ctx, int variant) {
     KernelFn fn = pick_kernel(ctx->cfg.softening, ctx->cfg.b2 > 0.f, variant);
@@ -1018,9 +993,18 @@ nf_status engine_coadd(nf_ctx *ctx, const Partial *part, int64_t n, void *out, c
                        float eps, const uint32_t *perm, int64_t p0) {
     if (n <= 0) return NF_OK;
     const nf_config &cfg = ctx->cfg;
-    coadd_kernel<<<ctx->sms * 8, 256, 0, st>>>(part, n, 2 * cfg.near_field_radius + 1,
-                                              cfg.b2 > 0.f ? 4 : 3, output_scale(cfg, eps),
-                                              cfg.out_kind, out, perm, p0);
+    coadd_kernel<<<ctx->sms * 8, 256, 0, st>>>(sums_view(cfg, part, n, eps), cfg.out_kind, out, perm,
+                                              p0);
+    NF_CUDA(cudaGetLastError());
+    return NF_OK;
+}
+
+nf_status engine_coadd_plan(nf_ctx *ctx, const Plan &pl, const void *scratch, void *out,
+                            cudaStream_t st, float eps, const uint32_t *perm) {
+    if (pl.n_range <= 0) return NF_OK;
+    const nf_config &cfg = ctx->cfg;
+    coadd_kernel<<<ctx->sms * 8, 256, 0, st>>>(sums_view(cfg, pl, scratch, eps), cfg.out_kind, out,
+                                              perm, pl.p0);
     NF_CUDA(cudaGetLastError());
     return NF_OK;
 }
@@ -1033,12 +1017,28 @@ nf_status engine_pack(nf_ctx *ctx, const float *x, const float *y, const float *
     return NF_OK;
 }
 
-// The pencil kernel of a plan into the box's partials, between events 0 and 1.
+// The sweep of a plan into the box's scratch, between events 0 and 1.
 static nf_status enqueue_pencil(nf_ctx *ctx, nf_box *box, Plan &pl, cudaStream_t st,
                                 unsigned evflags) {
+    if (pl.mutual) {
+        MutualLaunch L;
+        L.plan = &pl;
+        L.pos = box->d_pos;
+        L.cs = box->d_cs;
+        L.cpd = box->cpd;
+        L.eps = box->eps;
+        L.scratch = box->d_part;
+        L.counter = pl.d_counters;
+        L.before = ctx->ev[0];
+        L.event_flags = evflags;
+        nf_status s = mutual_launch(ctx, L, st);
+        if (s != NF_OK) return s;
+        NF_CUDA(cudaEventRecordWithFlags(ctx->ev[1], st, evflags));
+        return NF_OK;
+    }
     const nf_config &cfg = ctx->cfg;
     KParams kp = make_params(ctx, box, pl);
-    KernelFn fn = pick_kernel(cfg.softening, cfg.b2 > 0.f, pl.variant);
+    KernelFn fn = pick_kernel(cfg.softening, cfg.b2 > 0.f, BOX_VARIANT);
     NF_CUDA(cudaMemsetAsync(pl.d_counters, 0, 2 * sizeof(int), st));
     NF_CUDA(cudaEventRecordWithFlags(ctx->ev[0], st, evflags));
     if (pl.n_heavy_groups + pl.n_light > 0) {
@@ -1051,17 +1051,10 @@ static nf_status enqueue_pencil(nf_ctx *ctx, nf_box *box, Plan &pl, cudaStream_t
 }
 
 static nf_status enqueue_forces(nf_ctx *ctx, nf_box *box, Plan &pl, cudaStream_t st) {
-    const nf_config &cfg = ctx->cfg;
     nf_status est = enqueue_pencil(ctx, box, pl, st, cudaEventRecordExternal);
+    if (est == NF_OK)
+        est = engine_coadd_plan(ctx, pl, box->d_part, pl.d_out, st, box->eps, box->d_perm);
     if (est != NF_OK) return est;
-    const int nc = cfg.b2 > 0.f ? 4 : 3;
-    if (pl.n_range > 0) {
-        int W = 2 * cfg.near_field_radius + 1;
-        int blocks = ctx->sms * 8;
-        coadd_kernel<<<blocks, 256, 0, st>>>(box->d_part, pl.n_range, W, nc, output_scale(cfg, box->eps),
-                                            cfg.out_kind, pl.d_out, box->d_perm, pl.p0);
-        NF_CUDA(cudaGetLastError());
-    }
     NF_CUDA(cudaEventRecordWithFlags(ctx->ev[2], st, cudaEventRecordExternal));
     return NF_OK;
 }
@@ -1097,7 +1090,8 @@ size_t nf_box::device_bytes() const {
                (d_stage ? 3 * (size_t)np * sizeof(float) : 0) + sort_bytes +
                (d_perm ? (size_t)np * sizeof(uint32_t) : 0);
     for (auto &kv : plans) {
-        b += kv.second->out_bytes + (size_t)kv.second->n_light * sizeof(Item) +
+        b += kv.second->out_bytes + (size_t)kv.second->n_mutual * sizeof(MutualItem) +
+             (size_t)kv.second->n_light * sizeof(Item) +
              (size_t)kv.second->n_heavy_groups * WARPS_PER_CTA * sizeof(Item);
     }
     return b;
@@ -1349,12 +1343,14 @@ extern "C" nf_status nf_box_pair_count(nf_ctx *ctx, const nf_box *box, int lo, i
     return NF_OK;
 }
 
-// Partial scratch: (2R+1) slots x nc components x n_range (hi, lo) pairs, shared by
-// the box's plans (grown on demand; cached graphs that refer to the old
-// buffer are dropped).
-static nf_status ensure_scratch(nf_ctx *ctx, nf_box *box, int64_t n_range) {
-    int nc = ctx->cfg.b2 > 0.f ? 4 : 3;
-    size_t need = (size_t)(2 * ctx->cfg.near_field_radius + 1) * nc * (size_t)n_range * sizeof(Partial);
+// Scratch of a plan's sums -- one-sided: (2R+1) slots x nc components x n_range
+// (hi, lo) pairs; mutual: fixed point -- shared by the box's plans (grown on
+// demand; cached graphs that refer to the old buffer are dropped).
+static nf_status ensure_scratch(nf_ctx *ctx, nf_box *box, const Plan &pl) {
+    const int nc = ctx->cfg.b2 > 0.f ? 4 : 3;
+    const size_t need =
+        pl.mutual ? mutual_scratch_bytes(pl.n_range, nc)
+                  : (size_t)(2 * ctx->cfg.near_field_radius + 1) * nc * (size_t)pl.n_range * sizeof(Partial);
     if (need <= box->part_bytes) return NF_OK;
     cudaFree(box->d_part);
     box->d_part = nullptr;
@@ -1377,7 +1373,7 @@ static nf_status new_plan(nf_ctx *ctx, nf_box *box, int lo, int hi, int variant,
                           std::unique_ptr<Plan> &out) {
     std::unique_ptr<Plan> pl(new Plan);
     nf_status st = build_plan(ctx, box, lo, hi, variant, *pl);
-    if (st == NF_OK) st = ensure_scratch(ctx, box, pl->n_range);
+    if (st == NF_OK) st = ensure_scratch(ctx, box, *pl);
     if (st != NF_OK) {
         free_plan(*pl);
         return st;
@@ -1401,7 +1397,7 @@ static nf_status time_pencil(nf_ctx *ctx, nf_box *box, Plan &pl, float *ms) {
 // again and the second launch counts; a long first launch counts as it is.
 static nf_status autotune(nf_ctx *ctx, nf_box *box, int lo, int hi) {
     const bool tun = tunable(ctx->cfg.softening, ctx->cfg.b2 > 0.f);
-    const int nv = tun ? NVARIANTS : 1;
+    const int nv = tun ? MUTUAL_SHAPES : 1;
     int best = 0;
     float best_ms = 3.0e38f;
     for (int v = 0; v < nv; v++) {
@@ -1457,10 +1453,10 @@ nf_status nf::box_plan(nf_ctx *ctx, nf_box *box, int lo, int hi, const Plan **ou
     return st;
 }
 
-extern "C" int nf_kernel_variant_count(void) { return NVARIANTS; }
+extern "C" int nf_kernel_variant_count(void) { return MUTUAL_SHAPES; }
 
 extern "C" const char *nf_kernel_variant_name(int v) {
-    return (v >= 0 && v < NVARIANTS) ? VARIANTS[v].name : "";
+    return (v >= 0 && v < MUTUAL_SHAPES) ? mutual_shape_name(v) : "";
 }
 
 extern "C" nf_status nf_box_tuning(const nf_box *box, int *variant, float *ms, int n) {
@@ -1469,8 +1465,14 @@ extern "C" nf_status nf_box_tuning(const nf_box *box, int *variant, float *ms, i
         return NF_EINVAL;
     }
     *variant = box->variant;
-    for (int i = 0; ms && i < n && i < NVARIANTS; i++) ms[i] = box->tune_ms[i];
+    for (int i = 0; ms && i < n && i < MUTUAL_SHAPES; i++) ms[i] = box->tune_ms[i];
     return NF_OK;
+}
+
+// Kernels of a plan's sweep: the mutual form zeroes its sums with one of its own.
+static int sweep_launches(const Plan &pl) {
+    if (pl.mutual) return 1 + (pl.n_mutual > 0);
+    return pl.n_heavy_groups + pl.n_light > 0;
 }
 
 extern "C" nf_status nf_box_forces(nf_ctx *ctx, nf_box *box, int lo, int hi, void *out,
@@ -1500,8 +1502,8 @@ extern "C" nf_status nf_box_forces(nf_ctx *ctx, nf_box *box, int lo, int hi, voi
     ctx->last.total_ms = t_ms;
     ctx->last.pairs = pl->pairs;
     ctx->last.padded_pairs = pl->padded_pairs;
-    ctx->last.launches = (pl->n_heavy_groups + pl->n_light > 0 ? 1 : 0) + (pl->n_range > 0 ? 1 : 0);
-    ctx->last.items = pl->n_heavy_groups * WARPS_PER_CTA + pl->n_light;
+    ctx->last.launches = sweep_launches(*pl) + (pl->n_range > 0 ? 1 : 0);
+    ctx->last.items = pl->n_mutual + pl->n_heavy_groups * WARPS_PER_CTA + pl->n_light;
     ctx->last.variant = pl->variant;
     return NF_OK;
 }
@@ -1538,9 +1540,8 @@ extern "C" nf_status nf_box_kick(nf_ctx *ctx, nf_box *box, int lo, int hi,
     KickConst k{kick->near_scale, kick->rescale, kick->kick1, kick->kick2, kick->b2};
     if (pl->n_range > 0 || cell_stats) {
         kick_kernel<<<ctx->sms * 8, 256, 0, s>>>(
-            box->d_part, pl->n_range, 2 * cfg.near_field_radius + 1, cfg.b2 > 0.f ? 4 : 3,
-            output_scale(cfg, box->eps), box->d_cs, (int64_t)lo * c2, (int64_t)(hi - lo) * c2,
-            pl->p0, box->d_perm, k, far_acc, vel, acc_out, cfg.out_kind, cell_stats);
+            sums_view(cfg, *pl, box->d_part, box->eps), box->d_cs, (int64_t)lo * c2,
+            (int64_t)(hi - lo) * c2, pl->p0, box->d_perm, k, far_acc, vel, acc_out, cfg.out_kind, cell_stats);
         NF_CUDA(cudaGetLastError());
     }
     NF_CUDA(cudaEventRecord(ctx->ev[2], s));
@@ -1554,8 +1555,8 @@ extern "C" nf_status nf_box_kick(nf_ctx *ctx, nf_box *box, int lo, int hi,
     ctx->last.total_ms = t_ms;
     ctx->last.pairs = pl->pairs;
     ctx->last.padded_pairs = pl->padded_pairs;
-    ctx->last.launches = (pl->n_heavy_groups + pl->n_light > 0 ? 1 : 0) + 1;
-    ctx->last.items = pl->n_heavy_groups * WARPS_PER_CTA + pl->n_light;
+    ctx->last.launches = sweep_launches(*pl) + 1;
+    ctx->last.items = pl->n_mutual + pl->n_heavy_groups * WARPS_PER_CTA + pl->n_light;
     ctx->last.variant = pl->variant;
     return NF_OK;
 }
@@ -1807,8 +1808,8 @@ extern "C" nf_status nf_forces_noalloc(const nf_config *cfg, int cpd, const void
     void *args[] = {&kp, &pencil0, &npen};
     NF_CUDA(cudaLaunchKernel((const void *)fn, dim3(tmp.sms * std::max(per_sm, 1)),
                              dim3(WARPS_PER_CTA * 32), args, smem, st));
-    coadd_kernel<<<tmp.sms * 8, 256, 0, st>>>(L.part, n, 2 * R + 1, kp.nc, output_scale(*cfg),
-                                              cfg->out_kind, out, nullptr, 0);
+    coadd_kernel<<<tmp.sms * 8, 256, 0, st>>>(sums_view(*cfg, L.part, n, 0.f), cfg->out_kind, out,
+                                              nullptr, 0);
     NF_CUDA(cudaGetLastError());
     return NF_OK;
 }

@@ -43,6 +43,16 @@ struct Item {
     int32_t pad0, pad1;
 };
 
+// One warp work item of the mutual sweep (nf_mutual.cu): chunks [c0, c1) of
+// the tile's stream of sources.
+struct MutualItem {
+    int32_t pencil;             // linear id of the pencil's centre cell
+    int32_t sink_begin, nsink;  // the tile, in the pencil's sink stream
+    int32_t S;                  // sinks per lane
+    int32_t c0, c1;
+    int32_t pad0, pad1;
+};
+
 struct Plan {
     int lo = 0, hi = 0;
     int variant = 0;  // kernel shape (index into the variant table)
@@ -51,6 +61,11 @@ struct Plan {
     int n_heavy_groups = 0;
     Item *d_light = nullptr;
     int n_light = 0;
+    // the mutual sweep's work list and fixed-point units (2^-bits)
+    bool mutual = false;
+    MutualItem *d_mutual = nullptr;
+    int n_mutual = 0;
+    int fbits = 0, wbits = 0;
     int *d_counters = nullptr;
     void *d_out = nullptr;
     size_t out_bytes = 0;
@@ -58,6 +73,10 @@ struct Plan {
     int grid = 0, warps = 0;
     cudaGraphExec_t graph = nullptr;
 };
+
+}  // namespace nf
+struct nf_box;
+namespace nf {
 
 // The pencil engine, shared by the batched form (nf_box.cu) and the plain
 // drop-in (nf_sic.cu).  A launch covers the pencils listed in `items` of a
@@ -79,6 +98,28 @@ struct EngineLaunch {
     float eps = 0.f;              // softening parameter (0: the context's)
 };
 nf_status engine_launch(nf_ctx *ctx, const EngineLaunch &L, double box_h, cudaStream_t st);
+// The sweep of a mutual plan: scratch (mutual_scratch_bytes) and counter are
+// zeroed first; `before`, if given, is recorded between that and the sweep.
+struct MutualLaunch {
+    const Plan *plan = nullptr;
+    const float4 *pos = nullptr;
+    const int64_t *cs = nullptr;
+    int cpd = 0;
+    float eps = 0.f;  // softening parameter (0: the context's)
+    void *scratch = nullptr;
+    int *counter = nullptr;
+    cudaEvent_t before = nullptr;
+    unsigned event_flags = 0;
+};
+constexpr int MUTUAL_SHAPES = 5;  // kernel shapes the autotuner chooses among
+const char *mutual_shape_name(int v);
+nf_status mutual_plan(nf_ctx *ctx, const nf_box *box, int lo, int hi, int variant, Plan &pl,
+                      cudaStream_t st);
+nf_status mutual_launch(nf_ctx *ctx, const MutualLaunch &L, cudaStream_t st);
+size_t mutual_scratch_bytes(int64_t n_range, int nc);
+// Records of a plan's sums (one-sided: partials; mutual: fixed point).
+nf_status engine_coadd_plan(nf_ctx *ctx, const Plan &pl, const void *scratch, void *out,
+                            cudaStream_t st, float eps, const uint32_t *perm);
 // perm (optional): the caller's index of each packed slot; record p of the
 // range [p0, p0 + n) is written at perm[p0 + p] - p0.
 nf_status engine_coadd(nf_ctx *ctx, const Partial *part, int64_t n, void *out, cudaStream_t st,
@@ -86,8 +127,8 @@ nf_status engine_coadd(nf_ctx *ctx, const Partial *part, int64_t n, void *out, c
 nf_status engine_pack(nf_ctx *ctx, const float *x, const float *y, const float *z, int64_t n,
                       float4 *out, cudaStream_t st);
 int engine_grid(nf_ctx *ctx, int variant);
-int engine_variant_smax(int variant);
 int engine_plain_variant();
+int engine_box_variant();
 constexpr int ENGINE_WARPS_PER_CTA = 8;
 // SIC size limits from a buffer budget (the reference's bytes-per-block model).
 nf_status sic_limits(int out_kind, int cpd, uint64_t max_buffer_bytes, nf_gpu_limits *lim);

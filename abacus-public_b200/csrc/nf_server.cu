@@ -232,24 +232,37 @@ static nf_status apply_booking(nf_server *s, Booking &bk) {
 
 static nf_status launch_request(nf_server *s, Req *r, Slot &sl, const Plan *pl) {
     nf_ctx *ctx = s->ctx;
-    EngineLaunch L;
-    L.pos = r->box->d_pos;
-    L.cs = r->box->d_cs;
-    L.cpd = r->box->cpd;
-    L.heavy = pl->d_heavy;
-    L.n_heavy_groups = pl->n_heavy_groups;
-    L.light = pl->d_light;
-    L.n_light = pl->n_light;
-    L.counters = sl.counters;
-    L.part = sl.part;
-    L.p0 = pl->p0;
-    L.n_range = pl->n_range;
-    L.variant = pl->variant;
-    L.grid = pl->grid;
-    L.eps = r->box->eps;
-    nf_status st = engine_launch(ctx, L, 0.0, sl.stream);
-    if (st == NF_OK) st = engine_coadd(ctx, sl.part, pl->n_range, sl.out, sl.stream, r->box->eps, r->box->d_perm,
-                                          pl->p0);
+    nf_status st;
+    if (pl->mutual) {
+        MutualLaunch L;
+        L.plan = pl;
+        L.pos = r->box->d_pos;
+        L.cs = r->box->d_cs;
+        L.cpd = r->box->cpd;
+        L.eps = r->box->eps;
+        L.scratch = sl.part;
+        L.counter = sl.counters;
+        st = mutual_launch(ctx, L, sl.stream);
+    } else {
+        EngineLaunch L;
+        L.pos = r->box->d_pos;
+        L.cs = r->box->d_cs;
+        L.cpd = r->box->cpd;
+        L.heavy = pl->d_heavy;
+        L.n_heavy_groups = pl->n_heavy_groups;
+        L.light = pl->d_light;
+        L.n_light = pl->n_light;
+        L.counters = sl.counters;
+        L.part = sl.part;
+        L.p0 = pl->p0;
+        L.n_range = pl->n_range;
+        L.variant = engine_box_variant();
+        L.grid = pl->grid;
+        L.eps = r->box->eps;
+        st = engine_launch(ctx, L, 0.0, sl.stream);
+    }
+    if (st == NF_OK)
+        st = engine_coadd_plan(ctx, *pl, sl.part, sl.out, sl.stream, r->box->eps, r->box->d_perm);
     if (st != NF_OK) return st;
     size_t bytes = (size_t)pl->n_range * rec_bytes(ctx);
     if (bytes)
