@@ -26,6 +26,25 @@ nf_status cuda_fail(cudaError_t e, const char *what) {
 
 using namespace nf;
 
+// On the library's own stream, whatever stream the caller has set: it lives as
+// long as the context.  A block is handed out once it is usable on any stream,
+// and every call waits for its own work before it frees one.
+cudaError_t nf::pool_alloc(nf_ctx *ctx, void **p, size_t bytes) {
+    cudaError_t e = cudaMallocFromPoolAsync(p, bytes ? bytes : 16, ctx->pool, ctx->own_stream);
+    if (e == cudaSuccess && ctx->stream != ctx->own_stream) e = cudaStreamSynchronize(ctx->own_stream);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        *p = nullptr;
+    }
+    return e;
+}
+
+void nf::pool_free(nf_ctx *ctx, void *p) {
+    if (!p) return;
+    if (ctx) cudaFreeAsync(p, ctx->own_stream);
+    else cudaFree(p);
+}
+
 extern "C" const char *nf_last_error(void) { return g_err.c_str(); }
 extern "C" int nf_abi_version(void) { return NF_ABI_VERSION; }
 
@@ -141,6 +160,20 @@ extern "C" nf_status nf_init(const nf_config *cfg, nf_ctx **out) {
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->own_stream, cudaStreamNonBlocking);
     ctx->stream = ctx->own_stream;
     for (int i = 0; i < 4 && e == cudaSuccess; i++) e = cudaEventCreate(&ctx->ev[i]);
+    if (e == cudaSuccess) {
+        cudaMemPoolProps pp{};
+        pp.allocType = cudaMemAllocationTypePinned;
+        pp.location.type = cudaMemLocationTypeDevice;
+        pp.location.id = cfg->device;
+        e = cudaMemPoolCreate(&ctx->pool, &pp);
+    }
+    if (e == cudaSuccess) {
+        size_t freeb = 0, total = 0;
+        e = cudaMemGetInfo(&freeb, &total);
+        uint64_t keep = total / 32;
+        if (e == cudaSuccess)
+            e = cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    }
     if (e != cudaSuccess) {
         nf_status s2 = cuda_fail(e, "nf_init");
         nf_shutdown(ctx);
@@ -160,6 +193,7 @@ extern "C" void nf_shutdown(nf_ctx *ctx) {
     for (int i = 0; i < 4; i++)
         if (ctx->ev[i]) cudaEventDestroy(ctx->ev[i]);
     if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
+    if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
     delete ctx;
 }
 

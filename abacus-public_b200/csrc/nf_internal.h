@@ -71,7 +71,8 @@ struct Plan {
     size_t out_bytes = 0;
     uint64_t pairs = 0, padded_pairs = 0;
     int grid = 0, warps = 0;
-    cudaGraphExec_t graph = nullptr;
+    cudaGraphExec_t graph = nullptr;  // the sweep, captured when it is run again
+    int runs = 0;
 };
 
 }  // namespace nf
@@ -113,9 +114,15 @@ struct MutualLaunch {
 };
 constexpr int MUTUAL_SHAPES = 5;  // kernel shapes the autotuner chooses among
 const char *mutual_shape_name(int v);
-nf_status mutual_plan(nf_ctx *ctx, const nf_box *box, int lo, int hi, int variant, Plan &pl,
-                      cudaStream_t st);
+nf_status mutual_plan(nf_ctx *ctx, const nf_box *box, int lo, int hi, int variant, Plan &pl);
 nf_status mutual_launch(nf_ctx *ctx, const MutualLaunch &L, cudaStream_t st);
+// Device memory from the context's pool (ctx->mu held).
+cudaError_t pool_alloc(nf_ctx *ctx, void **p, size_t bytes);
+template <class T>
+cudaError_t pool_alloc(nf_ctx *ctx, T **p, size_t bytes) {
+    return pool_alloc(ctx, (void **)p, bytes);
+}
+void pool_free(nf_ctx *ctx, void *p);  // null ctx: of a context that is gone
 size_t mutual_scratch_bytes(int64_t n_range, int nc);
 // Records of a plan's sums (one-sided: partials; mutual: fixed point).
 nf_status engine_coadd_plan(nf_ctx *ctx, const Plan &pl, const void *scratch, void *out,
@@ -163,6 +170,14 @@ struct nf_box {
     size_t device_bytes() const;
 };
 
+namespace nf {
+// A kernel shape chosen by the autotuner, and what each candidate took.
+struct Tuned {
+    int variant = -1;
+    float ms[8] = {};
+};
+}  // namespace nf
+
 struct nf_ctx {
     nf_config cfg{};
     int device = 0;
@@ -172,6 +187,12 @@ struct nf_ctx {
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
     nf_timing last{};
     std::mutex mu;  // serialises nf_box_forces on one context
+    // device memory of boxes and plans; freed blocks up to 1/32 of the device
+    // stay here for the next box, until nf_shutdown
+    cudaMemPool_t pool = nullptr;
+    // shapes chosen so far, by size of the work: (log2 of the range's
+    // particles, log2 of their mean number of pairs)
+    std::map<std::pair<int, int>, nf::Tuned> tuned;
     // plain drop-in GPU control (nf_sic.cu)
     struct Sic;
     Sic *sic = nullptr;

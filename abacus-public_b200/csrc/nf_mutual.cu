@@ -890,8 +890,8 @@ static int mutual_grid(nf_ctx *ctx, int variant) {
 
 // The work list of slabs [lo, hi): NF_OK with pl.mutual false where the engine
 // does not apply (the caller then plans the one-sided sweep).
-nf_status mutual_plan(nf_ctx *ctx, const nf_box *box, int lo, int hi, int variant, Plan &pl,
-                      cudaStream_t st) {
+nf_status mutual_plan(nf_ctx *ctx, const nf_box *box, int lo, int hi, int variant, Plan &pl) {
+    cudaStream_t st = ctx->stream;
     pl.mutual = false;
     const nf_config &cfg = ctx->cfg;
     if (cfg.accumulation != NF_ACC_COMPENSATED) return NF_OK;
@@ -900,7 +900,7 @@ nf_status mutual_plan(nf_ctx *ctx, const nf_box *box, int lo, int hi, int varian
     a.g = Geometry{box->d_cs, box->cpd, R, lo, hi};
     a.smax = smax_of(cfg, variant);
     a.forced = cfg.sinks_per_lane;
-    NF_CUDA(cudaMallocAsync(&a.sums, sizeof(PlanSums), st));
+    NF_CUDA(pool_alloc(ctx, &a.sums, sizeof(PlanSums)));
     PlanSums h;
     const int64_t pencils = (int64_t)(hi - lo) * box->cpd * box->cpd;
     const int blocks = (int)std::min<int64_t>((pencils + 7) / 8, (int64_t)ctx->sms * 16);
@@ -914,7 +914,7 @@ nf_status mutual_plan(nf_ctx *ctx, const nf_box *box, int lo, int hi, int varian
     if (e != cudaSuccess || h.max_sources > INT32_MAX / 8 || h.max_sinks > INT32_MAX / 8 ||
         !mutual_bits(cfg.softening, eps, cfg.b2, box->cpd, (double)W * h.max_sources, &pl.fbits,
                      &pl.wbits)) {
-        cudaFreeAsync(a.sums, st);
+        pool_free(ctx, a.sums);
         return e != cudaSuccess ? cuda_fail(e, "work list (sums)") : NF_OK;
     }
     pl.grid = mutual_grid(ctx, variant);
@@ -930,10 +930,10 @@ nf_status mutual_plan(nf_ctx *ctx, const nf_box *box, int lo, int hi, int varian
             n += h.hist[i];
         }
         if (n > (uint64_t)INT32_MAX / 2) {
-            cudaFreeAsync(a.sums, st);
+            pool_free(ctx, a.sums);
             return NF_OK;
         }
-        e = cudaMalloc(&pl.d_mutual, std::max<uint64_t>(n, 1) * sizeof(MutualItem));
+        e = pool_alloc(ctx, &pl.d_mutual, n * sizeof(MutualItem));
     }
     if (e == cudaSuccess) {
         a.items = pl.d_mutual;
@@ -943,8 +943,8 @@ nf_status mutual_plan(nf_ctx *ctx, const nf_box *box, int lo, int hi, int varian
         plan_kernel<2><<<blocks, 256, 0, st>>>(a);
         e = cudaGetLastError();
     }
-    cudaFreeAsync(a.sums, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    pool_free(ctx, a.sums);
     if (e != cudaSuccess) return cuda_fail(e, "work list");
     pl.mutual = true;
     pl.n_mutual = (int)n;

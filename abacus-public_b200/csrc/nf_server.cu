@@ -374,6 +374,10 @@ extern "C" nf_status nf_server_start(nf_ctx *ctx, const nf_server_config *cfg, n
         set_error("nf_server_start: max_inflight above 256");
         return NF_EINVAL;
     }
+    {
+        std::lock_guard<std::mutex> lk(ctx->mu);
+        NF_CUDA(cudaMemPoolTrimTo(ctx->pool, 0));  // what the context keeps but does not use
+    }
     size_t freeb = 0, total = 0;
     NF_CUDA(cudaMemGetInfo(&freeb, &total));
     s->budget = s->cfg.hbm_budget_bytes ? s->cfg.hbm_budget_bytes : (size_t)(0.9 * (double)freeb);

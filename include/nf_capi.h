@@ -375,7 +375,9 @@ nf_status nf_last_timing(nf_ctx *ctx, nf_timing *t);
 
 /* Kernel shapes the autotuner chooses among (sinks per lane, unroll depth,
  * CTAs per SM).  The first nf_box_forces call on a box times every shape on
- * the requested slab range and keeps the fastest for that box. */
+ * the requested slab range and keeps the fastest for that box, and for later
+ * boxes of the context whose first call does work of the same size
+ * (particles, and pairs per particle, within a factor of two). */
 int nf_kernel_variant_count(void);
 const char *nf_kernel_variant_name(int variant);
 /* The box's chosen shape (-1 before tuning) and the kernel time of each
