@@ -65,6 +65,7 @@ struct Plan {
     bool mutual = false;
     MutualItem *d_mutual = nullptr;
     int n_mutual = 0;
+    bool onesided = false;  // met one-sided throughout (drop-in SICs)
     int fbits = 0, wbits = 0;
     int *d_counters = nullptr;
     void *d_out = nullptr;
@@ -109,11 +110,25 @@ struct MutualLaunch {
     float eps = 0.f;  // softening parameter (0: the context's)
     void *scratch = nullptr;
     int *counter = nullptr;
+    bool zeroed = false;  // scratch and counter are zero already (mutual_unpack)
     cudaEvent_t before = nullptr;
     unsigned event_flags = 0;
 };
 constexpr int MUTUAL_SHAPES = 5;  // kernel shapes the autotuner chooses among
 const char *mutual_shape_name(int v);
+int mutual_grid(nf_ctx *ctx, int variant);
+// A SIC's positions (x, y, z of n4 each, a multiple of four, 16-byte aligned)
+// to float4 records; zeroes scratch and counter.
+nf_status mutual_unpack(nf_ctx *ctx, const Plan &pl, const float *xyz, int64_t n4, float4 *pos,
+                        void *scratch, int *counter, cudaStream_t st);
+// A sink pencil of a drop-in SIC: centre cell (y, z) of the middle slab, its
+// sinks [first, first + n) in the pencil's sink stream, its sources.
+struct SicPencil {
+    int y, z;
+    int64_t first, n, sources;
+};
+bool mutual_sic_list(const nf_config &cfg, int cpd, const std::vector<SicPencil> &pencils, const int64_t *cs,
+                     int warps, Plan &pl, std::vector<MutualItem> &items);
 nf_status mutual_plan(nf_ctx *ctx, const nf_box *box, int lo, int hi, int variant, Plan &pl);
 nf_status mutual_launch(nf_ctx *ctx, const MutualLaunch &L, cudaStream_t st);
 // Device memory from the context's pool (ctx->mu held).

@@ -92,7 +92,7 @@ struct Seg {
 constexpr int NSEG = 6;
 
 // Segment i of a tile's pass over its stream; false if it holds no pair.
-__device__ __forceinline__ bool segment(const Stream &s, int R, int i, Seg &g) {
+__host__ __device__ __forceinline__ bool segment(const Stream &s, int R, int i, Seg &g) {
     const unsigned own = 1u << R;
     const bool tri = s.triangle && (s.present & own);
     const int o = s.Ms;
@@ -108,41 +108,45 @@ __device__ __forceinline__ bool segment(const Stream &s, int R, int i, Seg &g) {
     return g.mask != 0 && g.e > g.b;
 }
 
-__device__ __forceinline__ int wrapc(int i, int cpd) {
+__host__ __device__ __forceinline__ int wrapc(int i, int cpd) {
     return i < 0 ? i + cpd : (i >= cpd ? i - cpd : i);
 }
 
+// Cells, and the slabs [lo, hi) that hold the sinks.  onesided: no pair is met
+// mutually (a drop-in SIC: a sink's sum then has the same order whatever rows
+// and z cells the SIC holds).
 struct Geometry {
     const int64_t *__restrict__ cs;
     int cpd, R, lo, hi;
+    bool onesided;
 };
 
-// Class of source column c (dx, dy) for a pencil at slab x: 0 mutual, 1 the
-// own column, 2 one-sided, 3 not met here (its pencil meets this one).
-__device__ __forceinline__ int column_class(const Geometry &g, int x, int dx, int dy) {
+// Class of source column (dx, dy) for a pencil at slab x: 0 mutual, 1 the own
+// column, 2 one-sided, 3 not met here (its pencil meets this one).
+__host__ __device__ __forceinline__ int column_class(const Geometry &g, int x, int dx, int dy) {
     if (dx == 0 && dy == 0) return 1;
     const int xs = wrapc(x + dx, g.cpd);
-    if (xs < g.lo || xs >= g.hi) return 2;
+    if (g.onesided || xs < g.lo || xs >= g.hi) return 2;
     return dx > 0 || (dx == 0 && dy > 0) ? 0 : 3;
 }
 
 // Counts of the pencil's sink cells -> the own column's part of Stream.
-__device__ __forceinline__ void own_column(Stream &s, const int *spre, int R) {
+__host__ __device__ __forceinline__ void own_column(Stream &s, const int *spre, int R, bool onesided) {
     const int W = 2 * R + 1;
     s.own_begin = spre[R];
     s.own = spre[R + 1] - spre[R];
-    s.triangle = s.own >= DENSE_CELL;
+    s.triangle = !onesided && s.own >= DENSE_CELL;
     s.mutual = s.onesided = 0;
     for (int a = 0; a < W; a++) {
         if (a == R) continue;
-        const bool dense = max(s.own, spre[a + 1] - spre[a]) >= DENSE_CELL;
+        const bool dense = !onesided && max(s.own, spre[a + 1] - spre[a]) >= DENSE_CELL;
         if (!dense) s.onesided |= 1u << a;
         else if (a > R) s.mutual |= 1u << a;
     }
 }
 
 // The tile's part of Stream: sinks [s0, s1) of the pencil's sink stream.
-__device__ __forceinline__ void own_tile(Stream &s, const int *spre, int R, int s0, int s1) {
+__host__ __device__ __forceinline__ void own_tile(Stream &s, const int *spre, int R, int s0, int s1) {
     s.present = 0;
     for (int a = 0; a < 2 * R + 1; a++)
         if (max(s0, spre[a]) < min(s1, spre[a + 1])) s.present |= 1u << a;
@@ -156,10 +160,10 @@ __device__ __forceinline__ void own_tile(Stream &s, const int *spre, int R, int 
 
 // SM sub-partition cycles of one chunk of 64 sources, by sinks per lane,
 // mutual and one-sided, and of a tile's set-up: what the list is balanced by.
-__device__ __forceinline__ long long chunk_cost(int S, bool mutual) {
+__host__ __device__ __forceinline__ long long chunk_cost(int S, bool mutual) {
     return mutual ? 600 + 1150 * S : 300 + 900 * S;
 }
-__device__ __forceinline__ long long tile_cost(int S) { return 2500 + 500 * S; }
+__host__ __device__ __forceinline__ long long tile_cost(int S) { return 2500 + 500 * S; }
 
 struct PlanSums {
     unsigned long long pairs, slots;  // interactions, and slots evaluated for them
@@ -185,7 +189,7 @@ __device__ __forceinline__ int cost_class(long long cost) {  // 0 = longest (2^2
 // Sinks per lane of the next tile of a pencil with `rem` sinks left: the
 // smallest tile that holds them, but 65-96 take 64 + 32 slots instead of 128
 // and 129-192 take 128 + 32 or 128 + 64 instead of 256 (by chunk_cost).
-__device__ __forceinline__ int tile_S(int rem, int smax, int forced) {
+__host__ __device__ __forceinline__ int tile_S(int rem, int smax, int forced) {
     if (forced) return min(forced, smax);
     return rem <= 32 ? 1 : rem <= 96 ? 2 : (rem <= 192 || smax == 4) ? 4 : 8;
 }
@@ -244,7 +248,7 @@ __global__ void plan_kernel(PlanArgs p) {
         if (PASS == 0 && lane == 0) pairs += (unsigned long long)np * mt;
         Stream s;
         s.Ms = ms;
-        own_column(s, spre, R);
+        own_column(s, spre, R, g.onesided);
         s.M = ms + s.own + mo;
         // full tiles of smax * 32 sinks, then the rest in smaller ones
         const int Sf = p.forced ? min(p.forced, p.smax) : p.smax;
@@ -401,7 +405,7 @@ __device__ int setup_tables(const MParams &kp, int pencil, WarpSmem &ws, int lan
     __syncwarp();
     s.Ms = ws.cpre[nm];
     s.M = ws.cpre[ncol];
-    own_column(s, ws.spre, R);
+    own_column(s, ws.spre, R, g.onesided);
     return nm;
 }
 
@@ -640,6 +644,10 @@ __device__ void run_item(const MParams &kp, WarpSmem &ws, float4 *hl, const Mutu
             fold_smem(hl[(2 * N + q) * 32], k.pz[q]);
         }
     };
+    // drop-in SICs fold every chunk (+1 %): their long one-sided streams, split
+    // less finely than the former 64-sink tiles, would otherwise have raised
+    // the error of uniform 64^3 from 2.1e-7 to 3.0e-7
+    const int fold_every = kp.g.onesided ? 1 : FOLD;
     int vc = 0, since_fold = 0;  // chunks before this segment; chunks since the last fold
 #pragma unroll 1
     for (int i = 0; i < NSEG; i++) {
@@ -715,7 +723,7 @@ __device__ void run_item(const MParams &kp, WarpSmem &ws, float4 *hl, const Mutu
                         group_onesided<SOFT, DENS, S, false, SIDE>(bxy, bz, mp, k, kp.pc);
                 }
             }
-            if (++since_fold == FOLD) {
+            if (++since_fold >= fold_every) {
                 fold_all();
                 since_fold = 0;
             }
@@ -874,7 +882,7 @@ size_t mutual_scratch_bytes(int64_t n_range, int nc) { return (size_t)n_range * 
 
 const char *mutual_shape_name(int v) { return SHAPES[v].name; }
 
-static int mutual_grid(nf_ctx *ctx, int variant) {
+int mutual_grid(nf_ctx *ctx, int variant) {
     MutualFn fn = pick(ctx->cfg.softening, ctx->cfg.b2 > 0.f, variant);
     const size_t smem = smem_bytes(smax_of(ctx->cfg, variant));
     int per_sm = 0;
@@ -888,6 +896,69 @@ static int mutual_grid(nf_ctx *ctx, int variant) {
     return ctx->sms * std::max(per_sm, 1);
 }
 
+// The work list of sink pencils of the middle slab of a drop-in SIC's mini box
+// (2R+1 slabs, cell table cs on the host), made on the host: a SIC is a few
+// hundred pencils, and its list travels with its positions.  Every pair is
+// met one-sided.  Fills pl's units and counts and `items`; false where the
+// engine does not apply.  `warps`: of a full launch.
+bool mutual_sic_list(const nf_config &cfg, int cpd, const std::vector<SicPencil> &pencils, const int64_t *cs,
+                     int warps, Plan &pl, std::vector<MutualItem> &items) {
+    if (cfg.accumulation != NF_ACC_COMPENSATED) return false;
+    const int R = cfg.near_field_radius, W = 2 * R + 1;
+    const int smax = smax_of(cfg, 0);
+    struct Tile {
+        MutualItem it;
+        int chunks, pieces;
+        long long cost;  // of the tile, then of a piece
+    };
+    std::vector<Tile> tiles;
+    tiles.reserve(4 * pencils.size());
+    int64_t max_sources = 0;
+    long long total = 0;
+    pl.pairs = 0;
+    for (const SicPencil &p : pencils) {
+        if (p.sources > INT32_MAX / 8 || p.first + p.n > INT32_MAX / 8) return false;
+        max_sources = std::max(max_sources, p.sources);
+        pl.pairs += (uint64_t)p.n * (uint64_t)p.sources;
+        const int64_t centre = ((int64_t)R * cpd + p.y) * cpd + p.z;
+        const int own = (int)(cs[centre + 1] - cs[centre]);
+        // the stream: the centre cell, then all other columns
+        const int chunks = (own + CHUNK - 1) / CHUNK + ((int)p.sources - own + CHUNK - 1) / CHUNK;
+        for (int64_t s0 = p.first, end = p.first + p.n; s0 < end;) {
+            const int S = tile_S((int)(end - s0), smax, cfg.sinks_per_lane);
+            const int n = (int)std::min<int64_t>(end - s0, 32 * S);
+            const long long cost = chunks * chunk_cost(S, false);
+            tiles.push_back(Tile{MutualItem{(int)centre, (int)s0, n, S, 0, 0, 0, 0}, chunks, 1, cost});
+            total += cost + tile_cost(S);
+            s0 += n;
+        }
+    }
+    if (!mutual_bits(cfg.softening, cfg.eps, cfg.b2, cpd, (double)W * max_sources, &pl.fbits, &pl.wbits))
+        return false;
+    // pieces of bounded cost, longest first
+    const long long cap = std::max(1LL, total / ((long long)warps * 2));
+    for (Tile &t : tiles) {
+        t.pieces = (int)std::max(1LL, std::min((long long)(t.chunks / 4), (t.cost + cap - 1) / cap));
+        t.cost /= t.pieces;
+    }
+    std::sort(tiles.begin(), tiles.end(), [](const Tile &a, const Tile &b) { return a.cost > b.cost; });
+    items.clear();
+    for (const Tile &t : tiles)
+        for (int k = 0; k < t.pieces; k++) {
+            MutualItem it = t.it;
+            it.c0 = (int)((int64_t)t.chunks * k / t.pieces);
+            it.c1 = (int)((int64_t)t.chunks * (k + 1) / t.pieces);
+            items.push_back(it);
+        }
+    pl.mutual = true;
+    pl.variant = 0;
+    pl.lo = R;
+    pl.hi = R + 1;
+    pl.onesided = true;
+    pl.n_mutual = (int)items.size();
+    return true;
+}
+
 // The work list of slabs [lo, hi): NF_OK with pl.mutual false where the engine
 // does not apply (the caller then plans the one-sided sweep).
 nf_status mutual_plan(nf_ctx *ctx, const nf_box *box, int lo, int hi, int variant, Plan &pl) {
@@ -897,7 +968,7 @@ nf_status mutual_plan(nf_ctx *ctx, const nf_box *box, int lo, int hi, int varian
     if (cfg.accumulation != NF_ACC_COMPENSATED) return NF_OK;
     const int R = cfg.near_field_radius, W = 2 * R + 1;
     PlanArgs a{};
-    a.g = Geometry{box->d_cs, box->cpd, R, lo, hi};
+    a.g = Geometry{box->d_cs, box->cpd, R, lo, hi, false};
     a.smax = smax_of(cfg, variant);
     a.forced = cfg.sinks_per_lane;
     NF_CUDA(pool_alloc(ctx, &a.sums, sizeof(PlanSums)));
@@ -953,29 +1024,76 @@ nf_status mutual_plan(nf_ctx *ctx, const nf_box *box, int lo, int hi, int varian
     return NF_OK;
 }
 
-static __global__ void zero_kernel(uint4 *a, size_t n16, unsigned char *tail, size_t tail_bytes, int *counter) {
-    const size_t i0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    for (size_t i = i0; i < n16; i += (size_t)gridDim.x * blockDim.x) a[i] = make_uint4(0, 0, 0, 0);
-    if (i0 < tail_bytes) tail[i0] = 0;
-    if (i0 == 0) *counter = 0;
+struct ZeroArgs {
+    uint4 *a;
+    size_t n16;
+    unsigned char *tail;
+    int tail_bytes;
+    int *counter;
+};
+
+static ZeroArgs zero_args(nf_ctx *ctx, const Plan &pl, void *scratch, int *counter) {
+    const size_t bytes = mutual_scratch_bytes(pl.n_range, ctx->cfg.b2 > 0.f ? 4 : 3);
+    return ZeroArgs{(uint4 *)scratch, bytes / 16, (unsigned char *)scratch + bytes / 16 * 16,
+                    (int)(bytes % 16), counter};
 }
 
-// Zero the sums and run the sweep of a plan.
+static __device__ __forceinline__ void zero_range(const ZeroArgs &z, int64_t i0, int64_t stride) {
+    for (int64_t i = i0; i < (int64_t)z.n16; i += stride) z.a[i] = make_uint4(0, 0, 0, 0);
+    if (i0 < z.tail_bytes) z.tail[i0] = 0;
+    if (i0 == 0) *z.counter = 0;
+}
+
+static __global__ void zero_kernel(ZeroArgs z) {
+    zero_range(z, (int64_t)blockIdx.x * blockDim.x + threadIdx.x, (int64_t)gridDim.x * blockDim.x);
+}
+
+// A SIC's start on the device in one launch: positions packed from SoA to
+// float4 records, four to a thread (n4, a multiple of four, in each of x, y,
+// z), and the sums zeroed.  (Reading the positions from pinned host memory
+// here, without the copy before it, was slower: uniform 64^3 driver sweep 3.80
+// against 3.30 ms, clustered 96^3 11.4 against 10.1.)
+static __global__ void unpack_kernel(const float4 *__restrict__ x, const float4 *__restrict__ y,
+                                     const float4 *__restrict__ z, int64_t n4, float4 *pos,
+                                     ZeroArgs zero) {
+    const int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t i = i0; i < n4 / 4; i += stride) {
+        const float4 a = x[i], b = y[i], c = z[i];
+        pos[4 * i] = make_float4(a.x, b.x, c.x, 0.f);
+        pos[4 * i + 1] = make_float4(a.y, b.y, c.y, 0.f);
+        pos[4 * i + 2] = make_float4(a.z, b.z, c.z, 0.f);
+        pos[4 * i + 3] = make_float4(a.w, b.w, c.w, 0.f);
+    }
+    zero_range(zero, i0, stride);
+}
+
+nf_status mutual_unpack(nf_ctx *ctx, const Plan &pl, const float *xyz, int64_t n4, float4 *pos,
+                        void *scratch, int *counter, cudaStream_t st) {
+    const ZeroArgs zero = zero_args(ctx, pl, scratch, counter);
+    const int64_t work = std::max<int64_t>(n4 / 4, (int64_t)zero.n16);
+    const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((work + 255) / 256, ctx->sms * 4));
+    unpack_kernel<<<blocks, 256, 0, st>>>((const float4 *)xyz, (const float4 *)(xyz + n4),
+                                          (const float4 *)(xyz + 2 * n4), n4, pos, zero);
+    NF_CUDA(cudaGetLastError());
+    return NF_OK;
+}
+
+// Zero the sums (unless mutual_unpack has) and run the sweep of a plan.
 nf_status mutual_launch(nf_ctx *ctx, const MutualLaunch &L, cudaStream_t st) {
     const nf_config &cfg = ctx->cfg;
     const Plan &pl = *L.plan;
     const int nc = cfg.b2 > 0.f ? 4 : 3;
-    const size_t bytes = mutual_scratch_bytes(pl.n_range, nc);
-    zero_kernel<<<ctx->sms * 4, 256, 0, st>>>((uint4 *)L.scratch, bytes / 16,
-                                              (unsigned char *)L.scratch + bytes / 16 * 16, bytes % 16,
-                                              L.counter);
-    NF_CUDA(cudaGetLastError());
+    if (!L.zeroed) {
+        zero_kernel<<<ctx->sms * 4, 256, 0, st>>>(zero_args(ctx, pl, L.scratch, L.counter));
+        NF_CUDA(cudaGetLastError());
+    }
     if (L.before) NF_CUDA(cudaEventRecordWithFlags(L.before, st, L.event_flags));
     if (pl.n_mutual == 0) return NF_OK;
     MParams kp;
     memset(&kp, 0, sizeof(kp));
     kp.pos = L.pos;
-    kp.g = Geometry{L.cs, L.cpd, cfg.near_field_radius, pl.lo, pl.hi};
+    kp.g = Geometry{L.cs, L.cpd, cfg.near_field_radius, pl.lo, pl.hi, pl.onesided};
     kp.items = pl.d_mutual;
     kp.n_items = pl.n_mutual;
     kp.counter = L.counter;

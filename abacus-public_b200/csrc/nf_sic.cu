@@ -11,13 +11,13 @@
 // How a SIC runs here (B200-first, not the reference's pencil gather):
 //   1. the SIC's source rows of the 2R+1 slabs (each particle once, rather
 //      than the reference's five copies per pencil, PencilPlan.cc:22-90,
-//      214-255) are packed into pinned staging and copied to the device;
+//      214-255) are packed into pinned staging with the work list and the cell table, and
+//      copied to the device at once;
 //   2. a pack kernel builds float4 records, forming a "mini box" of 2R+1
 //      slabs with the SIC's cell offsets;
-//   3. one launch of the pencil engine (the reference's block shape: tiles of
-//      64 sinks, in SIC order, no splitting, no graph) writes per-pencil
-//      compensated FP32 partials, and the co-add kernel sums the 2R+1 pencils of each
-//      sink on the device (PencilPlan.cc:140-207 co-adds on the host);
+//   3. one launch of the engine of nf_mutual.cu, one-sided, sums the 2R+1
+//      pencils of each sink on the device (PencilPlan.cc:140-207 co-adds on
+//      the host);
 //   4. the rows' accelerations are copied back and stored into AccSlab.
 #include <algorithm>
 #include <chrono>
@@ -58,6 +58,13 @@ struct SicBuffer {
     int64_t *h_cs = nullptr;
     Item *h_items = nullptr;
     size_t cap_particles = 0, cap_sinks = 0, cap_items = 0, cap_cells = 0;
+    // mutual form: cell table, work list and positions in one block, one copy
+    void *h_block = nullptr, *d_block = nullptr;
+    size_t cap_block = 0, cap_pos = 0;
+    int grid = 0;  // CTAs of a full mutual launch
+    std::vector<int64_t> cnt, rowstart, cellstart, cs;
+    std::vector<SicPencil> pencils;
+    std::vector<MutualItem> list;
 };
 
 static void host_free(void *p, bool pinned) {
@@ -83,6 +90,10 @@ static void release(SicBuffer &b) {
     cudaFree(b.d_part);
     cudaFree(b.d_out);
     cudaFree(b.d_counters);
+    cudaFree(b.d_block);
+    host_free(b.h_block, b.pinned);
+    b.d_block = b.h_block = nullptr;
+    b.cap_block = b.cap_pos = 0;
     host_free(b.h_raw, b.pinned);
     host_free(b.h_out, b.pinned);
     host_free(b.h_cs, b.pinned);
@@ -107,23 +118,39 @@ static void release(SicBuffer &b) {
 }
 
 // Grow a buffer's arrays to hold a task (1.25x headroom; never shrinks).
+// block: bytes of the mutual form's block, 0 for the one-sided form.
 static nf_status grow(nf_ctx *ctx, SicBuffer &b, size_t particles, size_t sinks, size_t items,
-                      size_t cells) {
+                      size_t cells, size_t block) {
     const int W = 2 * ctx->cfg.near_field_radius + 1;
     const int nc = ctx->cfg.b2 > 0.f ? 4 : 3;
     const size_t rec = ctx->cfg.out_kind == NF_OUT_FLOAT4 ? 16 : 12;
     auto up = [](size_t n) { return n + n / 4 + 1024; };
-    if (particles > b.cap_particles) {
+    if (particles > b.cap_pos) {
+        size_t c = up(particles);
+        cudaFree(b.d_pos);
+        b.d_pos = nullptr;
+        b.cap_pos = 0;
+        NF_CUDA(cudaMalloc(&b.d_pos, c * sizeof(float4)));
+        b.cap_pos = c;
+    }
+    if (block > b.cap_block) {
+        size_t c = up(block);
+        cudaFree(b.d_block);
+        host_free(b.h_block, b.pinned);
+        b.d_block = b.h_block = nullptr;
+        b.cap_block = 0;
+        NF_CUDA(cudaMalloc(&b.d_block, c));
+        NF_CUDA(host_alloc(&b.h_block, c, b.pinned, true));
+        b.cap_block = c;
+    }
+    if (block == 0 && particles > b.cap_particles) {
         size_t c = up(particles);
         cudaFree(b.d_raw);
-        cudaFree(b.d_pos);
         host_free(b.h_raw, b.pinned);
         b.d_raw = nullptr;
-        b.d_pos = nullptr;
         b.h_raw = nullptr;
         b.cap_particles = 0;
         NF_CUDA(cudaMalloc(&b.d_raw, 3 * c * sizeof(float)));
-        NF_CUDA(cudaMalloc(&b.d_pos, c * sizeof(float4)));
         NF_CUDA(host_alloc((void **)&b.h_raw, 3 * c * sizeof(float), b.pinned, true));
         b.cap_particles = c;
     }
@@ -212,101 +239,168 @@ static nf_status check_desc(nf_ctx *ctx, const nf_sic_desc &d, int jlow, int jhi
     return NF_OK;
 }
 
-static uint64_t items_pairs(const std::vector<Item> &items) {
-    uint64_t p = 0;
-    for (const Item &it : items) p += (uint64_t)it.nsink * (uint64_t)(it.src_end - it.src_begin);
-    return p;
+// Pencil k of a row is centred on z = (k + R) mod cpd (index_to_zcen,
+// PencilOnPencil.cc:37-43, one z-domain per node); 2D: on node_z_start + k + R,
+// brought back by node_z_size + 2R past the upper ghost edge, so the centres
+// cover the primary cells and R ghost cells on each side.
+static int pencil_z(const nf_sic_desc &d, int k) {
+    const int R = d.nfradius, zs = d.node_z_start, zn = d.node_z_size;
+    if (zn == 0) return (k + R) % d.cpd;
+    int kk = k + zs + R;
+    if (kk >= zs + zn + R) kk -= zn + 2 * R;
+    return wrapi(kk, d.cpd);
+}
+
+static bool primary_z(const nf_sic_desc &d, int z) {
+    return d.node_z_size == 0 || wrapi(z - d.node_z_start, d.cpd) < d.node_z_size;
 }
 
 static void sic_account(nf_ctx *ctx, float kernel_ms, uint64_t pairs);
 
-static nf_status run_task(nf_ctx *ctx, SicBuffer &b, const SicTask &t) {
+// Stage the SIC's source cells (each particle once) as SoA at hx, hy, hz; runs
+// that follow each other in the slab and in the mini box go as one copy.  1D:
+// whole rows; 2D: cell by cell (ghost cells included).
+static nf_status stage_sources(const SicBuffer &b, const SicTask &t, float *hx, float *hy, float *hz) {
     const nf_sic_desc &d = t.d;
-    nf_status st = check_desc(ctx, d, t.jlow, t.jhigh);
-    if (st != NF_OK) return st;
-    NF_CUDA(cudaSetDevice(b.device));
-    const int R = d.nfradius, W = 2 * R + 1, cpd = d.cpd, nk = d.nk;
-    const int jw = t.jhigh - t.jlow, nrows = jw + 2 * R;
-    const int64_t ncell = (int64_t)W * cpd * cpd;
-    // Pencil k of a row is centred on z = (k + R) mod cpd (index_to_zcen,
-    // PencilOnPencil.cc:37-43, one z-domain per node); 2D: on node_z_start +
-    // k + R, brought back by node_z_size + 2R past the upper ghost edge, so
-    // the centres cover the primary cells and R ghost cells on each side.
+    const int R = d.nfradius, W = 2 * R + 1, cpd = d.cpd;
     const bool two_d = d.node_z_size > 0;
-    const int zs = d.node_z_start, zn = d.node_z_size;
-    auto zcen = [&](int k) {
-        if (!two_d) return (k + R) % cpd;
-        int kk = k + zs + R;
-        if (kk >= zs + zn + R) kk -= zn + 2 * R;
-        return wrapi(kk, cpd);
-    };
-    auto primary = [&](int z) { return !two_d || wrapi(z - zs, cpd) < zn; };
-    // cell counts of the mini box: slot s = source slab x-R+s, rows of the SIC
-    std::vector<int64_t> cnt(ncell, 0), rowstart(W * cpd, -1), cellstart(two_d ? ncell : 0, -1);
-    std::vector<char> row_used(cpd, 0);
-    for (int r = 0; r < nrows; r++) {
-        int y = wrapi(t.jlow - R + r, cpd);
-        row_used[y] = 1;
-        for (int k = 0; k < nk; k++) {
-            int z = zcen(k);
-            const nf_cell_plan *pl = d.source_plan + ((int64_t)r * nk + k) * W;
-            for (int s = 0; s < W; s++) {
-                if (pl[s].n < 0) {
-                    set_error("nf_sic_execute: negative cell count");
-                    return NF_EINVAL;
-                }
-                cnt[((int64_t)s * cpd + y) * cpd + z] = pl[s].n;
-                if (two_d) cellstart[((int64_t)s * cpd + y) * cpd + z] = pl[s].start;
-                else if (z == 0) rowstart[s * cpd + y] = pl[s].start;
-            }
-        }
-    }
-    // dense mirror offsets (linear cell order)
-    size_t nitems = 0;
-    NF_CUDA(cudaSetDevice(b.device));
-    std::vector<int64_t> cs(ncell + 1, 0);
-    for (int64_t c = 0; c < ncell; c++) cs[c + 1] = cs[c] + cnt[c];
-    const int64_t n_mini = cs[ncell];
-    const int64_t p0 = cs[((int64_t)R * cpd + t.jlow) * cpd];
-    const int64_t p1 = cs[((int64_t)R * cpd + t.jhigh) * cpd];
-    const int64_t n_sinks = p1 - p0;
-    // work items: every sink pencil in tiles of 64 sinks (the reference block)
-    std::vector<Item> items;
-    items.reserve((size_t)d.nsinksets * 2);
-    auto count = [&](int s, int y, int z) {
-        return cnt[((int64_t)s * cpd + wrapi(y, cpd)) * cpd + wrapi(z, cpd)];
-    };
-    for (int j = 0; j < jw; j++)
-        for (int k = 0; k < nk; k++) {
-            int y = t.jlow + j, zc = zcen(k);
-            // 2D: the primary cells of a pencil are contiguous in its sink
-            // stream, after g_lo ghost sinks; only they are swept (the
-            // reference truncates sink pencils the same way,
-            // PencilPlan.cc:110-116)
-            int64_t np_ = 0, g_lo = 0;
-            bool seen_primary = false;
-            for (int a = -R; a <= R; a++) {
-                if (primary(zc + a)) {
-                    np_ += count(R, y, zc + a);
-                    seen_primary = true;
-                } else if (!seen_primary) {
-                    g_lo += count(R, y, zc + a);
-                }
-            }
-            if (np_ != d.sink_set_count[j * nk + k]) {
-                set_error("nf_sic_execute: SinkSetCount disagrees with the source plans");
+    const int step = two_d ? 1 : cpd;  // cells of a unit
+    for (int s = 0; s < W; s++) {
+        const float *slab = d.source_pos_slab[s];
+        const uint64_t ns = d.source_nslab[s];
+        int64_t run_src = 0, run_dst = 0, run_n = 0;
+        auto flush = [&]() {
+            if (run_n == 0) return;
+            memcpy(hx + run_dst, slab + run_src, run_n * sizeof(float));
+            memcpy(hy + run_dst, slab + ns + run_src, run_n * sizeof(float));
+            memcpy(hz + run_dst, slab + 2 * ns + run_src, run_n * sizeof(float));
+        };
+        const int64_t c_end = (int64_t)(s + 1) * cpd * cpd;
+        for (int64_t c = (int64_t)s * cpd * cpd; c < c_end; c += step) {
+            const int64_t dst = b.cs[c], n = b.cs[c + step] - dst;
+            if (n == 0) continue;
+            const int64_t src = two_d ? b.cellstart[c] : b.rowstart[c / cpd];
+            if (src < 0 || (uint64_t)(src + n) > ns) {
+                set_error(two_d ? "nf_sic_execute: source cell outside its slab"
+                                : "nf_sic_execute: source row outside its slab");
                 return NF_EINVAL;
             }
-            if (np_ == 0) continue;
-            int64_t M = 0;
-            for (int dx = -R; dx <= R; dx++)
-                for (int dy = -R; dy <= R; dy++) M += count(R + dx, y + dy, zc);
-            int pencil = (int)(((int64_t)R * cpd + y) * cpd + zc);
-            for (int64_t b0 = 0; b0 < np_; b0 += NFBLOCK) {
-                int take = (int)std::min<int64_t>(NFBLOCK, np_ - b0);
-                items.push_back(
-                    Item{pencil, (int)(g_lo + b0), take, take <= 32 ? 1 : 2, 0, (int)M, 0, 0});
+            if (run_n > 0 && src == run_src + run_n && dst == run_dst + run_n) {
+                run_n += n;
+            } else {
+                flush();
+                run_src = src;
+                run_dst = dst;
+                run_n = n;
             }
+        }
+        flush();
+    }
+    return NF_OK;
+}
+
+// Copy a SIC's records to AccSlab.  1D: rows [jlow, jhigh) are contiguous from
+// the first sink cell of row jlow, the centre cell of the row-jlow pencil
+// centred on z = 0.  2D: primary cells only, each at its AccSlab start (the
+// centre cell of the pencil centred on it); cells adjacent in both go as one
+// run.
+static nf_status store_records(nf_ctx *ctx, const SicBuffer &b, const SicTask &t, int64_t p0,
+                               int64_t n_sinks) {
+    const nf_sic_desc &d = t.d;
+    const int R = d.nfradius, W = 2 * R + 1, cpd = d.cpd, nk = d.nk;
+    const size_t rec = ctx->cfg.out_kind == NF_OUT_FLOAT4 ? 16 : 12;
+    if (d.node_z_size == 0) {
+        if (n_sinks <= 0) return NF_OK;
+        const int k0 = (cpd - R) % cpd;
+        const int64_t acc0 = d.sink_plan[(int64_t)k0 * W + R].start;
+        memcpy((char *)d.sink_acc_slab + acc0 * rec, b.h_out, (size_t)n_sinks * rec);
+        return NF_OK;
+    }
+    size_t run_acc = 0, run_out = 0, run_bytes = 0;
+    auto flush = [&]() {
+        if (run_bytes) memcpy((char *)d.sink_acc_slab + run_acc, (char *)b.h_out + run_out, run_bytes);
+        run_bytes = 0;
+    };
+    for (int j = 0; j < t.jhigh - t.jlow; j++)
+        for (int k = 0; k < nk; k++) {
+            const int y = t.jlow + j, zc = pencil_z(d, k);
+            if (!primary_z(d, zc)) continue;
+            const nf_cell_plan &ce = d.sink_plan[((int64_t)j * nk + k) * W + R];
+            const int64_t c = ((int64_t)R * cpd + y) * cpd + zc;
+            if (ce.n != b.cnt[c]) {
+                set_error("nf_sic_execute: sink plan and source plan disagree on a cell");
+                return NF_EINVAL;
+            }
+            if (ce.n == 0) continue;
+            const size_t acc = (size_t)ce.start * rec, out = (size_t)(b.cs[c] - p0) * rec;
+            const size_t bytes = (size_t)ce.n * rec;
+            if (run_bytes && acc == run_acc + run_bytes && out == run_out + run_bytes) {
+                run_bytes += bytes;
+            } else {
+                flush();
+                run_acc = acc;
+                run_out = out;
+                run_bytes = bytes;
+            }
+        }
+    flush();
+    return NF_OK;
+}
+
+// A SIC on the engine of nf_mutual.cu, every pair met one-sided: tiles are up
+// to 128 sinks and split until the launch is full.  Work list, cell table and
+// positions go over in one copy.
+static nf_status launch_list(nf_ctx *ctx, SicBuffer &b, const SicTask &t, Plan &pl, int64_t n_mini,
+                             uint64_t *bytes_to_device) {
+    const size_t items_b = b.list.size() * sizeof(MutualItem);
+    const size_t cs_b = (b.cs.size() * sizeof(int64_t) + 15) / 16 * 16, tables = items_b + cs_b;
+    const size_t n4 = ((size_t)n_mini + 3) / 4 * 4, bytes = tables + 3 * n4 * sizeof(float);
+    nf_status st = grow(ctx, b, n4, (size_t)pl.n_range, 0, 0, bytes);
+    if (st != NF_OK) return st;
+    char *h = (char *)b.h_block, *dev = (char *)b.d_block;
+    memcpy(h, b.list.data(), items_b);
+    memcpy(h + items_b, b.cs.data(), b.cs.size() * sizeof(int64_t));
+    float *hx = (float *)(h + tables);
+    st = stage_sources(b, t, hx, hx + n4, hx + 2 * n4);
+    if (st != NF_OK) return st;
+    cudaStream_t sm = b.stream;
+    NF_CUDA(cudaMemcpyAsync(dev, h, bytes, cudaMemcpyHostToDevice, sm));
+    st = mutual_unpack(ctx, pl, (const float *)(dev + tables), (int64_t)n4, b.d_pos, b.d_part,
+                       b.d_counters, sm);
+    if (st != NF_OK) return st;
+    pl.d_mutual = (MutualItem *)dev;
+    // a short list takes no more CTAs than it fills: the rest is for other SICs
+    pl.grid = (int)std::min<int64_t>(b.grid, (pl.n_mutual + ENGINE_WARPS_PER_CTA - 1) / ENGINE_WARPS_PER_CTA);
+    MutualLaunch L;
+    L.zeroed = true;
+    L.plan = &pl;
+    L.pos = b.d_pos;
+    L.cs = (const int64_t *)(dev + items_b);
+    L.cpd = t.d.cpd;
+    L.scratch = b.d_part;
+    L.counter = b.d_counters;
+    L.before = b.ev0;
+    st = mutual_launch(ctx, L, sm);
+    if (st != NF_OK) return st;
+    NF_CUDA(cudaEventRecord(b.ev1, sm));
+    *bytes_to_device = bytes;
+    // the records: written to pinned host memory by the co-add itself
+    return engine_coadd_plan(ctx, pl, b.d_part, b.pinned ? b.h_out : b.d_out, sm, 0.f, nullptr);
+}
+
+// A SIC on the one-sided engine of nf_box.cu (plain accumulation, softenings
+// below the other's fixed-point range): tiles of 64 sinks (the reference
+// block).
+static nf_status launch_tiles(nf_ctx *ctx, SicBuffer &b, const SicTask &t, int64_t n_mini, int64_t p0,
+                              int64_t n_sinks, uint64_t *bytes_to_device) {
+    const int cpd = t.d.cpd, R = t.d.nfradius;
+    std::vector<Item> items;
+    items.reserve(2 * b.pencils.size());
+    for (const SicPencil &p : b.pencils)
+        for (int64_t b0 = 0; b0 < p.n; b0 += NFBLOCK) {
+            const int take = (int)std::min<int64_t>(NFBLOCK, p.n - b0);
+            items.push_back(Item{(int)(((int64_t)R * cpd + p.y) * cpd + p.z), (int)(p.first + b0), take,
+                                 take <= 32 ? 1 : 2, 0, (int)p.sources, 0, 0});
         }
     // longest tiles first (the order of execution does not change any
     // result: every tile writes its own partials)
@@ -345,68 +439,20 @@ static nf_status run_task(nf_ctx *ctx, SicBuffer &b, const SicTask &t) {
         }
         launch_items.insert(launch_items.end(), keep.begin(), keep.end());
     }
-    nitems = launch_items.size();
-    st = grow(ctx, b, (size_t)n_mini, (size_t)n_sinks, nitems, (size_t)ncell + 1);
+    const size_t nitems = launch_items.size();
+    nf_status st = grow(ctx, b, (size_t)n_mini, (size_t)n_sinks, nitems, b.cs.size(), 0);
     if (st != NF_OK) return st;
-    // stage the source rows (each particle once) into pinned memory
     float *hx = b.h_raw, *hy = b.h_raw + b.cap_particles, *hz = b.h_raw + 2 * b.cap_particles;
-    for (int s = 0; s < W; s++) {
-        const float *slab = d.source_pos_slab[s];
-        const uint64_t ns = d.source_nslab[s];
-        // 2D: cell by cell (ghost cells included), cells that follow each
-        // other in both the slab and the mini box copied as one run
-        int64_t run_src = 0, run_dst = 0, run_n = 0;
-        auto flush = [&]() {
-            if (run_n == 0) return;
-            memcpy(hx + run_dst, slab + run_src, run_n * sizeof(float));
-            memcpy(hy + run_dst, slab + ns + run_src, run_n * sizeof(float));
-            memcpy(hz + run_dst, slab + 2 * ns + run_src, run_n * sizeof(float));
-            run_n = 0;
-        };
-        for (int y = 0; y < cpd && two_d; y++) {
-            if (!row_used[y]) continue;
-            for (int z = 0; z < cpd; z++) {
-                const int64_t c = ((int64_t)s * cpd + y) * cpd + z;
-                const int64_t n = cnt[c], src = cellstart[c], dst = cs[c];
-                if (n == 0) continue;
-                if (src < 0 || (uint64_t)(src + n) > ns) {
-                    set_error("nf_sic_execute: source cell outside its slab");
-                    return NF_EINVAL;
-                }
-                if (run_n > 0 && src == run_src + run_n && dst == run_dst + run_n) {
-                    run_n += n;
-                } else {
-                    flush();
-                    run_src = src;
-                    run_dst = dst;
-                    run_n = n;
-                }
-            }
-        }
-        flush();
-        for (int y = 0; y < cpd && !two_d; y++) {
-            if (!row_used[y]) continue;
-            int64_t dst = cs[((int64_t)s * cpd + y) * cpd];
-            int64_t n = cs[((int64_t)s * cpd + y + 1) * cpd] - dst;
-            if (n == 0) continue;
-            int64_t src = rowstart[s * cpd + y];
-            if (src < 0 || (uint64_t)(src + n) > ns) {
-                set_error("nf_sic_execute: source row outside its slab");
-                return NF_EINVAL;
-            }
-            memcpy(hx + dst, slab + src, n * sizeof(float));
-            memcpy(hy + dst, slab + ns + src, n * sizeof(float));
-            memcpy(hz + dst, slab + 2 * ns + src, n * sizeof(float));
-        }
-    }
-    memcpy(b.h_cs, cs.data(), cs.size() * sizeof(int64_t));
+    st = stage_sources(b, t, hx, hy, hz);
+    if (st != NF_OK) return st;
+    memcpy(b.h_cs, b.cs.data(), b.cs.size() * sizeof(int64_t));
     if (nitems) memcpy(b.h_items, launch_items.data(), nitems * sizeof(Item));
     cudaStream_t sm = b.stream;
-    size_t pb = (size_t)n_mini * sizeof(float);
+    const size_t pb = (size_t)n_mini * sizeof(float), cs_b = b.cs.size() * sizeof(int64_t);
     NF_CUDA(cudaMemcpyAsync(b.d_raw, hx, pb, cudaMemcpyHostToDevice, sm));
     NF_CUDA(cudaMemcpyAsync(b.d_raw + b.cap_particles, hy, pb, cudaMemcpyHostToDevice, sm));
     NF_CUDA(cudaMemcpyAsync(b.d_raw + 2 * b.cap_particles, hz, pb, cudaMemcpyHostToDevice, sm));
-    NF_CUDA(cudaMemcpyAsync(b.d_cs, b.h_cs, cs.size() * sizeof(int64_t), cudaMemcpyHostToDevice, sm));
+    NF_CUDA(cudaMemcpyAsync(b.d_cs, b.h_cs, cs_b, cudaMemcpyHostToDevice, sm));
     if (nitems)
         NF_CUDA(cudaMemcpyAsync(b.d_items, b.h_items, nitems * sizeof(Item), cudaMemcpyHostToDevice, sm));
     st = engine_pack(ctx, b.d_raw, b.d_raw + b.cap_particles, b.d_raw + 2 * b.cap_particles, n_mini,
@@ -429,55 +475,103 @@ static nf_status run_task(nf_ctx *ctx, SicBuffer &b, const SicTask &t) {
     st = engine_launch(ctx, L, 1.0 / cpd, sm);
     if (st != NF_OK) return st;
     NF_CUDA(cudaEventRecord(b.ev1, sm));
-    st = engine_coadd(ctx, b.d_part, n_sinks, b.d_out, sm);
+    *bytes_to_device = 3 * pb + cs_b + nitems * sizeof(Item);
+    return engine_coadd(ctx, b.d_part, n_sinks, b.d_out, sm);
+}
+
+static nf_status run_task(nf_ctx *ctx, SicBuffer &b, const SicTask &t) {
+    const nf_sic_desc &d = t.d;
+    nf_status st = check_desc(ctx, d, t.jlow, t.jhigh);
+    if (st != NF_OK) return st;
+    NF_CUDA(cudaSetDevice(b.device));
+    const int R = d.nfradius, W = 2 * R + 1, cpd = d.cpd, nk = d.nk;
+    const int jw = t.jhigh - t.jlow, nrows = jw + 2 * R;
+    const int64_t ncell = (int64_t)W * cpd * cpd;
+    const bool two_d = d.node_z_size > 0;
+    // cell counts of the mini box: slot s = source slab x-R+s, rows of the SIC
+    std::vector<int64_t> &cnt = b.cnt, &cs = b.cs;
+    cnt.assign(ncell, 0);
+    b.rowstart.assign(W * cpd, -1);
+    if (two_d) b.cellstart.assign(ncell, -1);
+    for (int r = 0; r < nrows; r++) {
+        const int y = wrapi(t.jlow - R + r, cpd);
+        for (int k = 0; k < nk; k++) {
+            const int z = pencil_z(d, k);
+            const nf_cell_plan *pl = d.source_plan + ((int64_t)r * nk + k) * W;
+            for (int s = 0; s < W; s++) {
+                if (pl[s].n < 0) {
+                    set_error("nf_sic_execute: negative cell count");
+                    return NF_EINVAL;
+                }
+                const int64_t c = ((int64_t)s * cpd + y) * cpd + z;
+                cnt[c] = pl[s].n;
+                if (two_d) b.cellstart[c] = pl[s].start;
+                else if (z == 0) b.rowstart[s * cpd + y] = pl[s].start;
+            }
+        }
+    }
+    // dense mirror offsets (linear cell order)
+    cs.resize(ncell + 1);
+    cs[0] = 0;
+    for (int64_t c = 0; c < ncell; c++) cs[c + 1] = cs[c] + cnt[c];
+    const int64_t n_mini = cs[ncell];
+    const int64_t p0 = cs[((int64_t)R * cpd + t.jlow) * cpd];
+    const int64_t p1 = cs[((int64_t)R * cpd + t.jhigh) * cpd];
+    const int64_t n_sinks = p1 - p0;
+    // sink pencils, checked against the descriptor
+    auto count = [&](int s, int y, int z) {
+        return cnt[((int64_t)s * cpd + wrapi(y, cpd)) * cpd + wrapi(z, cpd)];
+    };
+    b.pencils.clear();
+    for (int j = 0; j < jw; j++)
+        for (int k = 0; k < nk; k++) {
+            SicPencil p{t.jlow + j, pencil_z(d, k), 0, 0, 0};
+            // 2D: the primary cells of a pencil are contiguous in its sink
+            // stream, after `first` ghost sinks; only they are swept (the
+            // reference truncates sink pencils the same way,
+            // PencilPlan.cc:110-116)
+            bool seen_primary = false;
+            for (int a = -R; a <= R; a++) {
+                if (primary_z(d, p.z + a)) {
+                    p.n += count(R, p.y, p.z + a);
+                    seen_primary = true;
+                } else if (!seen_primary) {
+                    p.first += count(R, p.y, p.z + a);
+                }
+            }
+            if (p.n != d.sink_set_count[j * nk + k]) {
+                set_error("nf_sic_execute: SinkSetCount disagrees with the source plans");
+                return NF_EINVAL;
+            }
+            if (p.n == 0) continue;
+            for (int dx = -R; dx <= R; dx++)
+                for (int dy = -R; dy <= R; dy++) p.sources += count(R + dx, p.y + dy, p.z);
+            b.pencils.push_back(p);
+        }
+    uint64_t pairs = 0, to_device = 0;
+    for (const SicPencil &p : b.pencils) pairs += (uint64_t)p.n * (uint64_t)p.sources;
+    if (!b.grid) b.grid = mutual_grid(ctx, 0);
+    Plan pl;
+    pl.p0 = p0;
+    pl.n_range = n_sinks;
+    const bool listed =
+        mutual_sic_list(ctx->cfg, cpd, b.pencils, cs.data(), b.grid * ENGINE_WARPS_PER_CTA, pl, b.list);
+    if (listed)
+        st = launch_list(ctx, b, t, pl, n_mini, &to_device);
+    else
+        st = launch_tiles(ctx, b, t, n_mini, p0, n_sinks, &to_device);
     if (st != NF_OK) return st;
     const size_t rec = ctx->cfg.out_kind == NF_OUT_FLOAT4 ? 16 : 12;
-    NF_CUDA(cudaMemcpyAsync(b.h_out, b.d_out, (size_t)n_sinks * rec, cudaMemcpyDeviceToHost, sm));
+    cudaStream_t sm = b.stream;
+    if (n_sinks && !(listed && b.pinned))
+        NF_CUDA(cudaMemcpyAsync(b.h_out, b.d_out, (size_t)n_sinks * rec, cudaMemcpyDeviceToHost, sm));
     NF_CUDA(cudaStreamSynchronize(sm));
     float kms = 0.f;
     NF_CUDA(cudaEventElapsedTime(&kms, b.ev0, b.ev1));
-    sic_account(ctx, kms, items_pairs(items));
-    if (two_d) {
-        // primary cells only, each at its AccSlab start (the centre cell of
-        // the pencil centred on it); cells adjacent in both go as one run
-        size_t run_acc = 0, run_out = 0, run_bytes = 0;
-        auto flush = [&]() {
-            if (run_bytes)
-                memcpy((char *)d.sink_acc_slab + run_acc, (char *)b.h_out + run_out, run_bytes);
-            run_bytes = 0;
-        };
-        for (int j = 0; j < jw; j++)
-            for (int k = 0; k < nk; k++) {
-                const int y = t.jlow + j, zc = zcen(k);
-                if (!primary(zc)) continue;
-                const nf_cell_plan &ce = d.sink_plan[((int64_t)j * nk + k) * W + R];
-                const int64_t c = ((int64_t)R * cpd + y) * cpd + zc;
-                if (ce.n != cnt[c]) {
-                    set_error("nf_sic_execute: sink plan and source plan disagree on a cell");
-                    return NF_EINVAL;
-                }
-                if (ce.n == 0) continue;
-                const size_t acc = (size_t)ce.start * rec, out = (size_t)(cs[c] - p0) * rec;
-                const size_t bytes = (size_t)ce.n * rec;
-                if (run_bytes && acc == run_acc + run_bytes && out == run_out + run_bytes) {
-                    run_bytes += bytes;
-                } else {
-                    flush();
-                    run_acc = acc;
-                    run_out = out;
-                    run_bytes = bytes;
-                }
-            }
-        flush();
-    } else if (n_sinks > 0) {
-        // AccSlab rows [jlow, jhigh) are contiguous from the first sink cell of row jlow
-        // the centre cell of the row-jlow pencil centred on z = 0 is cell (jlow, 0)
-        int k0 = (cpd - R) % cpd;
-        int64_t acc0 = d.sink_plan[(int64_t)k0 * W + R].start;
-        memcpy((char *)d.sink_acc_slab + acc0 * rec, b.h_out, (size_t)n_sinks * rec);
-    }
-    if (d.bytes_to_device)
-        *d.bytes_to_device += 3 * pb + cs.size() * sizeof(int64_t) + nitems * sizeof(Item);
+    sic_account(ctx, kms, pairs);
+    st = store_records(ctx, b, t, p0, n_sinks);
+    if (st != NF_OK) return st;
+    if (d.bytes_to_device) *d.bytes_to_device += to_device;
     if (d.bytes_from_device) *d.bytes_from_device += (size_t)n_sinks * rec;
     return NF_OK;
 }
