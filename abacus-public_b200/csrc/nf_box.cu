@@ -989,11 +989,15 @@ nf_status engine_launch(nf_ctx *ctx, const EngineLaunch &L, double, cudaStream_t
     return NF_OK;
 }
 
+static int coadd_blocks(const nf_ctx *ctx, int64_t n) {
+    return (int)std::min<int64_t>((int64_t)ctx->sms * 8, (n + 255) / 256);
+}
+
 nf_status engine_coadd(nf_ctx *ctx, const Partial *part, int64_t n, void *out, cudaStream_t st,
                        float eps, const uint32_t *perm, int64_t p0) {
     if (n <= 0) return NF_OK;
     const nf_config &cfg = ctx->cfg;
-    coadd_kernel<<<ctx->sms * 8, 256, 0, st>>>(sums_view(cfg, part, n, eps), cfg.out_kind, out, perm,
+    coadd_kernel<<<coadd_blocks(ctx, n), 256, 0, st>>>(sums_view(cfg, part, n, eps), cfg.out_kind, out, perm,
                                               p0);
     NF_CUDA(cudaGetLastError());
     return NF_OK;
@@ -1003,7 +1007,7 @@ nf_status engine_coadd_plan(nf_ctx *ctx, const Plan &pl, const void *scratch, vo
                             cudaStream_t st, float eps, const uint32_t *perm) {
     if (pl.n_range <= 0) return NF_OK;
     const nf_config &cfg = ctx->cfg;
-    coadd_kernel<<<ctx->sms * 8, 256, 0, st>>>(sums_view(cfg, pl, scratch, eps), cfg.out_kind, out,
+    coadd_kernel<<<coadd_blocks(ctx, pl.n_range), 256, 0, st>>>(sums_view(cfg, pl, scratch, eps), cfg.out_kind, out,
                                               perm, pl.p0);
     NF_CUDA(cudaGetLastError());
     return NF_OK;
@@ -1737,7 +1741,8 @@ constexpr size_t NOALLOC_COUNTER_BYTES = 256;
 static_assert(NOALLOC_COUNTER_BYTES + (size_t)MAXW * 4 * sizeof(Partial) * NOALLOC_MAX_SINKS <=
                   NOALLOC_SCRATCH_BYTES,
               "scratch holds (2R+1) x 4 pencil partials per sink");
-// [0, 256): work counters; then (2R+1) x nc x n pencil partials.
+// [0, 256): work counters and particle bounds; then the sums: fixed point, or
+// (2R+1) x nc x n pencil partials.
 static __device__ __align__(256) unsigned char g_noalloc_scratch[NOALLOC_SCRATCH_BYTES];
 
 // Warps take whole pencils from a counter and run their tiles in order.
@@ -1829,12 +1834,18 @@ extern "C" nf_status nf_forces_noalloc(const nf_config *cfg, int cpd, const void
         }
         base = g_noalloc_base[dev];
     }
+    nf_ctx tmp;  // parameters only; no stream, event or memory of its own
+    tmp.cfg = *cfg;
+    tmp.device = dev;
+    NF_CUDA(cudaDeviceGetAttribute(&tmp.sms, cudaDevAttrMultiProcessorCount, dev));
+    char *const sums = (char *)base + NOALLOC_COUNTER_BYTES;
+    int64_t *const d_bounds = (int64_t *)((char *)base + NOALLOC_COUNTER_BYTES / 2);
+    nf_status bst = mutual_noalloc_begin(tmp.sms, *cfg, cpd, cell_start, slab_lo, slab_hi,
+                                         NOALLOC_MAX_SINKS, sums, (int *)base, d_bounds, st);
+    if (bst != NF_OK) return bst;
     const int64_t c2 = (int64_t)cpd * cpd;
-    int64_t bounds[2] = {0, 0};
-    NF_CUDA(cudaMemcpyAsync(&bounds[0], cell_start + slab_lo * c2, sizeof(int64_t),
-                            cudaMemcpyDeviceToHost, st));
-    NF_CUDA(cudaMemcpyAsync(&bounds[1], cell_start + slab_hi * c2, sizeof(int64_t),
-                            cudaMemcpyDeviceToHost, st));
+    int64_t bounds[3] = {0, 0, 0};
+    NF_CUDA(cudaMemcpyAsync(bounds, d_bounds, sizeof(bounds), cudaMemcpyDeviceToHost, st));
     NF_CUDA(cudaStreamSynchronize(st));
     const int64_t n = bounds[1] - bounds[0];
     if (n < 0 || n > NOALLOC_MAX_SINKS) {
@@ -1843,10 +1854,24 @@ extern "C" nf_status nf_forces_noalloc(const nf_config *cfg, int cpd, const void
         return NF_EINVAL;
     }
     if (n == 0) return NF_OK;
-    nf_ctx tmp;  // parameters only; no stream, event or memory of its own
-    tmp.cfg = *cfg;
-    tmp.device = dev;
-    NF_CUDA(cudaDeviceGetAttribute(&tmp.sms, cudaDevAttrMultiProcessorCount, dev));
+    {
+        Plan pl;
+        pl.lo = slab_lo;
+        pl.hi = slab_hi;
+        pl.p0 = bounds[0];
+        pl.n_range = n;
+        MutualLaunch L;
+        L.plan = &pl;
+        L.pos = (const float4 *)pos;
+        L.cs = cell_start;
+        L.cpd = cpd;
+        L.scratch = sums;
+        L.counter = (int *)base;
+        bool done = false;
+        nf_status mst = mutual_noalloc(dev, tmp.sms, *cfg, L, pl, bounds[2], &done, st);
+        if (mst == NF_OK && done) mst = engine_coadd_plan(&tmp, pl, sums, out, st, 0.f, nullptr);
+        if (mst != NF_OK || done) return mst;
+    }
     NF_CUDA(cudaMemsetAsync(base, 0, NOALLOC_COUNTER_BYTES, st));
     EngineLaunch L;
     L.pos = (const float4 *)pos;

@@ -117,6 +117,11 @@ struct MutualLaunch {
 constexpr int MUTUAL_SHAPES = 5;  // kernel shapes the autotuner chooses among
 const char *mutual_shape_name(int v);
 int mutual_grid(nf_ctx *ctx, int variant);
+nf_status mutual_noalloc_begin(int sms, const nf_config &cfg, int cpd, const int64_t *cs, int lo, int hi,
+                               int64_t max_n, void *acc, int *counters, int64_t *bounds,
+                               cudaStream_t st);
+nf_status mutual_noalloc(int dev, int sms, const nf_config &cfg, const MutualLaunch &L, Plan &pl,
+                         int64_t np_total, bool *done, cudaStream_t st);
 // A SIC's positions (x, y, z of n4 each, a multiple of four, 16-byte aligned)
 // to float4 records; zeroes scratch and counter.
 nf_status mutual_unpack(nf_ctx *ctx, const Plan &pl, const float *xyz, int64_t n4, float4 *pos,

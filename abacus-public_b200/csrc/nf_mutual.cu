@@ -48,8 +48,9 @@
 //
 // Work list.  Built on the device: tiles cut into pieces of bounded cost
 // along their chunks (any piece adds its own sums: no combining), ordered by
-// cost class, longest first, taken by warps from a counter.
+// sinks per lane and cost, taken by warps from a counter.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 
@@ -68,7 +69,7 @@ constexpr int GROUP = 32;
 constexpr int WPC = ENGINE_WARPS_PER_CTA;
 constexpr int FOLD = 2;    // chunks between folds of the FP32 partials
 constexpr int DENSE_CELL = 192;
-constexpr int NCLASS = 64;  // cost classes of the work list, four per octave
+constexpr int NCLASS = 64;  // classes of the work list: sinks per lane x octave of cost
 
 // What a pencil's stream of sources consists of, in stream order: mutual
 // columns [0, Ms), the centre cell [Ms, Ms + own), one-sided columns up to M.
@@ -181,9 +182,22 @@ struct PlanArgs {
     MutualItem *items;
 };
 
-__device__ __forceinline__ int cost_class(long long cost) {  // 0 = longest (2^25.75 or more)
-    const int c = (int)(4.f * log2f((float)max(cost, 1LL)));
-    return min(max(103 - c, 0), NCLASS - 1);
+// Order of the list: tiles of one S together, longest first within them.
+// Warps that run at the same time then run the same loops (an unrolled loop
+// is 3-6 KB of code; with S mixed by cost alone, clustered 128^3 took 8.2 ms
+// in the unroll-8 shape instead of 6.9, clustered 60^3 0.81 instead of 0.76).
+__device__ __forceinline__ int cost_class(int S, long long cost) {
+    const int octave = 31 - __clz((int)min(max(cost, 1LL), 1LL << 24));  // 2^10 .. 2^24 told apart
+    return (S >= 8 ? 0 : S == 4 ? 16 : S == 2 ? 32 : 48) + min(max(24 - octave, 0), 15);
+}
+
+// Pieces of a tile: none above `cap`, in proportion for tiles of few sinks,
+// which come last; at least four chunks each.
+__host__ __device__ __forceinline__ int tile_pieces(int S, int chunks, long long cost, long long cap) {
+    if (S < 4) cap = cap * S / 4;
+    const long long want = cap > 0 ? (cost + cap - 1) / cap : chunks, most = chunks / 4;
+    const long long n = want < most ? want : most;
+    return n > 1 ? (int)n : 1;
 }
 
 // Sinks per lane of the next tile of a pencil with `rem` sinks left: the
@@ -288,8 +302,8 @@ __global__ void plan_kernel(PlanArgs p) {
                 cost += c + tile_cost(S);
                 continue;
             }
-            const int pieces = max(1, (int)min((long long)(chunks / 4), (c + p.cap - 1) / p.cap));
-            const int cl = cost_class(c / pieces);
+            const int pieces = tile_pieces(S, chunks, c, p.cap);
+            const int cl = cost_class(S, c / pieces);
             if (PASS == 1) {
                 atomicAdd(&s_hist[cl], (unsigned)pieces);
             } else {
@@ -442,7 +456,7 @@ struct Sinks {
     static constexpr int N = S >= 2 ? S / 2 : 1;
     float2 x[N], y[N], z[N];     // positions (S == 1: .x only)
     float2 px[N], py[N], pz[N];  // FP32 partials
-    float2 w[N];                 // density
+    float2 w[N];                 // density, FP32 partials
 };
 
 struct Reaction {
@@ -599,7 +613,7 @@ __device__ void run_item(const MParams &kp, WarpSmem &ws, float4 *hl, const Mutu
     for (int q = 0; q < N; q++) {
         k.px[q] = k.py[q] = k.pz[q] = k.w[q] = zero;
 #pragma unroll
-        for (int c = 0; c < 3; c++) hl[(c * N + q) * 32] = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int c = 0; c < (DENS ? 4 : 3); c++) hl[(c * N + q) * 32] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
     own_tile(s, ws.spre, R, it.sink_begin, it.sink_begin + it.nsink);
     unsigned loaded = s.present;
@@ -642,6 +656,7 @@ __device__ void run_item(const MParams &kp, WarpSmem &ws, float4 *hl, const Mutu
             fold_smem(hl[q * 32], k.px[q]);
             fold_smem(hl[(N + q) * 32], k.py[q]);
             fold_smem(hl[(2 * N + q) * 32], k.pz[q]);
+            if (DENS) fold_smem(hl[(3 * N + q) * 32], k.w[q]);
         }
     };
     // drop-in SICs fold every chunk (+1 %): their long one-sided streams, split
@@ -749,7 +764,11 @@ __device__ void run_item(const MParams &kp, WarpSmem &ws, float4 *hl, const Mutu
         add_fixed(o, __float2ll_rn(hx * f) + __float2ll_rn(lx * f));
         add_fixed(o + kp.n_range, __float2ll_rn(hy * f) + __float2ll_rn(ly * f));
         add_fixed(o + 2 * kp.n_range, __float2ll_rn(hz * f) + __float2ll_rn(lz * f));
-        if (DENS) add_fixed(o + 3 * kp.n_range, __float2ll_rn((odd ? k.w[q].y : k.w[q].x) * kp.wscale));
+        if (DENS) {
+            const float4 vw = hl[(3 * N + q) * 32];
+            add_fixed(o + 3 * kp.n_range, __float2ll_rn((odd ? vw.y : vw.x) * kp.wscale) +
+                                              __float2ll_rn((odd ? vw.w : vw.z) * kp.wscale));
+        }
         if (!finite3(hx, hy, hz)) kp.bad[idx] = 1;
     }
 }
@@ -768,7 +787,7 @@ __global__ void __launch_bounds__(WPC * 32, MINB) mutual_kernel(const __grid_con
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     WarpSmem &ws = reinterpret_cast<WarpSmem *>(smem_raw)[warp];
     float4 *hl = reinterpret_cast<float4 *>(smem_raw + sizeof(WarpSmem) * WPC) +
-                 warp * (3 * (SMAX / 2) * 32) + lane;
+                 warp * ((DENS ? 4 : 3) * (SMAX / 2) * 32) + lane;
     for (;;) {
         int i = 0;
         if (lane == 0) i = atomicAdd(kp.counter, 1);
@@ -785,6 +804,65 @@ __global__ void __launch_bounds__(WPC * 32, MINB) mutual_kernel(const __grid_con
             run_item<SOFT, DENS, 4, UNR>(kp, ws, hl, it, lane, s, nm);
         else
             run_item<SOFT, DENS, (SMAX >= 8 ? 8 : 4), UNR>(kp, ws, hl, it, lane, s, nm);
+    }
+}
+
+// The sweep without a work list (allocation-free entry point): warps take
+// (pencil, piece) pairs from the counter; a piece is every pieces-th part of
+// each of the pencil's tiles.
+template <int SOFT, bool DENS>
+__global__ void __launch_bounds__(WPC * 32, 2)
+    mutual_noalloc_kernel(const __grid_constant__ MParams kp, int pencil0, int n_pencils, int pieces) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    WarpSmem &ws = reinterpret_cast<WarpSmem *>(smem_raw)[warp];
+    float4 *hl = reinterpret_cast<float4 *>(smem_raw + sizeof(WarpSmem) * WPC) + warp * ((DENS ? 4 : 3) * 2 * 32) + lane;
+    const int W = 2 * kp.g.R + 1;
+    for (;;) {
+        int q = 0;
+        if (lane == 0) q = atomicAdd(kp.counter, 1);
+        q = __shfl_sync(FULL, q, 0);
+        if (q >= n_pencils * pieces) break;
+        const int piece = q % pieces;
+        MutualItem it{pencil0 + q / pieces, 0, 0, 0, 0, 0, 0, 0};
+        Stream s;
+        const int nm = setup_tables(kp, it.pencil, ws, lane, s);
+        const int np = ws.spre[W];
+        while (it.sink_begin < np) {
+            it.S = tile_S(np - it.sink_begin, 4, 0);
+            it.nsink = min(np - it.sink_begin, 32 * it.S);
+            own_tile(s, ws.spre, kp.g.R, it.sink_begin, it.sink_begin + it.nsink);
+            int chunks = 0;
+            for (int i = 0; i < NSEG; i++) {
+                Seg sg;
+                if (segment(s, kp.g.R, i, sg)) chunks += (sg.e - sg.b + CHUNK - 1) / CHUNK;
+            }
+            it.c0 = (int)((int64_t)chunks * piece / pieces);
+            it.c1 = (int)((int64_t)chunks * (piece + 1) / pieces);
+            if (it.c0 < it.c1) {
+                if (it.S == 1)
+                    run_item<SOFT, DENS, 1, 4>(kp, ws, hl, it, lane, s, nm);
+                else if (it.S == 2)
+                    run_item<SOFT, DENS, 2, 4>(kp, ws, hl, it, lane, s, nm);
+                else
+                    run_item<SOFT, DENS, 4, 4>(kp, ws, hl, it, lane, s, nm);
+            }
+            it.sink_begin += it.nsink;
+        }
+    }
+}
+
+typedef void (*NoallocFn)(MParams, int, int, int);
+
+NoallocFn noalloc_fn(int soft, bool dens) {
+    switch (soft) {
+    case SOFT_PLUMMER: return dens ? mutual_noalloc_kernel<SOFT_PLUMMER, true> : mutual_noalloc_kernel<SOFT_PLUMMER, false>;
+    case SOFT_SINGLE_SPLINE:
+        return dens ? mutual_noalloc_kernel<SOFT_SINGLE_SPLINE, true> : mutual_noalloc_kernel<SOFT_SINGLE_SPLINE, false>;
+    case SOFT_CUBIC_SPLINE:
+        return dens ? mutual_noalloc_kernel<SOFT_CUBIC_SPLINE, true> : mutual_noalloc_kernel<SOFT_CUBIC_SPLINE, false>;
+    default:
+        return dens ? mutual_noalloc_kernel<SOFT_CUBIC_PLUMMER, true> : mutual_noalloc_kernel<SOFT_CUBIC_PLUMMER, false>;
     }
 }
 
@@ -840,7 +918,9 @@ int smax_of(const nf_config &cfg, int v) {
     return SHAPES[tunable(cfg.softening, cfg.b2 > 0.f) ? v : 0].smax;
 }
 
-size_t smem_bytes(int smax) { return (sizeof(WarpSmem) + 3 * (smax / 2) * 32 * sizeof(float4)) * WPC; }
+size_t smem_bytes(int smax, bool dens) {
+    return (sizeof(WarpSmem) + (dens ? 4 : 3) * (smax / 2) * 32 * sizeof(float4)) * WPC;
+}
 
 }  // namespace
 
@@ -884,7 +964,7 @@ const char *mutual_shape_name(int v) { return SHAPES[v].name; }
 
 int mutual_grid(nf_ctx *ctx, int variant) {
     MutualFn fn = pick(ctx->cfg.softening, ctx->cfg.b2 > 0.f, variant);
-    const size_t smem = smem_bytes(smax_of(ctx->cfg, variant));
+    const size_t smem = smem_bytes(smax_of(ctx->cfg, variant), ctx->cfg.b2 > 0.f);
     int per_sm = 0;
     if (cudaFuncSetAttribute((const void *)fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)smem) != cudaSuccess ||
@@ -935,13 +1015,16 @@ bool mutual_sic_list(const nf_config &cfg, int cpd, const std::vector<SicPencil>
     }
     if (!mutual_bits(cfg.softening, cfg.eps, cfg.b2, cpd, (double)W * max_sources, &pl.fbits, &pl.wbits))
         return false;
-    // pieces of bounded cost, longest first
-    const long long cap = std::max(1LL, total / ((long long)warps * 2));
+    // pieces of two warps' share: several SICs run side by side (driver over
+    // uniform 160^3: 31 ms, with one warp's share 36, clustered 96^3 9.0 and 10.1)
+    const long long cap = std::max(1LL, 2 * total / warps);
     for (Tile &t : tiles) {
-        t.pieces = (int)std::max(1LL, std::min((long long)(t.chunks / 4), (t.cost + cap - 1) / cap));
+        t.pieces = tile_pieces(t.it.S, t.chunks, t.cost, cap);
         t.cost /= t.pieces;
     }
-    std::sort(tiles.begin(), tiles.end(), [](const Tile &a, const Tile &b) { return a.cost > b.cost; });
+    std::sort(tiles.begin(), tiles.end(), [](const Tile &a, const Tile &b) {
+        return a.it.S != b.it.S ? a.it.S > b.it.S : a.cost > b.cost;
+    });
     items.clear();
     for (const Tile &t : tiles)
         for (int k = 0; k < t.pieces; k++) {
@@ -990,7 +1073,9 @@ nf_status mutual_plan(nf_ctx *ctx, const nf_box *box, int lo, int hi, int varian
     }
     pl.grid = mutual_grid(ctx, variant);
     pl.warps = pl.grid * WPC;
-    a.cap = std::max<long long>(1, (long long)(h.cost / ((unsigned long long)pl.warps * 6)));
+    // an eighth of a warp's share: 6, 12 and 20 parts were within 2 % on large
+    // sweeps, 3-6 % slower on ones of a millisecond
+    a.cap = std::max<long long>(1, (long long)(h.cost / ((unsigned long long)pl.warps * 8)));
     plan_kernel<1><<<blocks, 256, 0, st>>>(a);
     e = cudaMemcpyAsync(h.hist, a.sums->hist, sizeof(h.hist), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
@@ -1079,17 +1164,9 @@ nf_status mutual_unpack(nf_ctx *ctx, const Plan &pl, const float *xyz, int64_t n
     return NF_OK;
 }
 
-// Zero the sums (unless mutual_unpack has) and run the sweep of a plan.
-nf_status mutual_launch(nf_ctx *ctx, const MutualLaunch &L, cudaStream_t st) {
-    const nf_config &cfg = ctx->cfg;
+static MParams mutual_params(const nf_config &cfg, const MutualLaunch &L) {
     const Plan &pl = *L.plan;
     const int nc = cfg.b2 > 0.f ? 4 : 3;
-    if (!L.zeroed) {
-        zero_kernel<<<ctx->sms * 4, 256, 0, st>>>(zero_args(ctx, pl, L.scratch, L.counter));
-        NF_CUDA(cudaGetLastError());
-    }
-    if (L.before) NF_CUDA(cudaEventRecordWithFlags(L.before, st, L.event_flags));
-    if (pl.n_mutual == 0) return NF_OK;
     MParams kp;
     memset(&kp, 0, sizeof(kp));
     kp.pos = L.pos;
@@ -1107,10 +1184,97 @@ nf_status mutual_launch(nf_ctx *ctx, const MutualLaunch &L, cudaStream_t st) {
     kp.near_w = near_width(cfg, L.eps, L.cpd);
     for (int a = 0; a < 2 * kp.g.R + 1; a++)
         kp.zshift[a] = kp.xyshift[a] = (float)((a - kp.g.R) * (1.0 / (double)L.cpd));
+    return kp;
+}
+
+// Zero the sums (unless mutual_unpack has) and run the sweep of a plan.
+nf_status mutual_launch(nf_ctx *ctx, const MutualLaunch &L, cudaStream_t st) {
+    const nf_config &cfg = ctx->cfg;
+    const Plan &pl = *L.plan;
+    if (!L.zeroed) {
+        zero_kernel<<<ctx->sms * 4, 256, 0, st>>>(zero_args(ctx, pl, L.scratch, L.counter));
+        NF_CUDA(cudaGetLastError());
+    }
+    if (L.before) NF_CUDA(cudaEventRecordWithFlags(L.before, st, L.event_flags));
+    if (pl.n_mutual == 0) return NF_OK;
+    MParams kp = mutual_params(cfg, L);
     MutualFn fn = pick(cfg.softening, cfg.b2 > 0.f, pl.variant);
     void *args[] = {&kp};
     NF_CUDA(cudaLaunchKernel((const void *)fn, dim3(pl.grid), dim3(WPC * 32), args,
-                             smem_bytes(smax_of(cfg, pl.variant)), st));
+                             smem_bytes(smax_of(cfg, pl.variant), cfg.b2 > 0.f), st));
+    return NF_OK;
+}
+
+// First launch of an allocation-free call: the slab range's particle bounds and
+// the box's particle count to bounds[0..2], and, where the range fits max_n,
+// its sums and the counters zeroed.
+static __global__ void noalloc_begin_kernel(const int64_t *__restrict__ cs, int64_t c_lo, int64_t c_hi,
+                                            int64_t ncell, int64_t max_n, int bytes_per, uint4 *acc,
+                                            int *counters, int64_t *bounds) {
+    const int64_t p0 = cs[c_lo], p1 = cs[c_hi];
+    const int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i0 < 4) counters[i0] = 0;
+    if (i0 == 0) {
+        bounds[0] = p0;
+        bounds[1] = p1;
+        bounds[2] = cs[ncell];
+    }
+    if (p1 - p0 > max_n || p1 < p0) return;
+    // whole 16-byte words: the scratch is larger than any range's sums
+    const int64_t n16 = ((p1 - p0) * bytes_per + 15) / 16;
+    for (int64_t i = i0; i < n16; i += (int64_t)gridDim.x * blockDim.x) acc[i] = make_uint4(0, 0, 0, 0);
+}
+
+nf_status mutual_noalloc_begin(int sms, const nf_config &cfg, int cpd, const int64_t *cs, int lo, int hi,
+                               int64_t max_n, void *acc, int *counters, int64_t *bounds,
+                               cudaStream_t st) {
+    const int64_t c2 = (int64_t)cpd * cpd;
+    noalloc_begin_kernel<<<sms, 256, 0, st>>>(cs, lo * c2, hi * c2, c2 * cpd, max_n,
+                                              8 * (cfg.b2 > 0.f ? 4 : 3) + 1, (uint4 *)acc, counters, bounds);
+    NF_CUDA(cudaGetLastError());
+    return NF_OK;
+}
+
+// CTAs per SM of the allocation-free sweep, asked once per device and kernel.
+static nf_status noalloc_grid(int dev, int sms, const nf_config &cfg, int *grid) {
+    static std::atomic<int> per_sm[128][8];
+    const bool dens = cfg.b2 > 0.f;
+    std::atomic<int> &slot = per_sm[dev][2 * cfg.softening + dens];
+    int n = slot.load();
+    if (n == 0) {
+        const void *fn = (const void *)noalloc_fn(cfg.softening, dens);
+        NF_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes(4, cfg.b2 > 0.f)));
+        NF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, WPC * 32, smem_bytes(4, cfg.b2 > 0.f)));
+        n = std::max(n, 1);
+        slot.store(n);
+    }
+    *grid = sms * n;
+    return NF_OK;
+}
+
+// The sweep of an allocation-free call (after mutual_noalloc_begin): pl holds
+// the range; its units are set here.  *done stays false where the engine does
+// not apply.
+nf_status mutual_noalloc(int dev, int sms, const nf_config &cfg, const MutualLaunch &L, Plan &pl,
+                         int64_t np_total, bool *done, cudaStream_t st) {
+    *done = false;
+    if (cfg.accumulation != NF_ACC_COMPENSATED || np_total > INT32_MAX / 8 ||
+        !mutual_bits(cfg.softening, cfg.eps, cfg.b2, L.cpd, (double)np_total, &pl.fbits, &pl.wbits))
+        return NF_OK;
+    int grid = 0;
+    nf_status s = noalloc_grid(dev, sms, cfg, &grid);
+    if (s != NF_OK) return s;
+    MParams kp = mutual_params(cfg, L);
+    const int64_t c2 = (int64_t)L.cpd * L.cpd;
+    int pencil0 = (int)(pl.lo * c2), n_pencils = (int)((pl.hi - pl.lo) * c2);
+    // few pencils are cut into pieces, two a warp
+    int pieces = (int)std::max<int64_t>(1, std::min<int64_t>(8, 2 * (int64_t)grid * WPC / n_pencils));
+    if ((int64_t)n_pencils * pieces > INT32_MAX / 2) pieces = 1;
+    void *args[] = {&kp, &pencil0, &n_pencils, &pieces};
+    NF_CUDA(cudaLaunchKernel((const void *)noalloc_fn(cfg.softening, cfg.b2 > 0.f), dim3(grid),
+                             dim3(WPC * 32), args, smem_bytes(4, cfg.b2 > 0.f), st));
+    pl.mutual = true;
+    *done = true;
     return NF_OK;
 }
 

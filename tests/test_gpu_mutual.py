@@ -149,3 +149,42 @@ def test_bits_do_not_depend_on_the_order_of_the_work(capi, synth):
     for o in outs[1:]:
         for x, y in zip(o, outs[0]):
             assert np.array_equal(x.view(np.uint32), y.view(np.uint32))
+
+
+@pytest.mark.parametrize("soft,R,counts", [
+    (0, 2, "one"), (1, 2, "edges"), (1, 2, "dense"), (2, 1, "edges"), (3, 2, "edges"), (0, 1, "dense")])
+def test_allocation_free_sweep(capi, oracle, synth, soft, R, counts):
+    """nf_forces_noalloc cuts few pencils into pieces: one particle, pencils
+    around the tile sizes, a dense cell, whole boxes and slab ranges."""
+    import ctypes
+
+    import torch
+    cpd = 7
+    c = np.zeros((cpd, cpd, cpd), int)
+    if counts == "one":
+        c[2, 3, 4] = 1
+    elif counts == "edges":
+        c[:] = np.arange(cpd ** 3).reshape(c.shape) % 41
+        c[3, 3, :3] = 129, 64, 0
+    else:
+        c[3, 3, 3], c[3, 3, 4], c[4, 3, 3] = 700, 200, 33
+    box = _box(synth, cpd, c, seed=5)
+    eps = synth.kernel_eps(soft, 0.02 / cpd)
+    cfg = capi.default_config(softening=soft, eps=eps, near_field_radius=R)
+    pos = torch.zeros((box.n, 4), device="cuda")
+    for k, v in enumerate((box.x, box.y, box.z)):
+        pos[:, k] = torch.from_numpy(v).cuda()
+    cs = torch.from_numpy(box.cell_start).cuda()
+    for lo, hi in ((0, cpd), (2, 5), (3, 4), (6, 7)):
+        p0, p1 = int(box.cell_start[lo * cpd * cpd]), int(box.cell_start[hi * cpd * cpd])
+        out = torch.full((max(p1 - p0, 1), 4), float("nan"), device="cuda")
+        capi.check(capi.lib().nf_forces_noalloc(
+            ctypes.byref(cfg), cpd, pos.data_ptr(), cs.data_ptr(), lo, hi, out.data_ptr(),
+            ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
+        if p1 == p0:
+            continue
+        a = out[:p1 - p0].cpu().numpy()
+        if counts == "one":
+            assert np.all(a == 0)
+        else:
+            _check(oracle, box, soft, eps, a, R=R, first=p0)
