@@ -1021,9 +1021,10 @@ nf_status engine_pack(nf_ctx *ctx, const float *x, const float *y, const float *
     return NF_OK;
 }
 
-// The sweep of a plan into the box's scratch, between events 0 and 1.
+// The sweep of a plan into the box's scratch, or a mutual plan's into another,
+// between events 0 and 1.
 static nf_status enqueue_pencil(nf_ctx *ctx, nf_box *box, Plan &pl, cudaStream_t st,
-                                unsigned evflags) {
+                                unsigned evflags, void *scratch = nullptr) {
     if (pl.mutual) {
         MutualLaunch L;
         L.plan = &pl;
@@ -1031,7 +1032,7 @@ static nf_status enqueue_pencil(nf_ctx *ctx, nf_box *box, Plan &pl, cudaStream_t
         L.cs = box->d_cs;
         L.cpd = box->cpd;
         L.eps = box->eps;
-        L.scratch = box->d_part;
+        L.scratch = scratch ? scratch : box->d_part;
         L.counter = pl.d_counters;
         L.before = ctx->ev[0];
         L.event_flags = evflags;
@@ -1108,6 +1109,7 @@ using namespace nf;
 
 size_t nf_box::device_bytes() const {
     size_t b = (size_t)np * sizeof(float4) + cell_start.size() * sizeof(int64_t) + part_bytes +
+               part2_bytes +
                (d_stage ? 3 * (size_t)np * sizeof(float) : 0) + sort_bytes +
                (d_perm ? (size_t)np * sizeof(uint32_t) : 0);
     for (auto &kv : plans) {
@@ -1319,10 +1321,11 @@ extern "C" void nf_box_destroy(nf_ctx *ctx, nf_box *box) {
     if (ctx) lk = std::unique_lock<std::mutex>(ctx->mu);
     for (auto &kv : box->plans) free_plan(ctx, *kv.second);
     for (void *p : {(void *)box->d_pos, (void *)box->d_cs, (void *)box->d_part, (void *)box->d_stage,
-                    (void *)box->d_perm, box->d_sort})
+                    (void *)box->d_perm, box->d_sort, box->d_part2})
         pool_free(ctx, p);
     if (box->s_in) cudaStreamDestroy(box->s_in);
     if (box->s_out) cudaStreamDestroy(box->s_out);
+    if (box->s_sweep) cudaStreamDestroy(box->s_sweep);
     for (cudaEvent_t e : box->step_ev) cudaEventDestroy(e);
     delete box;
 }
@@ -1652,23 +1655,36 @@ extern "C" nf_status nf_box_step(nf_ctx *ctx, nf_box *box, const float *x, const
     if (ost != NF_OK) return ost;
     if (!box->s_in) NF_CUDA(cudaStreamCreateWithFlags(&box->s_in, cudaStreamNonBlocking));
     if (!box->s_out) NF_CUDA(cudaStreamCreateWithFlags(&box->s_out, cudaStreamNonBlocking));
-    while ((int)box->step_ev.size() < 2 * K + 2) {
+    // Chunks are swept on the context's stream and a second one in turn, each
+    // with its own sums: a chunk's CTAs start as the chunk before it drains
+    bool two = true;
+    for (Plan *pl : pls) two = two && pl->mutual;
+    if (two && box->part2_bytes < box->part_bytes) {
+        pool_free(ctx, box->d_part2);
+        box->d_part2 = nullptr;
+        box->part2_bytes = 0;
+        if (pool_alloc(ctx, &box->d_part2, box->part_bytes) == cudaSuccess) box->part2_bytes = box->part_bytes;
+        else two = false;
+    }
+    if (two && !box->s_sweep) NF_CUDA(cudaStreamCreateWithFlags(&box->s_sweep, cudaStreamNonBlocking));
+    while ((int)box->step_ev.size() < 2 * K + 3) {
         cudaEvent_t e;
         NF_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
         box->step_ev.push_back(e);
     }
     cudaEvent_t *ev_in = box->step_ev.data(), *ev_out = ev_in + K, ev_go = ev_in[2 * K],
-                ev_done = ev_in[2 * K + 1];
+                ev_done = ev_in[2 * K + 1], ev_two = ev_in[2 * K + 2];
     cudaStream_t sc = ctx->stream, si = box->s_in, so = box->s_out;
     const int64_t c2 = (int64_t)cpd * cpd, n = box->np;
     auto P = [&](int slab) { return box->cell_start[(int64_t)slab * c2]; };
     const size_t rec = ctx->cfg.out_kind == NF_OUT_FLOAT4 ? 16 : 12;
     float *tmp = box->d_stage;
-    // copies in on s_in, ordering and sweeps on the context stream, copies
-    // out on s_out; the context stream waits for both at the end
+    // copies in and ordering on s_in, sweeps on the context's stream and
+    // s_sweep, copies out on s_out; the context's stream waits for all at the end
     NF_CUDA(cudaEventRecord(ev_go, sc));
     NF_CUDA(cudaStreamWaitEvent(si, ev_go, 0));
     NF_CUDA(cudaStreamWaitEvent(so, ev_go, 0));
+    if (two) NF_CUDA(cudaStreamWaitEvent(box->s_sweep, ev_go, 0));
     for (int k = 0; k < K; k++) {
         const int64_t p0 = P(b[k]), m = P(b[k + 1]) - p0;
         if (m > 0) {
@@ -1677,30 +1693,31 @@ extern "C" nf_status nf_box_step(nf_ctx *ctx, nf_box *box, const float *x, const
             NF_CUDA(cudaMemcpyAsync(tmp + n + p0, y + p0, by, cudaMemcpyDefault, si));
             NF_CUDA(cudaMemcpyAsync(tmp + 2 * n + p0, z + p0, by, cudaMemcpyDefault, si));
         }
+        cudaError_t e = order_range(ctx, box, o, tmp, tmp + n, tmp + 2 * n, 1, p0, p0 + m, si);
+        if (e != cudaSuccess) return cuda_fail(e, "nf_box_step (ordering)");
         NF_CUDA(cudaEventRecord(ev_in[k], si));
     }
+    int turn = 0;
     auto sweep = [&](int k) -> nf_status {
-        // range k: its halo chunks are ordered already (stream order on sc)
-        nf_status st = run_sweep(ctx, box, *pls[k]);
-        if (st == NF_OK)
-            st = engine_coadd_plan(ctx, *pls[k], box->d_part, pls[k]->d_out, sc, box->eps, box->d_perm);
-        if (st != NF_OK) return st;
-        NF_CUDA(cudaEventRecord(ev_out[k], sc));
+        // s_in is in order: the last chunk of the range's halo is enough
+        const bool other = two && (turn++ & 1);
+        cudaStream_t st = other ? box->s_sweep : sc;
+        void *sums = other ? box->d_part2 : box->d_part;
+        NF_CUDA(cudaStreamWaitEvent(st, ev_in[k == 0 || k == K - 1 ? K - 1 : k + 1], 0));
+        nf_status s = enqueue_pencil(ctx, box, *pls[k], st, cudaEventRecordDefault, sums);
+        if (s == NF_OK) s = engine_coadd_plan(ctx, *pls[k], sums, pls[k]->d_out, st, box->eps, box->d_perm);
+        if (s != NF_OK) return s;
+        NF_CUDA(cudaEventRecord(ev_out[k], st));
         NF_CUDA(cudaStreamWaitEvent(so, ev_out[k], 0));
         if (pls[k]->out_bytes)
             NF_CUDA(cudaMemcpyAsync((char *)out + (size_t)(P(b[k]) - P(0)) * rec, pls[k]->d_out,
                                     pls[k]->out_bytes, cudaMemcpyDefault, so));
         return NF_OK;
     };
-    for (int k = 0; k < K; k++) {
-        NF_CUDA(cudaStreamWaitEvent(sc, ev_in[k], 0));
-        cudaError_t e = order_range(ctx, box, o, tmp, tmp + n, tmp + 2 * n, 1, P(b[k]),
-                                    P(b[k + 1]), sc);
-        if (e != cudaSuccess) return cuda_fail(e, "nf_box_step (ordering)");
-        if (k >= 2) {  // range k-1 has both halos: chunks k-2 and k
-            nf_status st = sweep(k - 1);
-            if (st != NF_OK) return st;
-        }
+    // range k needs chunks k-1 and k+1
+    for (int k = 1; k < K - 1; k++) {
+        nf_status st = sweep(k);
+        if (st != NF_OK) return st;
     }
     // the ranges next to the periodic wrap need the last chunk
     if (K >= 2) {
@@ -1709,6 +1726,10 @@ extern "C" nf_status nf_box_step(nf_ctx *ctx, nf_box *box, const float *x, const
     }
     nf_status st = sweep(0);
     if (st != NF_OK) return st;
+    if (two) {
+        NF_CUDA(cudaEventRecord(ev_two, box->s_sweep));
+        NF_CUDA(cudaStreamWaitEvent(sc, ev_two, 0));
+    }
     NF_CUDA(cudaEventRecord(ev_done, so));
     NF_CUDA(cudaStreamWaitEvent(sc, ev_done, 0));
     NF_CUDA(cudaStreamSynchronize(sc));
@@ -1719,7 +1740,8 @@ extern "C" nf_status nf_box_step(nf_ctx *ctx, nf_box *box, const float *x, const
     }
     ctx->last.pairs = pairs;
     ctx->last.padded_pairs = padded;
-    ctx->last.launches = 2 * K;
+    ctx->last.launches = K;
+    for (Plan *pl : pls) ctx->last.launches += sweep_launches(*pl);
     return NF_OK;
 }
 

@@ -181,6 +181,9 @@ struct nf_box {
     size_t sort_bytes = 0;
     // pipelined step (nf_box_step): copy-in and copy-out streams, per-chunk events
     cudaStream_t s_in = nullptr, s_out = nullptr;
+    cudaStream_t s_sweep = nullptr;   // every other chunk's sweep, with sums of its own
+    void *d_part2 = nullptr;
+    size_t part2_bytes = 0;
     std::vector<cudaEvent_t> step_ev;
     size_t part_bytes = 0;
     std::map<std::pair<int, int>, std::unique_ptr<nf::Plan>> plans;
