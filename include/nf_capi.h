@@ -476,8 +476,8 @@ nf_status nf_box_kick(nf_ctx *ctx, nf_box *box, int slab_lo, int slab_hi,
  * reference).  For callers that cannot call cudaMalloc -- code that runs
  * inside another framework's memory pool or caching allocator, or in a
  * process whose device allocations are fixed after start-up.  Nothing is
- * allocated on the device or the host: the scratch (pencil partials and a
- * work counter) is one 32 MiB static device array, held by every GPU that
+ * allocated on the device or the host: the scratch (the sums, work counters
+ * and particle bounds) is one 32 MiB static device array, held by every GPU that
  * loads this library until the process exits.
  *   pos        device float4 records (x, y, z, unused) in cell order
  *   cell_start device int64 prefix offsets, cpd^3 + 1 entries
@@ -489,8 +489,8 @@ nf_status nf_box_kick(nf_ctx *ctx, nf_box *box, int slab_lo, int slab_hi,
  * address with that device current; make that first call before any stream
  * capture.  All calls share the one array and it keeps the last call's
  * contents: calls that overlap on the GPU (other streams, other host
- * threads) race.  Every call first copies the slab range's two particle
- * bounds from cell_start to the host and synchronizes `stream` to read
+ * threads) race.  Every call first copies the slab range's particle bounds
+ * and the box's particle count to the host and synchronizes `stream` to read
  * them, so the host waits for all earlier work on `stream`; the sweep and
  * the co-add are then queued on `stream` and the call returns without
  * waiting for them. */
