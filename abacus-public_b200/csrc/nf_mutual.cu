@@ -6,9 +6,10 @@
 // belong to one particle; separation, r^2 and g are the same for the pair
 // seen from the other side.  Evaluating a pair once and accumulating it twice
 // costs 16 instructions for four interactions: 8 per two instead of 13.
-// Sweep times, one-sided -> mutual: uniform 64^3 0.922 -> 0.781 ms, clustered
-// 128^3 8.96 -> 7.02, clustered 256^3 119.1 -> 91.1 (2.75e12 pairs/s), density
-// 100^3 6.46 -> 4.36; 3.2e12 pairs/s where pencils hold thousands of sinks.
+// Sweep times, one-sided -> mutual (with the list ordered as below): uniform
+// 64^3 0.922 -> 0.768 ms, clustered 128^3 8.96 -> 6.87, clustered 256^3 119.1
+// -> 88.0 (2.8e12 pairs/s), density 100^3 6.46 -> 4.17; 3.2e12 pairs/s where
+// pencils hold thousands of sinks.
 // On clustered 256^3 the FMA pipe is busy 69 % (one instruction in three
 // reads three distinct register pairs and issues at 2/3 rate).  Of a warp's
 // time on uniform 160^3, 79 % is the mutual loop, 7 % the centre column
