@@ -180,7 +180,7 @@ __device__ __forceinline__ void chunk_scalar(const float4 *bxy, const float2 *bz
             float tz = bz[j + u].x;
             float dx = sx + t.x, dy = sy + t.z, dz = sz + tz;
             const float r2 = fmaf(dz, dz, fmaf(dy, dy, fmaf(dx, dx, r2_add<SOFT>(pc))));
-            const float g = pair_g<SOFT, NEAR>(r2, pc);
+            const float g = pair_g<SOFT, NEAR, Step::FULL>(r2, pc);
             px = fmaf(g, dx, px);
             py = fmaf(g, dy, py);
             pz = fmaf(g, dz, pz);
@@ -206,7 +206,7 @@ __device__ __forceinline__ void chunk_paired(const float4 *bxy, const float2 *bz
 #pragma unroll
             for (int q = 0; q < SP; q++) {
                 float2 dx = add2(sx[q], tx), dy = add2(sy[q], ty), dz = add2(sz[q], tz);
-                const float2 g = pair_g_x2<SOFT, NEAR>(r2_x2(dx, dy, dz, r2_add<SOFT>(pc)), pc);
+                const float2 g = pair_g_x2<SOFT, NEAR, Step::FULL>(r2_x2(dx, dy, dz, r2_add<SOFT>(pc)), pc);
                 px[q] = fma2(g, dx, px[q]);
                 py[q] = fma2(g, dy, py[q]);
                 pz[q] = fma2(g, dz, pz[q]);
@@ -896,7 +896,7 @@ static KParams params_from(nf_ctx *ctx, const EngineLaunch &L) {
     kp.n_range = L.n_range;
     kp.nc = cfg.b2 > 0.f ? 4 : 3;
     kp.plain = cfg.accumulation == NF_ACC_PLAIN;
-    kp.pc = pair_const(cfg, L.eps);
+    kp.pc = pair_const(cfg, L.eps, Step::FULL);
     kp.near_w = near_width(cfg, L.eps, L.cpd);
     double h = 1.0 / (double)L.cpd;
     for (int a = 0; a < 2 * R + 1; a++) {
@@ -925,18 +925,14 @@ static KParams make_params(nf_ctx *ctx, nf_box *box, const Plan &pl) {
     return params_from(ctx, L);
 }
 
-// Output scale of the co-add, formed in double on the host and rounded once
-// to float: out of the pair sums' unit, and for the single spline times
-// eps_int^3 (the raw kernel's units).
-// eps: the softening parameter in use (0: the context's).
-static double output_scale_exact(const nf_config &cfg, float eps) {
+// Output scale of the co-add, formed in double on the host: out of the pair
+// sums' unit, and for the single spline times eps_int^3 (the raw kernel's
+// units).  eps: the softening parameter in use (0: the context's).
+static double output_scale(const nf_config &cfg, float eps, Step step) {
     if (eps <= 0.f) eps = cfg.eps;
     const double eps3 =
         cfg.softening == SOFT_SINGLE_SPLINE ? pow((double)eps, -1.5) : 1.0;  // eps_int^3
-    return eps3 / pair_unit(cfg.softening);
-}
-static float output_scale(const nf_config &cfg, float eps = 0.f) {
-    return (float)output_scale_exact(cfg, eps);
+    return eps3 / pair_unit(cfg.softening, step);
 }
 
 static SumsView sums_view(const nf_config &cfg, const Partial *part, int64_t n, float eps) {
@@ -945,7 +941,7 @@ static SumsView sums_view(const nf_config &cfg, const Partial *part, int64_t n, 
     v.n = n;
     v.W = 2 * cfg.near_field_radius + 1;
     v.nc = cfg.b2 > 0.f ? 4 : 3;
-    v.scale = output_scale(cfg, eps);
+    v.scale = (float)output_scale(cfg, eps, Step::FULL);
     return v;
 }
 
@@ -954,7 +950,7 @@ static SumsView sums_view(const nf_config &cfg, const Plan &pl, const void *scra
     SumsView v = sums_view(cfg, nullptr, pl.n_range, eps);
     v.acc = (const unsigned long long *)scratch;
     v.bad = (const unsigned char *)scratch + (size_t)pl.n_range * 8 * v.nc;
-    v.scale = (float)std::ldexp(output_scale_exact(cfg, eps), -pl.fbits);
+    v.scale = (float)std::ldexp(output_scale(cfg, eps, Step::SHORT), -pl.fbits);
     v.wscale = (float)std::ldexp(1.0, -pl.wbits);
     return v;
 }

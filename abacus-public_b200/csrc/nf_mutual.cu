@@ -475,7 +475,7 @@ __device__ __forceinline__ void meet(const float4 &t, const float2 &tz, Sinks<S>
         if constexpr (S == 1) {
             const float dx = k.x[0].x + tx.x, dy = k.y[0].x + ty.x, dz = k.z[0].x + tz.x;
             const float r2 = fmaf(dz, dz, fmaf(dy, dy, fmaf(dx, dx, r2_add<SOFT>(pc))));
-            const float g = pair_g<SOFT, NEAR>(r2, pc);
+            const float g = pair_g<SOFT, NEAR, Step::SHORT>(r2, pc);
             k.px[0].x = fmaf(g, dx, k.px[0].x);
             k.py[0].x = fmaf(g, dy, k.py[0].x);
             k.pz[0].x = fmaf(g, dz, k.pz[0].x);
@@ -492,7 +492,7 @@ __device__ __forceinline__ void meet(const float4 &t, const float2 &tz, Sinks<S>
         } else {
             const float2 dx = add2(k.x[q], tx), dy = add2(k.y[q], ty), dz = add2(k.z[q], tz);
             const float2 r2 = r2_x2(dx, dy, dz, r2_add<SOFT>(pc));
-            const float2 g = pair_g_x2<SOFT, NEAR>(r2, pc);
+            const float2 g = pair_g_x2<SOFT, NEAR, Step::SHORT>(r2, pc);
             k.px[q] = fma2(g, dx, k.px[q]);
             k.py[q] = fma2(g, dy, k.py[q]);
             k.pz[q] = fma2(g, dz, k.pz[q]);
@@ -1181,7 +1181,7 @@ static MParams mutual_params(const nf_config &cfg, const MutualLaunch &L) {
     kp.n_range = pl.n_range;
     kp.fscale = (float)std::ldexp(1.0, pl.fbits);
     kp.wscale = (float)std::ldexp(1.0, pl.wbits);
-    kp.pc = pair_const(cfg, L.eps);
+    kp.pc = pair_const(cfg, L.eps, Step::SHORT);
     kp.near_w = near_width(cfg, L.eps, L.cpd);
     for (int a = 0; a < 2 * kp.g.R + 1; a++)
         kp.zshift[a] = kp.xyshift[a] = (float)((a - kp.g.R) * (1.0 / (double)L.cpd));

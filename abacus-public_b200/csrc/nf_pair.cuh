@@ -8,14 +8,17 @@
 //     Newton-Raphson step, applied to the cube:
 //       y = rsqrt(r2); q = r2*y^2 (1 up to the estimate's error)
 //       r2^-3/2 ~= y^3 * (1 - 1.5 (q - 1)) = y^3 * (q - 5/3) * (-3/2)
-//     The constant factor stays out of the pair: sums are accumulated in
-//     units of NEWTON_UNIT = 1 - float(5/3), and the co-add divides by it once
-//     per sink.  Four FP32 instructions instead of five with the step written
-//     as fma(y^3 * e, -1.5, y^3), and one three-operand FMA fewer.  Clustered
-//     256^3 sweep 123.4 -> 119.1 ms, uniform 64^3 (Plummer) 0.964 -> 0.922 ms;
-//     error against FP64 unchanged (uniform 64^3 2.7e-7, clustered 128^3
-//     2.8e-7): the step's own rounding is 4.6e-8 RMS a pair instead of
-//     3.8e-8, the sums' is above 2e-7.
+//     The one-sided engine writes the step as y^3 - 1.5 (q - 1) y^3, five
+//     instructions, 3.8e-8 RMS.  The mutual engine uses the product above,
+//     four instructions, 4.6e-8 RMS (q - 5/3 rounds to 2^-25 at 2/3), with
+//     the constant factor left out of the pair (Step::SHORT): sums are in
+//     units of NEWTON_UNIT = 1 - float(5/3), divided out once per sink.  Its
+//     64-bit sums are nearer to FP64 than the one-sided engine's compensated
+//     FP32 all the same (uniform boxes of 3000 and 20000 particles: 3.0e-7 and
+//     1.8e-7 beside 3.4e-7 and 2.6e-7), and the fifth instruction costs it
+//     3-4 % of a sweep (clustered 256^3 90.0 -> 93.3 ms, uniform 160^3
+//     12.1 -> 12.6) and 10 % of a single slab; the one-sided engine pays 1 %
+//     (uniform 160^3 15.75 -> 15.91 ms).
 //   * the single spline is accumulated in far units, g = f_ref / eps^3
 //     (r^-3 in the far branch), and the sum is multiplied by eps^3 once per
 //     sink.  Chunks of sources that hold none within the spline's reach of a
@@ -47,12 +50,26 @@ __device__ __forceinline__ float rsqrt_est(float x) {
 constexpr float NEWTON_K = 5.0f / 3.0f;
 constexpr double NEWTON_UNIT = 1.0 - (double)NEWTON_K;
 
-// NEWTON_UNIT * r2^-3/2 from the estimate plus one Newton step on the cube.
-__device__ __forceinline__ float inv_r3(float r2) {
-    float y = rsqrt_est(r2);
-    float y2 = y * y;
-    float c = fmaf(r2, y2, -NEWTON_K);
-    return (y2 * y) * c;
+// How the Newton step on the cube is written: in unit 1, or four instructions
+// in NEWTON_UNIT.
+enum class Step { FULL, SHORT };
+
+// y^3 with the step, from the estimate y of r2^-1/2.
+template <Step STEP>
+__device__ __forceinline__ float cube_step(float r2, float y) {
+    const float y2 = y * y;
+    const float y3 = y2 * y;
+    if constexpr (STEP == Step::SHORT) return y3 * fmaf(r2, y2, -NEWTON_K);
+    return fmaf(y3 * fmaf(r2, y2, -1.0f), -1.5f, y3);
+}
+
+// y with one Newton step.  SHORT shares cube_step's fma(r2, y^2, -K).
+constexpr float NEWTON_M = (float)(0.5 * (3.0 - (double)NEWTON_K));
+
+template <Step STEP>
+__device__ __forceinline__ float rsqrt_step(float r2, float y) {
+    if constexpr (STEP == Step::SHORT) return y * fmaf(fmaf(r2, y * y, -NEWTON_K), -0.5f, NEWTON_M);
+    return fmaf(-0.5f * fmaf(r2, y * y, -1.0f), y, y);
 }
 
 // Hardware reciprocal estimate (one MUFU.RCP).
@@ -76,7 +93,7 @@ struct PairConst {
     // single spline near branch in far units (g = f_ref / eps^3):
     //   (-15 u + 6 u^2 + 10) / eps^3 with u = r/eps = r^2 y / eps
     //   = (c1 y + c2) r^2 + c3,  c1 = -15 eps^-4, c2 = 6 eps^-5, c3 = 10 eps^-3,
-    // each times NEWTON_UNIT; cubic spline: c3 = eps^-3 NEWTON_UNIT
+    // cubic spline: c3 = eps^-3; all in the unit of the step
     float c1, c2, c3;
 };
 
@@ -93,9 +110,9 @@ __device__ __host__ __forceinline__ float r2_add(const PairConst &pc) {
 // GPU's branch on dr2 > 1, DirectGPUKernels.cuh:94-98, selects the same value
 // because the two branches touch to second order at u = 1 and the polynomial
 // is the smaller one for u < 1).  Here it is evaluated in far units with the
-// Newton-corrected yn = 1/r = y (3 - q) / 2, the step written on c = q - K:
+// Newton-corrected yn = 1/r:
 //   g = min(r^-3, (c1 yn + c2) r^2 + c3)
-// both in NEWTON_UNIT, which is negative, so that the smaller is the maximum.
+// (in NEWTON_UNIT, which is negative, the smaller is the maximum).
 // A self pair (d = 0, r^2 = 1e-25 floor) gives a finite g times d = 0; a
 // padding record far away gives an infinite polynomial and g ~ 0.
 // The cubic spline (Hernquist & Katz, DirectGPUKernels.cuh:31-65) is r^-3
@@ -103,30 +120,26 @@ __device__ __host__ __forceinline__ float r2_add(const PairConst &pc) {
 // to u = 1 and eps^-3 (4/3 - 6/5 u^2 + u^3/2) below.
 // Only sources within near_width() of a tile's sinks need these; all others
 // are evaluated as r^-3.
-constexpr float NEWTON_M = (float)(0.5 * (3.0 - (double)NEWTON_K));
 
-// g of a += g * d from r^2 (r2_add included), in pair_unit(SOFT).  NEAR: the
-// splines' full formula; otherwise their far branch.
-template <int SOFT, bool NEAR>
+// g of a += g * d from r^2 (r2_add included), in the unit of the step.  NEAR:
+// the splines' full formula; otherwise their far branch.
+template <int SOFT, bool NEAR, Step STEP>
 __device__ __forceinline__ float pair_g(float r2, const PairConst &pc) {
+    const float y = rsqrt_est(r2);
     if constexpr (SOFT == SOFT_CUBIC_PLUMMER) {
         // 1 / (r^3 + eps^3): reciprocal estimate and one Newton step; the
         // clamp keeps t * (1/t) defined for padding records
-        const float y = rsqrt_est(r2);
-        const float yn = y * fmaf(fmaf(r2, y * y, -NEWTON_K), -0.5f, NEWTON_M);
-        const float t = fminf(fmaf(r2 * r2, yn, pc.eps), 1e37f);
+        const float t = fminf(fmaf(r2 * r2, rsqrt_step<Step::FULL>(r2, y), pc.eps), 1e37f);
         const float g = rcp_est(t);
         return g * fmaf(-t, g, 2.0f);
     } else if constexpr (!NEAR || SOFT == SOFT_PLUMMER) {
-        return inv_r3(r2);
+        return cube_step<STEP>(r2, y);
     } else {
-        const float y = rsqrt_est(r2);
-        const float y2 = y * y;
-        const float c = fmaf(r2, y2, -NEWTON_K);
-        const float gfar = (y2 * y) * c;
-        const float yn = y * fmaf(c, -0.5f, NEWTON_M);
+        const float gfar = cube_step<STEP>(r2, y);
+        const float yn = rsqrt_step<SOFT == SOFT_SINGLE_SPLINE ? STEP : Step::FULL>(r2, y);
         if constexpr (SOFT == SOFT_SINGLE_SPLINE) {
-            return fmaxf(gfar, fmaf(fmaf(pc.c1, yn, pc.c2), r2, pc.c3));
+            const float gnear = fmaf(fmaf(pc.c1, yn, pc.c2), r2, pc.c3);
+            return STEP == Step::SHORT ? fmaxf(gfar, gnear) : fminf(gfar, gnear);
         } else {
             const float u = r2 * yn * pc.eps;
             const float u2 = u * u, u3 = u2 * u;
@@ -152,12 +165,19 @@ __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 __device__ __forceinline__ float2 dup2(float v) { return make_float2(v, v); }
 
-// inv_r3 on a pair.
-__device__ __forceinline__ float2 inv_r3_x2(float2 r2) {
-    float2 y = make_float2(rsqrt_est(r2.x), rsqrt_est(r2.y));
-    float2 y2 = mul2(y, y);
-    float2 c = fma2(r2, y2, dup2(-NEWTON_K));
-    return mul2(mul2(y2, y), c);
+// cube_step and rsqrt_step on a pair.
+template <Step STEP>
+__device__ __forceinline__ float2 cube_step_x2(float2 r2, float2 y) {
+    const float2 y2 = mul2(y, y);
+    const float2 y3 = mul2(y2, y);
+    if constexpr (STEP == Step::SHORT) return mul2(y3, fma2(r2, y2, dup2(-NEWTON_K)));
+    return fma2(mul2(y3, fma2(r2, y2, dup2(-1.0f))), dup2(-1.5f), y3);
+}
+template <Step STEP>
+__device__ __forceinline__ float2 rsqrt_step_x2(float2 r2, float2 y) {
+    if constexpr (STEP == Step::SHORT)
+        return mul2(y, fma2(fma2(r2, mul2(y, y), dup2(-NEWTON_K)), dup2(-0.5f), dup2(NEWTON_M)));
+    return fma2(mul2(dup2(-0.5f), fma2(r2, mul2(y, y), dup2(-1.0f))), y, y);
 }
 
 // r^2 (+ the kernel's additive constant a2) of a pair of separations.
@@ -166,36 +186,33 @@ __device__ __forceinline__ float2 r2_x2(float2 dx, float2 dy, float2 dz, float a
 }
 
 // pair_g on a pair.
-template <int SOFT, bool NEAR>
+template <int SOFT, bool NEAR, Step STEP>
 __device__ __forceinline__ float2 pair_g_x2(float2 r2, const PairConst &pc) {
-    if constexpr (SOFT != SOFT_CUBIC_PLUMMER && (!NEAR || SOFT == SOFT_PLUMMER)) {
-        return inv_r3_x2(r2);
+    const float2 y = make_float2(rsqrt_est(r2.x), rsqrt_est(r2.y));
+    if constexpr (SOFT == SOFT_CUBIC_PLUMMER) {
+        const float2 t0 = fma2(mul2(r2, r2), rsqrt_step_x2<Step::FULL>(r2, y), dup2(pc.eps));
+        const float2 t = make_float2(fminf(t0.x, 1e37f), fminf(t0.y, 1e37f));
+        const float2 g = make_float2(rcp_est(t.x), rcp_est(t.y));
+        return mul2(g, fma2(mul2(t, dup2(-1.0f)), g, dup2(2.0f)));
+    } else if constexpr (!NEAR || SOFT == SOFT_PLUMMER) {
+        return cube_step_x2<STEP>(r2, y);
     } else {
-        const float2 y = make_float2(rsqrt_est(r2.x), rsqrt_est(r2.y));
-        const float2 y2 = mul2(y, y);
-        const float2 c = fma2(r2, y2, dup2(-NEWTON_K));
-        const float2 yn = mul2(y, fma2(c, dup2(-0.5f), dup2(NEWTON_M)));
-        if constexpr (SOFT == SOFT_CUBIC_PLUMMER) {
-            const float2 t0 = fma2(mul2(r2, r2), yn, dup2(pc.eps));
-            const float2 t = make_float2(fminf(t0.x, 1e37f), fminf(t0.y, 1e37f));
-            const float2 g = make_float2(rcp_est(t.x), rcp_est(t.y));
-            return mul2(g, fma2(mul2(t, dup2(-1.0f)), g, dup2(2.0f)));
+        const float2 gfar = cube_step_x2<STEP>(r2, y);
+        const float2 yn = rsqrt_step_x2<SOFT == SOFT_SINGLE_SPLINE ? STEP : Step::FULL>(r2, y);
+        if constexpr (SOFT == SOFT_SINGLE_SPLINE) {
+            const float2 gnear = fma2(fma2(dup2(pc.c1), yn, dup2(pc.c2)), r2, dup2(pc.c3));
+            return STEP == Step::SHORT ? make_float2(fmaxf(gfar.x, gnear.x), fmaxf(gfar.y, gnear.y))
+                                       : make_float2(fminf(gfar.x, gnear.x), fminf(gfar.y, gnear.y));
         } else {
-            const float2 gfar = mul2(mul2(y2, y), c);
-            if constexpr (SOFT == SOFT_SINGLE_SPLINE) {
-                const float2 gnear = fma2(fma2(dup2(pc.c1), yn, dup2(pc.c2)), r2, dup2(pc.c3));
-                return make_float2(fmaxf(gfar.x, gnear.x), fmaxf(gfar.y, gnear.y));
-            } else {
-                const float2 u = mul2(mul2(r2, yn), dup2(pc.eps));
-                const float2 u2 = mul2(u, u), u3 = mul2(u2, u);
-                const float2 m1 = fma2(u, dup2(-1.f / 6.f), dup2(1.2f));
-                const float2 m2 = fma2(u, dup2(-3.f), dup2(8.f / 3.f));
-                const float2 mid = mul2(gfar, fma2(u3, fma2(u2, m1, m2), dup2(-1.f / 15.f)));
-                const float2 near =
-                    mul2(dup2(pc.c3), fma2(u2, fma2(u, dup2(0.5f), dup2(-1.2f)), dup2(4.f / 3.f)));
-                return make_float2(u.x >= 2.f ? gfar.x : u.x >= 1.f ? mid.x : near.x,
-                                   u.y >= 2.f ? gfar.y : u.y >= 1.f ? mid.y : near.y);
-            }
+            const float2 u = mul2(mul2(r2, yn), dup2(pc.eps));
+            const float2 u2 = mul2(u, u), u3 = mul2(u2, u);
+            const float2 m1 = fma2(u, dup2(-1.f / 6.f), dup2(1.2f));
+            const float2 m2 = fma2(u, dup2(-3.f), dup2(8.f / 3.f));
+            const float2 mid = mul2(gfar, fma2(u3, fma2(u2, m1, m2), dup2(-1.f / 15.f)));
+            const float2 near =
+                mul2(dup2(pc.c3), fma2(u2, fma2(u, dup2(0.5f), dup2(-1.2f)), dup2(4.f / 3.f)));
+            return make_float2(u.x >= 2.f ? gfar.x : u.x >= 1.f ? mid.x : near.x,
+                               u.y >= 2.f ? gfar.y : u.y >= 1.f ? mid.y : near.y);
         }
     }
 }
@@ -238,19 +255,25 @@ __device__ __forceinline__ float dens_term(float dx, float dy, float dz, float b
     return r2 < b2 ? b2 - r2 : 0.0f;
 }
 
+// The unit the pair sums of a softening are accumulated in.
+inline double pair_unit(int soft, Step step) {
+    return soft == SOFT_CUBIC_PLUMMER || step == Step::FULL ? 1.0 : NEWTON_UNIT;
+}
+
 // The pair constants of a launch; eps: the softening parameter (0: the configuration's).
-inline PairConst pair_const(const nf_config &cfg, float eps) {
+inline PairConst pair_const(const nf_config &cfg, float eps, Step step) {
+    const double unit = pair_unit(cfg.softening, step);
     PairConst pc{};
     if (!(eps > 0.f)) eps = cfg.eps;
     pc.eps = eps;
     pc.b2 = cfg.b2;
     if (cfg.softening == SOFT_SINGLE_SPLINE) {
         const double ie2 = (double)eps;  // eps_int^-2
-        pc.c1 = (float)(-15.0 * ie2 * ie2 * NEWTON_UNIT);
-        pc.c2 = (float)(6.0 * pow(ie2, 2.5) * NEWTON_UNIT);
-        pc.c3 = (float)(10.0 * pow(ie2, 1.5) * NEWTON_UNIT);
+        pc.c1 = (float)(-15.0 * ie2 * ie2 * unit);
+        pc.c2 = (float)(6.0 * pow(ie2, 2.5) * unit);
+        pc.c3 = (float)(10.0 * pow(ie2, 1.5) * unit);
     } else if (cfg.softening == SOFT_CUBIC_SPLINE) {
-        pc.c3 = (float)((double)eps * eps * eps * NEWTON_UNIT);
+        pc.c3 = (float)((double)eps * eps * eps * unit);
     }
     return pc;
 }
@@ -268,11 +291,6 @@ inline float near_width(const nf_config &cfg, float eps, int cpd) {
                      : cfg.softening == SOFT_CUBIC_SPLINE ? 2.0 / (double)eps
                                                           : 0.0;
     return (float)(e * 1.01 + 1e-6 / (double)cpd);
-}
-
-// The unit the pair sums of a softening are accumulated in.
-inline double pair_unit(int soft) {
-    return soft == SOFT_CUBIC_PLUMMER ? 1.0 : NEWTON_UNIT;
 }
 
 }  // namespace nf
