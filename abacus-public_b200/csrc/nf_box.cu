@@ -471,21 +471,31 @@ struct SumsView {
     const unsigned char *__restrict__ bad;
     int64_t n;
     int W, nc;
-    float scale;   // of x, y, z (mutual: out of the fixed-point unit as well)
-    float wscale;  // of w (mutual)
+    float scale;     // of x, y, z (mutual: out of the fixed-point unit as well)
+    float scale_lo;  // mutual: what scale's rounding left
+    float wscale;    // of w (mutual), a power of two
 };
 
 // The sums of particle p of the range.  One-sided: its 2R+1 partials summed
 // in compensated FP32 in pencil-slot order; x, y, z times the output scale
 // (one rounding: the correction is scaled and added inside the FMA), w
-// unscaled.
+// unscaled.  Mutual: the 64-bit sum as two floats times the scale as two
+// floats, also rounded once (products of low parts are below 2^-48).
+__device__ __forceinline__ float scale_fixed(long long v, float scale, float scale_lo) {
+    const float hi = __ll2float_rn(v);
+    const float lo = __ll2float_rn(v - __float2ll_rn(hi));
+    return fmaf(hi, scale, fmaf(hi, scale_lo, lo * scale));
+}
 __device__ __forceinline__ void coadd_sink(const SumsView &v, int64_t p, float r[4]) {
     if (v.acc) {
         const bool bad = v.bad[p];
 #pragma unroll
         for (int c = 0; c < 4; c++) {
             r[c] = 0.f;
-            if (c < v.nc) r[c] = __ll2float_rn((long long)v.acc[c * v.n + p]) * (c < 3 ? v.scale : v.wscale);
+            if (c < v.nc) {
+                const long long sum = (long long)v.acc[c * v.n + p];
+                r[c] = c < 3 ? scale_fixed(sum, v.scale, v.scale_lo) : __ll2float_rn(sum) * v.wscale;
+            }
             if (bad && c < 3) r[c] = __int_as_float(0x7fffffff);
         }
         return;
@@ -950,7 +960,9 @@ static SumsView sums_view(const nf_config &cfg, const Plan &pl, const void *scra
     SumsView v = sums_view(cfg, nullptr, pl.n_range, eps);
     v.acc = (const unsigned long long *)scratch;
     v.bad = (const unsigned char *)scratch + (size_t)pl.n_range * 8 * v.nc;
-    v.scale = (float)std::ldexp(output_scale(cfg, eps, Step::SHORT), -pl.fbits);
+    const double scale = std::ldexp(output_scale(cfg, eps, Step::SHORT), -pl.fbits);
+    v.scale = (float)scale;
+    v.scale_lo = (float)(scale - (double)v.scale);
     v.wscale = (float)std::ldexp(1.0, -pl.wbits);
     return v;
 }

@@ -15,10 +15,11 @@
 //     units of NEWTON_UNIT = 1 - float(5/3), divided out once per sink.  Its
 //     64-bit sums are nearer to FP64 than the one-sided engine's compensated
 //     FP32 all the same (uniform boxes of 3000 and 20000 particles: 3.0e-7 and
-//     1.8e-7 beside 3.4e-7 and 2.6e-7), and the fifth instruction costs it
-//     3-4 % of a sweep (clustered 256^3 90.0 -> 93.3 ms, uniform 160^3
-//     12.1 -> 12.6) and 10 % of a single slab; the one-sided engine pays 1 %
-//     (uniform 160^3 15.75 -> 15.91 ms).
+//     1.8e-7 beside 3.4e-7 and 2.6e-7; isolated pairs, where nothing is summed:
+//     Plummer 1.07e-7 beside 1.03e-7, single spline 1.24e-7 beside 1.45e-7),
+//     and the fifth instruction costs it 3-4 % of a sweep (clustered 256^3
+//     90.0 -> 93.3 ms, uniform 160^3 12.1 -> 12.6) and 10 % of a single slab;
+//     the one-sided engine pays 1 % (uniform 160^3 15.75 -> 15.91 ms).
 //   * the single spline is accumulated in far units, g = f_ref / eps^3
 //     (r^-3 in the far branch), and the sum is multiplied by eps^3 once per
 //     sink.  Chunks of sources that hold none within the spline's reach of a

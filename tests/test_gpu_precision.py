@@ -80,3 +80,29 @@ def test_one_sided_step(capi, synth, soft):
         emu = emu * F(unit)
     want, _ = _exact_separation_error(emu, unit * r64 ** -1.5, sep, sep.astype(D))
     assert rms <= 1.05 * want, (rms, want)
+
+
+def _newton_short(r2):
+    """The four-instruction step times NEWTON_UNIT, and that unit."""
+    k = F(5) / F(3)
+    y = (1 / np.sqrt(r2.astype(D))).astype(F)
+    y2 = y * y
+    return (y2 * y) * _fma(r2, y2, -k), 1.0 - D(k)
+
+
+@pytest.mark.parametrize("soft", [0, 1])
+def test_mutual_records_round_once(capi, synth, soft):
+    """Records of the fixed-point sums: the pair's own roundings and one more.
+    Within 2 % of their emulation (estimate and sampling error below 1 %); the
+    sum and the scale each rounded to a float first are 4 % above."""
+    length = 0.002 / CPD
+    eps = float(F(synth.kernel_eps(soft, length)))
+    a, sep = _records(capi, synth, soft, eps, capi.ACC_COMPENSATED, 0.05 / CPD, 0.38 / CPD)
+    add = eps if soft == 0 else 1e-25
+    unit = eps ** -1.5 if soft == 1 else 1.0
+    r64 = (sep.astype(D) ** 2).sum(1) + (eps if soft == 0 else 0.0)
+    rms, _ = _exact_separation_error(a, unit * r64 ** -1.5, sep, sep.astype(D))
+    g, newton_unit = _newton_short(_r2(sep, add))
+    emu = ((g[:, None] * sep).astype(F).astype(D) * (unit / newton_unit)).astype(F)
+    want, _ = _exact_separation_error(emu, unit * r64 ** -1.5, sep, sep.astype(D))
+    assert rms <= 1.02 * want, (rms, want)
