@@ -26,7 +26,9 @@
 //     tile's sinks use the far branch alone; the others the full formula.
 //   * the cubic kernels are free of branches and divisions (cubic spline,
 //     uniform 75^3: 3.26 -> 1.43 ms a sweep beside the scalar form with an
-//     IEEE division and three-way branch; error against FP64 7.8e-7 -> 6.3e-7).
+//     IEEE division and three-way branch).  Error against FP64 beside that
+//     form, uniform boxes of 20000: cubic spline 6.9e-7 -> 1.7e-7, cubic
+//     Plummer 2.6e-7 -> 1.7e-7 (2.6e-7 both in the one-sided engine).
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -118,7 +120,13 @@ __device__ __host__ __forceinline__ float r2_add(const PairConst &pc) {
 // padding record far away gives an infinite polynomial and g ~ 0.
 // The cubic spline (Hernquist & Katz, DirectGPUKernels.cuh:31-65) is r^-3
 // beyond u = r/eps = 2, r^-3 (-1/15 + u^3 (8/3 - 3 u + 6/5 u^2 - u^3/6)) down
-// to u = 1 and eps^-3 (4/3 - 6/5 u^2 + u^3/2) below.
+// to u = 1 and eps^-3 (4/3 - 6/5 u^2 + u^3/2) below.  The bracket is 1 at
+// u = 2 to fourth order,
+//   1 - (2 - u)^4 (1/15 + 2 u / 15 + u^2 / 6),
+// and evaluated in that form: the powers of u cancel to a part in 40 at
+// u = 2, and cost up to 2e-6 there (FP32 model, RMS over u in [1.75, 2));
+// this form keeps 6e-8, at one more instruction (uniform 75^3 1.389 -> 1.405
+// ms a sweep).
 // Only sources within near_width() of a tile's sinks need these; all others
 // are evaluated as r^-3.
 
@@ -128,11 +136,12 @@ template <int SOFT, bool NEAR, Step STEP>
 __device__ __forceinline__ float pair_g(float r2, const PairConst &pc) {
     const float y = rsqrt_est(r2);
     if constexpr (SOFT == SOFT_CUBIC_PLUMMER) {
-        // 1 / (r^3 + eps^3): reciprocal estimate and one Newton step; the
-        // clamp keeps t * (1/t) defined for padding records
+        // 1 / (r^3 + eps^3): reciprocal estimate and one Newton step written on
+        // the residual, so that only the last addition rounds; the clamp keeps
+        // t * (1/t) defined for padding records
         const float t = fminf(fmaf(r2 * r2, rsqrt_step<Step::FULL>(r2, y), pc.eps), 1e37f);
         const float g = rcp_est(t);
-        return g * fmaf(-t, g, 2.0f);
+        return fmaf(fmaf(-t, g, 1.0f), g, g);
     } else if constexpr (!NEAR || SOFT == SOFT_PLUMMER) {
         return cube_step<STEP>(r2, y);
     } else {
@@ -143,9 +152,9 @@ __device__ __forceinline__ float pair_g(float r2, const PairConst &pc) {
             return STEP == Step::SHORT ? fmaxf(gfar, gnear) : fminf(gfar, gnear);
         } else {
             const float u = r2 * yn * pc.eps;
-            const float u2 = u * u, u3 = u2 * u;
-            const float mid = fmaf(u3, fmaf(u2, fmaf(u, -1.f / 6.f, 1.2f), fmaf(u, -3.f, 8.f / 3.f)),
-                                   -1.f / 15.f);
+            const float u2 = u * u, w = 2.f - u, w2 = w * w;
+            const float p = fmaf(u, fmaf(u, -1.f / 6.f, -2.f / 15.f), -1.f / 15.f);
+            const float mid = fmaf(w2 * w2, p, 1.f);
             const float near = fmaf(u2, fmaf(u, 0.5f, -1.2f), 4.f / 3.f);
             return u >= 2.f ? gfar : u >= 1.f ? gfar * mid : pc.c3 * near;
         }
@@ -194,7 +203,7 @@ __device__ __forceinline__ float2 pair_g_x2(float2 r2, const PairConst &pc) {
         const float2 t0 = fma2(mul2(r2, r2), rsqrt_step_x2<Step::FULL>(r2, y), dup2(pc.eps));
         const float2 t = make_float2(fminf(t0.x, 1e37f), fminf(t0.y, 1e37f));
         const float2 g = make_float2(rcp_est(t.x), rcp_est(t.y));
-        return mul2(g, fma2(mul2(t, dup2(-1.0f)), g, dup2(2.0f)));
+        return fma2(fma2(mul2(t, dup2(-1.0f)), g, dup2(1.0f)), g, g);
     } else if constexpr (!NEAR || SOFT == SOFT_PLUMMER) {
         return cube_step_x2<STEP>(r2, y);
     } else {
@@ -206,10 +215,9 @@ __device__ __forceinline__ float2 pair_g_x2(float2 r2, const PairConst &pc) {
                                        : make_float2(fminf(gfar.x, gnear.x), fminf(gfar.y, gnear.y));
         } else {
             const float2 u = mul2(mul2(r2, yn), dup2(pc.eps));
-            const float2 u2 = mul2(u, u), u3 = mul2(u2, u);
-            const float2 m1 = fma2(u, dup2(-1.f / 6.f), dup2(1.2f));
-            const float2 m2 = fma2(u, dup2(-3.f), dup2(8.f / 3.f));
-            const float2 mid = mul2(gfar, fma2(u3, fma2(u2, m1, m2), dup2(-1.f / 15.f)));
+            const float2 u2 = mul2(u, u), w = fma2(u, dup2(-1.f), dup2(2.f)), w2 = mul2(w, w);
+            const float2 p = fma2(u, fma2(u, dup2(-1.f / 6.f), dup2(-2.f / 15.f)), dup2(-1.f / 15.f));
+            const float2 mid = mul2(gfar, fma2(mul2(w2, w2), p, dup2(1.f)));
             const float2 near =
                 mul2(dup2(pc.c3), fma2(u2, fma2(u, dup2(0.5f), dup2(-1.2f)), dup2(4.f / 3.f)));
             return make_float2(u.x >= 2.f ? gfar.x : u.x >= 1.f ? mid.x : near.x,

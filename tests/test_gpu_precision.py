@@ -106,3 +106,48 @@ def test_mutual_records_round_once(capi, synth, soft):
     emu = ((g[:, None] * sep).astype(F).astype(D) * (unit / newton_unit)).astype(F)
     want, _ = _exact_separation_error(emu, unit * r64 ** -1.5, sep, sep.astype(D))
     assert rms <= 1.02 * want, (rms, want)
+
+
+def _cubic_spline64(u, e):
+    far = (u * e) ** -3
+    mid = far * (-1 / 15 + u ** 3 * (8 / 3 - 3 * u + 1.2 * u ** 2 - u ** 3 / 6))
+    near = e ** -3 * (4 / 3 - 1.2 * u ** 2 + 0.5 * u ** 3)
+    return np.where(u >= 2, far, np.where(u >= 1, mid, near))
+
+
+@pytest.mark.parametrize("acc", [0, 1])
+def test_cubic_spline_over_its_reach(capi, synth, acc):
+    """RMS error below 1.6e-7 wherever the pair lies: the force factor's in an
+    FP32 emulation is at most 9.3e-8 (u just above 1), the product's and the
+    record's roundings add 3e-8 each.  Evaluated by powers of u, the middle
+    branch loses 2e-6 at u = 2."""
+    e = 0.17 / CPD
+    eps = float(F(synth.kernel_eps(2, e)))
+    a, sep = _records(capi, synth, 2, eps, acc, 0.02 * e, 2.3 * e)
+    d64 = sep.astype(D)
+    u = np.sqrt((d64 ** 2).sum(1)) * eps
+    _, err = _exact_separation_error(a, _cubic_spline64(u, 1.0 / eps), sep, d64)
+    edges = [0.02, 0.5, 1, 1.25, 1.5, 1.75, 2, 2.3]
+    for lo, hi in zip(edges, edges[1:]):
+        q = err[(u >= lo) & (u < hi)]
+        assert len(q) > 1000
+        rms = np.sqrt(np.mean(q ** 2))
+        assert rms <= 1.6e-7, (lo, hi, rms)
+
+
+@pytest.mark.parametrize("acc", [0, 1])
+def test_cubic_plummer_reciprocal(capi, synth, acc):
+    """The reciprocal is as good as a division: within 3 % of the emulation with
+    one (estimate and sampling error below 1 %); a Newton step whose factor is
+    rounded near 1 is 5 % above or more."""
+    e = 0.1 / CPD
+    eps = float(F(synth.kernel_eps(3, e)))
+    a, sep = _records(capi, synth, 3, eps, acc, 0.2 * e, 3.5 * e)
+    d64 = sep.astype(D)
+    g64 = 1 / (((d64 ** 2).sum(1) + D(F(1e-16))) ** 1.5 + eps)
+    rms, _ = _exact_separation_error(a, g64, sep, d64)
+    r2 = _r2(sep, 1e-16)
+    rinv = (1 / np.sqrt(r2.astype(D))).astype(F)
+    g = F(1) / _fma(r2 * r2, rinv, F(eps))
+    want, _ = _exact_separation_error((g[:, None] * sep).astype(F), g64, sep, d64)
+    assert rms <= 1.03 * want, (rms, want)
