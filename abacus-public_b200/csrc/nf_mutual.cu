@@ -469,7 +469,10 @@ template <int SOFT, bool DENS, int S, bool NEAR, bool MUTUAL>
 __device__ __forceinline__ void meet(const float4 &t, const float2 &tz, Sinks<S> &k, Reaction &r,
                                      const PairConst &pc) {
     const float2 tx = make_float2(t.x, t.y), ty = make_float2(t.z, t.w);
-    const float w_r2 = pc.b2 + r2_add<SOFT>(pc);  // density: b2 - |d|^2 = w_r2 - r2
+    // density terms b2 - |d|^2: from r^2 where its r2_add is below the rounding
+    // of b2 (mutual_bits); Plummer's eps^2 is not, and would leave its own
+    // rounding in every term, so there |d|^2 is formed for itself (uniform
+    // n = 6000, b2 = 32 eps^2: density error 1.6e-7 from r^2, 1.4e-7 so)
 #pragma unroll
     for (int q = 0; q < Sinks<S>::N; q++) {
         if constexpr (S == 1) {
@@ -485,7 +488,7 @@ __device__ __forceinline__ void meet(const float4 &t, const float2 &tz, Sinks<S>
                 r.z.x = fmaf(g, dz, r.z.x);
             }
             if (DENS) {
-                const float d = fmaxf(w_r2 - r2, 0.f);
+                const float d = SOFT == SOFT_PLUMMER ? dens_term(dx, dy, dz, pc.b2) : fmaxf(pc.b2 - r2, 0.f);
                 k.w[0].x += d;
                 if (MUTUAL) r.w.x += d;
             }
@@ -502,7 +505,8 @@ __device__ __forceinline__ void meet(const float4 &t, const float2 &tz, Sinks<S>
                 r.z = fma2(g, dz, r.z);
             }
             if (DENS) {
-                const float2 e = fma2(r2, dup2(-1.f), dup2(w_r2));
+                const float2 s2 = SOFT == SOFT_PLUMMER ? fma2(dz, dz, fma2(dy, dy, mul2(dx, dx))) : r2;
+                const float2 e = fma2(s2, dup2(-1.f), dup2(pc.b2));
                 const float2 d = make_float2(fmaxf(e.x, 0.f), fmaxf(e.y, 0.f));
                 k.w[q] = add2(k.w[q], d);
                 if (MUTUAL) r.w = add2(r.w, d);
@@ -950,10 +954,10 @@ static bool mutual_bits(int soft, double eps, double b2, int cpd, double n_max, 
     *fbits = 62 - (int)std::ceil(std::log2(bound));
     const double h = 1.0 / (double)cpd;
     if (std::ldexp(1.0, -*fbits) * h * h > std::ldexp(1.0, -25)) return false;
-    // the density sum, at most n_max b2; taken from r^2 with its r2_add, which
-    // must be small beside it
-    const double add = soft == SOFT_PLUMMER ? eps : soft == SOFT_CUBIC_PLUMMER ? 1e-16 : 1e-25;
-    if (b2 > 0.0 && b2 < 4.0 * add) return false;
+    // the density sum, at most n_max b2; taken from r^2 (Plummer: from |d|^2)
+    // with its r2_add, which must be below half a unit of b2's last place
+    const double add = soft == SOFT_PLUMMER ? 0.0 : soft == SOFT_CUBIC_PLUMMER ? 1e-16 : 1e-25;
+    if (b2 > 0.0 && b2 < std::ldexp(add, 25)) return false;
     *wbits = b2 > 0.0 ? 62 - (int)std::ceil(std::log2(1.02 * b2 * n_max)) : 0;
     // both scales are floats
     return std::abs(*fbits) <= 100 && std::abs(*wbits) <= 100;
