@@ -23,6 +23,7 @@ STATUS_NAMES = {0: "NF_OK", 1: "NF_EINVAL", 2: "NF_ENOMEM", 3: "NF_EADMISSION",
                 8: "NF_ECANCELLED"}
 SOFT_PLUMMER, SOFT_SINGLE_SPLINE, SOFT_CUBIC_SPLINE, SOFT_CUBIC_PLUMMER = range(4)
 ACC_COMPENSATED, ACC_PLAIN = 0, 1
+ENGINE_MUTUAL, ENGINE_ONE_SIDED = 0, 1
 OUT_FLOAT3, OUT_FLOAT4 = 0, 1
 ABI_VERSION = 2  # NF_ABI_VERSION of include/nf_capi.h
 
@@ -213,6 +214,7 @@ EXPORTS = {
                                      ctypes.c_int, ctypes.c_void_p, ctypes.c_int]),
     "nf_box_pair_count": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int,
                                          ctypes.c_int, ctypes.POINTER(ctypes.c_uint64)]),
+    "nf_last_engine": (ctypes.c_int, [ctypes.c_void_p, ctypes.POINTER(ctypes.c_int)]),
     "nf_last_timing": (ctypes.c_int, [ctypes.c_void_p, ctypes.POINTER(Timing)]),
     "nf_set_stream": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_void_p]),
     "nf_forces_noalloc": (ctypes.c_int, [ctypes.POINTER(Config), ctypes.c_int, ctypes.c_void_p,
@@ -316,6 +318,12 @@ class Context:
         check(lib().nf_measure_fp32_peak(self.h, seconds_sustained, ctypes.byref(b),
                                          ctypes.byref(s)), "nf_measure_fp32_peak")
         return b.value, s.value
+
+    def last_engine(self) -> int:
+        """ENGINE_MUTUAL or ENGINE_ONE_SIDED: what the last sweep ran on."""
+        e = ctypes.c_int(-1)
+        check(lib().nf_last_engine(self.h, ctypes.byref(e)), "nf_last_engine")
+        return e.value
 
     def last_timing(self) -> Timing:
         t = Timing()

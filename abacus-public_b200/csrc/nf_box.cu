@@ -986,6 +986,7 @@ int engine_grid(nf_ctx *ctx, int variant) {
 }
 
 nf_status engine_launch(nf_ctx *ctx, const EngineLaunch &L, double, cudaStream_t st) {
+    ctx->engine = NF_ENGINE_ONE_SIDED;
     if (L.n_heavy_groups + L.n_light == 0) return NF_OK;
     KParams kp = params_from(ctx, L);
     KernelFn fn = pick_kernel(ctx->cfg.softening, ctx->cfg.b2 > 0.f, L.variant);
@@ -1049,6 +1050,7 @@ static nf_status enqueue_pencil(nf_ctx *ctx, nf_box *box, Plan &pl, cudaStream_t
         NF_CUDA(cudaEventRecordWithFlags(ctx->ev[1], st, evflags));
         return NF_OK;
     }
+    ctx->engine = NF_ENGINE_ONE_SIDED;
     const nf_config &cfg = ctx->cfg;
     KParams kp = make_params(ctx, box, pl);
     KernelFn fn = pick_kernel(cfg.softening, cfg.b2 > 0.f, BOX_VARIANT);
@@ -1066,6 +1068,7 @@ static nf_status enqueue_pencil(nf_ctx *ctx, nf_box *box, Plan &pl, cudaStream_t
 // The sweep of a plan: launched as it is the first time (a box of one step's
 // cell counts is swept once), as a CUDA graph captured on the second.
 static nf_status run_sweep(nf_ctx *ctx, nf_box *box, Plan &pl) {
+    ctx->engine = pl.mutual ? NF_ENGINE_MUTUAL : NF_ENGINE_ONE_SIDED;
     cudaStream_t s = ctx->stream;
     if (!pl.graph && pl.runs++ == 0) return enqueue_pencil(ctx, box, pl, s, cudaEventRecordDefault);
     if (!pl.graph) {

@@ -274,6 +274,20 @@ extern "C" nf_status nf_measure_fp32_peak(nf_ctx *ctx, double seconds_sustained,
     return NF_OK;
 }
 
+extern "C" nf_status nf_last_engine(nf_ctx *ctx, int *engine) {
+    if (!ctx || !engine) {
+        set_error("nf_last_engine: null argument");
+        return NF_EINVAL;
+    }
+    const int e = ctx->engine.load();
+    if (e < 0) {
+        set_error("nf_last_engine: no sweep has run");
+        return NF_ENOTREADY;
+    }
+    *engine = e;
+    return NF_OK;
+}
+
 extern "C" nf_status nf_last_timing(nf_ctx *ctx, nf_timing *t) {
     if (!ctx || !t) {
         set_error("nf_last_timing: null argument");

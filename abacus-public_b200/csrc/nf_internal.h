@@ -209,6 +209,7 @@ struct nf_ctx {
     cudaStream_t own_stream = nullptr;  // created by nf_init
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
     nf_timing last{};
+    std::atomic<int> engine{-1};  // of the last sweep (NF_ENGINE_*)
     std::mutex mu;  // serialises nf_box_forces on one context
     // device memory of boxes and plans; freed blocks up to 1/32 of the device
     // stay here for the next box, until nf_shutdown

@@ -1194,6 +1194,7 @@ static MParams mutual_params(const nf_config &cfg, const MutualLaunch &L) {
 
 // Zero the sums (unless mutual_unpack has) and run the sweep of a plan.
 nf_status mutual_launch(nf_ctx *ctx, const MutualLaunch &L, cudaStream_t st) {
+    ctx->engine = NF_ENGINE_MUTUAL;
     const nf_config &cfg = ctx->cfg;
     const Plan &pl = *L.plan;
     if (!L.zeroed) {

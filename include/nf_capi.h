@@ -373,6 +373,24 @@ typedef struct nf_timing {
 /* Timing of the last nf_box_forces on this context. */
 nf_status nf_last_timing(nf_ctx *ctx, nf_timing *t);
 
+/* Which engine the context's last sweep ran on (nf_box_forces, nf_box_kick,
+ * nf_box_step, a slab of a server, a SIC): the mutual one evaluates each pair
+ * once and adds it to both particles, in 64-bit fixed point; the one-sided one
+ * evaluates it for each of the two, in FP32.  The one-sided engine, about 1.4
+ * times the time, serves plain accumulation and what the fixed point does not
+ * resolve: with F the largest force of a pair (Plummer 0.39 e^-2, single
+ * spline 2.1 e^-2, cubic spline 1.4 e^-2, cubic Plummer 0.54 e^-2, e the
+ * softening length in box units) and M the most sources a pencil of the slab
+ * range meets, it is taken where F (2R+1) M is above 2^36 to 2^37 cpd^2 --
+ * a softening below 4e-4 (Plummer) to 9e-4 (single spline) cells at R 2 and
+ * M = 10^4, in proportion to the root of M -- and where the density radius is tiny (b2 < 3.4e-9 with the cubic
+ * Plummer softening, < 3.4e-18 with a spline).  nf_forces_noalloc follows the
+ * same rule with M (2R+1) the number of particles of the box.
+ * NF_ENOTREADY before the first sweep. */
+#define NF_ENGINE_MUTUAL 0
+#define NF_ENGINE_ONE_SIDED 1
+nf_status nf_last_engine(nf_ctx *ctx, int *engine);
+
 /* Kernel shapes the autotuner chooses among (sinks per lane, unroll depth,
  * CTAs per SM).  The first nf_box_forces call on a box times every shape on
  * the requested slab range and keeps the fastest for that box, and for later
