@@ -222,6 +222,7 @@ EXPORTS = {
                                          ctypes.c_void_p, ctypes.c_void_p]),
     "nf_kernel_variant_count": (ctypes.c_int, []),
     "nf_kernel_variant_name": (ctypes.c_char_p, [ctypes.c_int]),
+    "nf_engine_variant_name": (ctypes.c_char_p, [ctypes.c_int, ctypes.c_int]),
     "nf_box_tuning": (ctypes.c_int, [ctypes.c_void_p, ctypes.POINTER(ctypes.c_int),
                                      ctypes.POINTER(ctypes.c_float), ctypes.c_int]),
     "nf_measure_fp32_peak": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_double,

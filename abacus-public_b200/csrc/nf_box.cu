@@ -675,22 +675,32 @@ __global__ void kick_kernel(SumsView v, const int64_t *__restrict__ cs, int64_t 
 
 typedef void (*KernelFn)(KParams);
 
-// Shapes of the one-sided kernel: 128-sink tiles, or the plain drop-in's 64.
-// (The autotuner's shapes are those of the mutual sweep, nf_mutual.cu; boxes
-// that take the one-sided sweep run shape 0 whatever it picks.)
+// Shapes of the one-sided kernel (those of the mutual one: nf_mutual.cu); the
+// kernels without a choice of shapes run shape 0.
 struct Variant {
     int smax, unr, minb;
+    const char *name;
 };
-static const Variant VARIANTS[] = {{4, 8, 2}, {2, 4, 3}};
-static constexpr int BOX_VARIANT = 0, PLAIN_VARIANT = 1;
+static const Variant VARIANTS[] = {
+    {4, 8, 2, "one-sided, sinks/lane<=4 unroll 8, 2 CTAs/SM"},
+    {4, 16, 2, "one-sided, sinks/lane<=4 unroll 16, 2 CTAs/SM"},
+    {8, 4, 1, "one-sided, sinks/lane<=8 unroll 4, 1 CTA/SM"},
+    {2, 4, 3, "one-sided, sinks/lane<=2 unroll 4, 3 CTAs/SM"},
+    {2, 2, 4, "one-sided, sinks/lane<=2 unroll 2, 4 CTAs/SM"},
+};
+static constexpr int NVARIANTS = sizeof(VARIANTS) / sizeof(VARIANTS[0]);
+static constexpr int PLAIN_VARIANT = 3;  // the plain drop-in's: 64-sink tiles
+static_assert(NVARIANTS == MUTUAL_SHAPES, "kernel_variant indexes the shapes of either engine");
 
 template <int SOFT, bool DENS>
 static KernelFn variant_kernel(int v) {
-    return v == PLAIN_VARIANT ? pencil_kernel<SOFT, DENS, 2, 4, 3> : pencil_kernel<SOFT, DENS, 4, 8, 2>;
-}
-
-static bool tunable(int soft, bool dens) {
-    return !dens && (soft == SOFT_PLUMMER || soft == SOFT_SINGLE_SPLINE);
+    switch (v) {
+    case 1: return pencil_kernel<SOFT, DENS, 4, 16, 2>;
+    case 2: return pencil_kernel<SOFT, DENS, 8, 4, 1>;
+    case 3: return pencil_kernel<SOFT, DENS, 2, 4, 3>;
+    case 4: return pencil_kernel<SOFT, DENS, 2, 2, 4>;
+    default: return pencil_kernel<SOFT, DENS, 4, 8, 2>;
+    }
 }
 
 static KernelFn pick_kernel(int soft, bool dens, int v) {
@@ -753,9 +763,10 @@ static nf_status build_plan(nf_ctx *ctx, nf_box *box, int lo, int hi, int varian
     };
     pl.lo = lo;
     pl.hi = hi;
+    if (!tunable(ctx->cfg.softening, ctx->cfg.b2 > 0.f)) variant = 0;
     pl.variant = variant;
-    const int smax = VARIANTS[BOX_VARIANT].smax;
-    const int unr = VARIANTS[BOX_VARIANT].unr;
+    const int smax = VARIANTS[variant].smax;
+    const int unr = VARIANTS[variant].unr;
     pl.p0 = cs[(int64_t)lo * cpd * cpd];
     pl.n_range = cs[(int64_t)hi * cpd * cpd] - pl.p0;
     const int rec = ctx->cfg.out_kind == NF_OUT_FLOAT4 ? 16 : 12;
@@ -808,7 +819,7 @@ static nf_status build_plan(nf_ctx *ctx, nf_box *box, int lo, int hi, int varian
     pl.pairs = pairs;
     pl.padded_pairs = padded;
     // occupancy-derived persistent grid
-    KernelFn fn = pick_kernel(ctx->cfg.softening, ctx->cfg.b2 > 0.f, BOX_VARIANT);
+    KernelFn fn = pick_kernel(ctx->cfg.softening, ctx->cfg.b2 > 0.f, variant);
     int per_sm = 0;
     NF_CUDA(cudaFuncSetAttribute((const void *)fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)kernel_smem()));
@@ -930,7 +941,7 @@ static KParams make_params(nf_ctx *ctx, nf_box *box, const Plan &pl) {
     L.part = box->d_part;
     L.p0 = pl.p0;
     L.n_range = pl.n_range;
-    L.variant = BOX_VARIANT;
+    L.variant = pl.variant;
     L.eps = box->eps;
     return params_from(ctx, L);
 }
@@ -969,7 +980,7 @@ static SumsView sums_view(const nf_config &cfg, const Plan &pl, const void *scra
 
 // The plain drop-in runs the reference's block shape: 64-sink tiles.
 int engine_plain_variant() { return PLAIN_VARIANT; }
-int engine_box_variant() { return BOX_VARIANT; }
+const char *engine_shape_name(int v) { return VARIANTS[v].name; }
 
 int engine_grid(nf_ctx *ctx, int variant) {
     KernelFn fn = pick_kernel(ctx->cfg.softening, ctx->cfg.b2 > 0.f, variant);
@@ -1053,7 +1064,7 @@ static nf_status enqueue_pencil(nf_ctx *ctx, nf_box *box, Plan &pl, cudaStream_t
     ctx->engine = NF_ENGINE_ONE_SIDED;
     const nf_config &cfg = ctx->cfg;
     KParams kp = make_params(ctx, box, pl);
-    KernelFn fn = pick_kernel(cfg.softening, cfg.b2 > 0.f, BOX_VARIANT);
+    KernelFn fn = pick_kernel(cfg.softening, cfg.b2 > 0.f, pl.variant);
     NF_CUDA(cudaMemsetAsync(pl.d_counters, 0, 2 * sizeof(int), st));
     NF_CUDA(cudaEventRecordWithFlags(ctx->ev[0], st, evflags));
     if (pl.n_heavy_groups + pl.n_light > 0) {
@@ -1435,35 +1446,51 @@ static nf_status time_pencil(nf_ctx *ctx, nf_box *box, Plan &pl, float *ms) {
     return NF_OK;
 }
 
-// The autotuner: run every candidate kernel shape on the requested slab
-// range and keep the fastest for the box, and for later boxes of the context
-// whose work is of the same size (particles and pairs per particle within a
-// factor of two): a simulation that drifts between cells makes a new box each
-// step and would otherwise time five shapes to sweep once (clustered 96^3,
-// create + sweep + destroy: 49.8 -> 3.3 ms, with the device memory kept in the
-// context's pool and the first sweep launched without a graph).  A candidate whose first launch
-// is short (< 50 ms, where loading the kernel and a cold L2 weigh) is timed
-// again and the second launch counts; a long first launch counts as it is.
-static nf_status autotune(nf_ctx *ctx, nf_box *box, int lo, int hi, Tuned &t) {
-    const bool tun = tunable(ctx->cfg.softening, ctx->cfg.b2 > 0.f);
-    const int nv = tun ? MUTUAL_SHAPES : 1;
-    float best_ms = 3.0e38f;
-    for (int v = 0; v < nv; v++) {
-        std::unique_ptr<Plan> pl;
-        nf_status st = new_plan(ctx, box, lo, hi, v, pl);
-        if (st != NF_OK) return st;
+// The autotuner: run every kernel shape of the engine that the requested slab
+// range takes and keep the fastest for the box, and for later sweeps of the
+// context with the same TuneKey: a simulation that drifts between cells makes
+// a new box each step and would otherwise time five shapes to sweep once
+// (clustered 96^3, create + sweep + destroy: 49.8 -> 3.3 ms, with the device
+// memory kept by the context and the first sweep launched without a graph).
+// A candidate whose first launch is short (< 50 ms, where loading the kernel
+// and a cold L2 weigh) is timed again and the second launch counts; a long
+// first launch counts as it is.  `pl`: the plan of shape 0; on return that of
+// the fastest.
+static nf_status autotune(nf_ctx *ctx, nf_box *box, int lo, int hi, std::unique_ptr<Plan> &pl, Tuned &t) {
+    std::unique_ptr<Plan> best = std::move(pl);
+    float best_ms = 0.f;
+    for (int v = 0; v < MUTUAL_SHAPES; v++) {
+        std::unique_ptr<Plan> own;
+        nf_status st = v == 0 ? NF_OK : new_plan(ctx, box, lo, hi, v, own);
         float ms = 0;
-        st = time_pencil(ctx, box, *pl, &ms);
-        if (st == NF_OK && ms < 50.f) st = time_pencil(ctx, box, *pl, &ms);
-        free_plan(ctx, *pl);
-        if (st != NF_OK) return st;
+        Plan *p = own ? own.get() : best.get();
+        if (st == NF_OK) st = time_pencil(ctx, box, *p, &ms);
+        if (st == NF_OK && ms < 50.f) st = time_pencil(ctx, box, *p, &ms);
+        if (st != NF_OK) {
+            if (own) free_plan(ctx, *own);
+            free_plan(ctx, *best);
+            return st;
+        }
         t.ms[v] = ms;
-        if (ms < best_ms) {
+        if (v == 0 || ms < best_ms) {
             best_ms = ms;
             t.variant = v;
+            if (own) std::swap(own, best);
         }
+        if (own) free_plan(ctx, *own);
     }
+    pl = std::move(best);
     return NF_OK;
+}
+
+static TuneKey tune_key(const nf_ctx *ctx, const nf_box *box, const Plan &pl) {
+    const nf_config &cfg = ctx->cfg;
+    const double n = (double)std::max<int64_t>(pl.n_range, 1);
+    auto lg = [](double v) { return (int)std::floor(std::log2(v)); };
+    return TuneKey{pl.mutual ? NF_ENGINE_MUTUAL : NF_ENGINE_ONE_SIDED,
+                   pl.hi - pl.lo == box->cpd ? -1 : lg(pl.hi - pl.lo), lg(n),
+                   lg(std::max((double)pl.pairs, 1.0) / n),
+                   has_near(cfg.softening) ? lg((double)near_width(cfg, box->eps, box->cpd) * box->cpd) : 0};
 }
 
 static nf_status get_plan(nf_ctx *ctx, nf_box *box, int lo, int hi, Plan **out) {
@@ -1473,33 +1500,44 @@ static nf_status get_plan(nf_ctx *ctx, nf_box *box, int lo, int hi, Plan **out) 
         *out = it->second.get();
         return NF_OK;
     }
-    int v = ctx->cfg.kernel_variant;
+    // the shape: fixed by the caller, or the box's (of the engine it took
+    // last, until the plan tells which one this range takes)
+    const bool fixed = ctx->cfg.kernel_variant >= 0;
+    const int v = fixed ? ctx->cfg.kernel_variant : std::max(box->tuned[box->engine].variant, 0);
     std::unique_ptr<Plan> pl;
-    nf_status st = NF_OK;
-    if (v < 0 && box->variant < 0) {
-        // the choice made on this context for work of this size, if there is one
-        st = new_plan(ctx, box, lo, hi, 0, pl);
-        if (st != NF_OK) return st;
-        const double n = (double)std::max<int64_t>(pl->n_range, 1);
-        const auto size = std::make_pair((int)std::log2(n), (int)std::log2(std::max((double)pl->pairs, 1.0) / n));
-        auto known = ctx->tuned.find(size);
-        if (known == ctx->tuned.end()) {
-            Tuned t;
-            st = autotune(ctx, box, lo, hi, t);
-            if (st != NF_OK) {
-                free_plan(ctx, *pl);
-                return st;
+    nf_status st = new_plan(ctx, box, lo, hi, v, pl);
+    if (st != NF_OK) return st;
+    box->engine = pl->mutual ? NF_ENGINE_MUTUAL : NF_ENGINE_ONE_SIDED;
+    if (!fixed) {
+        Tuned &t = box->tuned[box->engine];
+        if (t.variant < 0) {
+            if (!tunable(ctx->cfg.softening, ctx->cfg.b2 > 0.f)) {
+                t.variant = 0;  // nothing to choose among
+            } else {
+                const TuneKey key = tune_key(ctx, box, *pl);
+                auto known = ctx->tuned.find(key);
+                if (known != ctx->tuned.end()) {
+                    t = known->second;
+                } else {
+                    if (pl->variant != 0) {  // the other engine's shape
+                        free_plan(ctx, *pl);
+                        st = new_plan(ctx, box, lo, hi, 0, pl);
+                        if (st != NF_OK) return st;
+                    }
+                    st = autotune(ctx, box, lo, hi, pl, t);
+                    if (st != NF_OK) {
+                        t = Tuned{};
+                        return st;
+                    }
+                    ctx->tuned[key] = t;
+                }
             }
-            known = ctx->tuned.emplace(size, t).first;
         }
-        box->variant = known->second.variant;
-        memcpy(box->tune_ms, known->second.ms, sizeof(box->tune_ms));
-    }
-    if (v < 0) v = box->variant;
-    if (!pl || v != 0) {
-        if (pl) free_plan(ctx, *pl);
-        st = new_plan(ctx, box, lo, hi, v, pl);
-        if (st != NF_OK) return st;
+        if (pl->variant != t.variant) {
+            free_plan(ctx, *pl);
+            st = new_plan(ctx, box, lo, hi, t.variant, pl);
+            if (st != NF_OK) return st;
+        }
     }
     *out = pl.get();
     box->plans[key] = std::move(pl);
@@ -1519,8 +1557,13 @@ nf_status nf::box_plan(nf_ctx *ctx, nf_box *box, int lo, int hi, const Plan **ou
 
 extern "C" int nf_kernel_variant_count(void) { return MUTUAL_SHAPES; }
 
-extern "C" const char *nf_kernel_variant_name(int v) {
-    return (v >= 0 && v < MUTUAL_SHAPES) ? mutual_shape_name(v) : "";
+extern "C" const char *nf_kernel_variant_name(int v) { return nf_engine_variant_name(NF_ENGINE_MUTUAL, v); }
+
+extern "C" const char *nf_engine_variant_name(int engine, int v) {
+    if (v < 0 || v >= MUTUAL_SHAPES) return "";
+    return engine == NF_ENGINE_MUTUAL      ? mutual_shape_name(v)
+           : engine == NF_ENGINE_ONE_SIDED ? engine_shape_name(v)
+                                           : "";
 }
 
 extern "C" nf_status nf_box_tuning(const nf_box *box, int *variant, float *ms, int n) {
@@ -1528,8 +1571,9 @@ extern "C" nf_status nf_box_tuning(const nf_box *box, int *variant, float *ms, i
         set_error("nf_box_tuning: null argument");
         return NF_EINVAL;
     }
-    *variant = box->variant;
-    for (int i = 0; ms && i < n && i < MUTUAL_SHAPES; i++) ms[i] = box->tune_ms[i];
+    const Tuned &t = box->tuned[box->engine];
+    *variant = t.variant;
+    for (int i = 0; ms && i < n && i < MUTUAL_SHAPES; i++) ms[i] = t.ms[i];
     return NF_OK;
 }
 

@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <array>
 #include <atomic>
 #include <condition_variable>
 #include <cstdint>
@@ -55,7 +56,7 @@ struct MutualItem {
 
 struct Plan {
     int lo = 0, hi = 0;
-    int variant = 0;  // kernel shape (index into the variant table)
+    int variant = 0;  // kernel shape (index into the engine's table)
     int64_t p0 = 0, n_range = 0;
     Item *d_heavy = nullptr;
     int n_heavy_groups = 0;
@@ -75,6 +76,17 @@ struct Plan {
     cudaGraphExec_t graph = nullptr;  // the sweep, captured when it is run again
     int runs = 0;
 };
+
+// A kernel shape chosen by the autotuner, and what each candidate took.
+struct Tuned {
+    int variant = -1;
+    float ms[8] = {};
+};
+
+// What two sweeps have to have in common for one's shape to serve the other:
+// engine, slabs of the range (log2; the whole box -1), particles, pairs per
+// particle, and the spline's reach in cells (log2; 0 without one).
+typedef std::array<int, 5> TuneKey;
 
 }  // namespace nf
 struct nf_box;
@@ -155,15 +167,11 @@ nf_status engine_pack(nf_ctx *ctx, const float *x, const float *y, const float *
                       float4 *out, cudaStream_t st);
 int engine_grid(nf_ctx *ctx, int variant);
 int engine_plain_variant();
-int engine_box_variant();
+const char *engine_shape_name(int v);
 constexpr int ENGINE_WARPS_PER_CTA = 8;
 // SIC size limits from a buffer budget (the reference's bytes-per-block model).
 nf_status sic_limits(int out_kind, int cpd, uint64_t max_buffer_bytes, nf_gpu_limits *lim);
 // The cached work list of a box's slab range (nf_box.cu).
-struct Plan;
-}  // namespace nf
-struct nf_box;
-namespace nf {
 nf_status box_plan(nf_ctx *ctx, nf_box *box, int lo, int hi, const Plan **out);
 
 }  // namespace nf
@@ -187,19 +195,11 @@ struct nf_box {
     std::vector<cudaEvent_t> step_ev;
     size_t part_bytes = 0;
     std::map<std::pair<int, int>, std::unique_ptr<nf::Plan>> plans;
-    int variant = -1;       // kernel shape chosen by the autotuner (-1: not tuned yet)
+    nf::Tuned tuned[2];  // kernel shape by engine (NF_ENGINE_*), as chosen by the autotuner
+    int engine = 0;      // of the plan built last
     float eps = 0.f;        // the box's own softening parameter (0: the context's)
-    float tune_ms[8] = {};  // kernel time of each candidate during tuning
     size_t device_bytes() const;
 };
-
-namespace nf {
-// A kernel shape chosen by the autotuner, and what each candidate took.
-struct Tuned {
-    int variant = -1;
-    float ms[8] = {};
-};
-}  // namespace nf
 
 struct nf_ctx {
     nf_config cfg{};
@@ -214,9 +214,7 @@ struct nf_ctx {
     // device memory of boxes and plans; freed blocks up to 1/32 of the device
     // stay here for the next box, until nf_shutdown
     cudaMemPool_t pool = nullptr;
-    // shapes chosen so far, by size of the work: (log2 of the range's
-    // particles, log2 of their mean number of pairs)
-    std::map<std::pair<int, int>, nf::Tuned> tuned;
+    std::map<nf::TuneKey, nf::Tuned> tuned;  // shapes chosen so far
     // plain drop-in GPU control (nf_sic.cu)
     struct Sic;
     Sic *sic = nullptr;

@@ -901,12 +901,6 @@ MutualFn shape(int v) {
     }
 }
 
-// Kernels without a choice of shapes (the density channel, the cubic
-// softenings) run shape 0.
-bool tunable(int soft, bool dens) {
-    return !dens && (soft == SOFT_PLUMMER || soft == SOFT_SINGLE_SPLINE);
-}
-
 MutualFn pick(int soft, bool dens, int v) {
     switch (soft) {
     case SOFT_PLUMMER: return dens ? shape_fn<SOFT_PLUMMER, true, 0>() : shape<SOFT_PLUMMER>(v);

@@ -287,6 +287,12 @@ inline PairConst pair_const(const nf_config &cfg, float eps, Step step) {
     return pc;
 }
 
+// Whether a kernel comes in several shapes (either engine): the density
+// channel and the cubic softenings have shape 0 only.
+inline bool tunable(int soft, bool dens) {
+    return !dens && (soft == SOFT_PLUMMER || soft == SOFT_SINGLE_SPLINE);
+}
+
 // Whether sources are told near from far for a softening.
 __host__ __device__ constexpr bool has_near(int soft) {
     return soft == SOFT_SINGLE_SPLINE || soft == SOFT_CUBIC_SPLINE;

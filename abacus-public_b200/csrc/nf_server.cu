@@ -256,7 +256,7 @@ static nf_status launch_request(nf_server *s, Req *r, Slot &sl, const Plan *pl) 
         L.part = sl.part;
         L.p0 = pl->p0;
         L.n_range = pl->n_range;
-        L.variant = engine_box_variant();
+        L.variant = pl->variant;
         L.grid = pl->grid;
         L.eps = r->box->eps;
         st = engine_launch(ctx, L, 0.0, sl.stream);

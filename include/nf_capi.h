@@ -89,7 +89,8 @@ typedef struct nf_config {
     int out_kind;           /* NF_OUT_* */
     int sinks_per_lane;     /* 0 = tile shapes from the occupancy; else cap at 1, 2 or 4 */
     int kernel_variant;     /* -1 = autotuned per box; else a fixed kernel shape
-                               0 .. nf_kernel_variant_count()-1 */
+                               0 .. nf_kernel_variant_count()-1 of whichever engine runs
+                               (softenings and options with one shape run that) */
 } nf_config;
 
 typedef struct nf_ctx nf_ctx;
@@ -368,7 +369,7 @@ typedef struct nf_timing {
     uint64_t padded_pairs;/* pairs including null-padded lanes/sources */
     int launches;         /* kernel launches of the call */
     int items;            /* warp work items */
-    int variant;          /* kernel shape that ran */
+    int variant;          /* kernel shape that ran, of the engine that ran (nf_last_engine) */
 } nf_timing;
 /* Timing of the last nf_box_forces on this context. */
 nf_status nf_last_timing(nf_ctx *ctx, nf_timing *t);
@@ -392,14 +393,22 @@ nf_status nf_last_timing(nf_ctx *ctx, nf_timing *t);
 nf_status nf_last_engine(nf_ctx *ctx, int *engine);
 
 /* Kernel shapes the autotuner chooses among (sinks per lane, unroll depth,
- * CTAs per SM).  The first nf_box_forces call on a box times every shape on
- * the requested slab range and keeps the fastest for that box, and for later
- * boxes of the context whose first call does work of the same size
- * (particles, and pairs per particle, within a factor of two). */
+ * CTAs per SM), as many for either engine.  The first nf_box_forces call on a
+ * box times every shape of the engine that the requested slab range takes and
+ * keeps the fastest for that box and engine, and for later boxes of the
+ * context whose first call is alike: the same engine, and number of slabs,
+ * particles, pairs per particle and reach of the spline in cells within a
+ * factor of two.  The shape sets the grouping of FP32 partials, so runs that
+ * choose differently differ in the last bits; nf_config.kernel_variant fixes
+ * it.  The density channel and the cubic softenings have one shape, 0, which
+ * is not timed. */
 int nf_kernel_variant_count(void);
-const char *nf_kernel_variant_name(int variant);
-/* The box's chosen shape (-1 before tuning) and the kernel time of each
- * candidate during tuning (ms[0 .. n-1]). */
+const char *nf_kernel_variant_name(int variant);                    /* mutual engine */
+const char *nf_engine_variant_name(int engine, int variant);
+/* The box's shape for the engine it took last (-1 before tuning) and the
+ * kernel times of the candidates it was chosen by (ms[0 .. n-1]): those of
+ * the box itself, or of the box of the same context the choice was taken over
+ * from; 0 where there was nothing to choose or kernel_variant is fixed. */
 nf_status nf_box_tuning(const nf_box *box, int *variant, float *ms, int n);
 
 /* ---------------- 4. serving: slab requests over resident boxes ---------------- */
