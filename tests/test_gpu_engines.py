@@ -10,7 +10,7 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 RMS, MAX = 2e-6, 1e-4
-SMALL = 1e-6  # softening length, cells: below the fixed-point range of these boxes
+SMALL = 2e-5  # softening length, cells: below the fixed-point range of these boxes
 
 
 def _check(oracle, box, soft, eps, a, R=2, sinks=None):
@@ -117,3 +117,107 @@ def test_one_shape_is_not_tuned(capi, synth, kw):
                 db.close()
     for o in outs:
         np.testing.assert_allclose(o, outs[0], rtol=0, atol=2e-6 * np.abs(outs[0]).max())
+
+
+def _engine_of(capi, drv):
+    e = ctypes.c_int(-1)
+    capi.check(capi.lib().nf_last_engine(capi.lib().nf_driver_context(drv.h), ctypes.byref(e)))
+    return e.value
+
+
+@pytest.mark.parametrize("pinned", [0, 1])
+@pytest.mark.parametrize("nodes", [[None], [(11, 5), (3, 8)]])
+@pytest.mark.parametrize("soft,plain", [(0, 1), (1, 1), (2, 1), (3, 1), (0, 0), (1, 0), (2, 0), (3, 0)])
+def test_drop_in_on_the_one_sided_engine(capi, oracle, synth, soft, plain, nodes, pinned):
+    """SICs that the mutual engine's lists do not serve: plain accumulation, and
+    compensated with a tiny softening; whole domain and a 2D split whose nodes
+    lie across z = 0, buffers pinned and not."""
+    box = synth.clustered_box(20000, 13, seed=6, n_clumps=15)
+    length = synth.plummer_eps(27) if plain else SMALL / 13
+    acc = capi.ACC_PLAIN if plain else capi.ACC_COMPENSATED
+    a = np.zeros((box.n, 4), np.float32)
+    for node in nodes:
+        drv = capi.Driver(box, softening=soft, softening_length=length, direct_bpd=2, node_z=node,
+                          accumulation=acc, use_pinned=pinned)
+        try:
+            got = drv.run_all()
+            assert _engine_of(capi, drv) == capi.ENGINE_ONE_SIDED
+            m = drv.slabs.mask if node else np.ones(box.n, bool)
+        finally:
+            drv.close()
+        a[m] = got[m]
+    _check(oracle, box, soft, synth.kernel_eps(soft, length), a, sinks=np.arange(0, box.n, 9))
+
+
+@pytest.mark.parametrize("soft", [0, 1, 2, 3])
+@pytest.mark.parametrize("dens", [False, True])
+def test_allocation_free_call_on_the_one_sided_engine(capi, oracle, synth, soft, dens):
+    """nf_forces_noalloc with plain accumulation, and with a tiny softening:
+    whole boxes and slab ranges, with and without the density channel."""
+    import torch
+    box = synth.clustered_box(15000, 9, seed=7, n_clumps=10)
+    b2 = float(np.float32((0.2 / box.cpd) ** 2)) if dens else 0.0
+    pos = torch.zeros((box.n, 4), device="cuda")
+    for k, v in enumerate((box.x, box.y, box.z)):
+        pos[:, k] = torch.from_numpy(v).cuda()
+    cs = torch.from_numpy(box.cell_start).cuda()
+    c2 = box.cpd ** 2
+    for acc, cells in ((capi.ACC_PLAIN, 0.02), (capi.ACC_COMPENSATED, SMALL)):
+        eps = synth.kernel_eps(soft, cells / box.cpd)
+        cfg = capi.default_config(softening=soft, eps=eps, b2=b2, accumulation=acc)
+        for lo, hi in ((0, box.cpd), (4, 6)):
+            p0, p1 = int(box.cell_start[lo * c2]), int(box.cell_start[hi * c2])
+            out = torch.full((p1 - p0, 4), float("nan"), device="cuda")
+            capi.check(capi.lib().nf_forces_noalloc(
+                ctypes.byref(cfg), box.cpd, pos.data_ptr(), cs.data_ptr(), lo, hi, out.data_ptr(),
+                ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
+            a = out.cpu().numpy()
+            sinks = np.arange(p0, p1, 5)
+            rms, mx, _ = oracle.frac_errors(a[::5, :3], oracle.fp64_sinks(box, soft, eps, sinks))
+            assert rms <= RMS and mx <= MAX, (rms, mx)
+            if dens:  # positive terms, FP32 sums
+                np.testing.assert_allclose(a[::5, 3], oracle.fp64_density(box, b2, sinks), rtol=1e-5,
+                                           atol=1e-6 * b2)
+            else:
+                assert np.all(a[:, 3] == 0)
+
+
+@pytest.mark.parametrize("soft", [0, 1, 2, 3])
+@pytest.mark.parametrize("cells", [0.02, 0.09, 0.3])
+def test_density_of_every_softening(capi, oracle, synth, soft, cells):
+    """The density channel beside every softening, from lengths far below the
+    density radius (0.2 cells) to above it, on both engines."""
+    box = synth.clustered_box(15000, 9, seed=8, n_clumps=10)
+    b2 = float(np.float32((0.2 / box.cpd) ** 2))
+    eps = synth.kernel_eps(soft, cells / box.cpd)
+    sinks = np.arange(0, box.n, 4)
+    want = oracle.fp64_density(box, b2, sinks)
+    for acc, engine in ((capi.ACC_COMPENSATED, capi.ENGINE_MUTUAL), (capi.ACC_PLAIN, capi.ENGINE_ONE_SIDED)):
+        with capi.Context(softening=soft, eps=eps, b2=b2, accumulation=acc) as ctx:
+            db = ctx.box(box)
+            a = db.forces()
+            assert ctx.last_engine() == engine
+            db.close()
+        np.testing.assert_allclose(a[sinks, 3], want, rtol=1e-5, atol=1e-6 * b2)
+        _check(oracle, box, soft, eps, a, sinks=sinks)
+
+
+def test_serving_on_the_one_sided_engine(capi, synth):
+    """Served slabs of plain and of tiny-softening boxes: the bits of the same
+    slabs swept alone."""
+    box = synth.clustered_box(15000, 9, seed=9, n_clumps=10)
+    for acc, cells in ((capi.ACC_PLAIN, 0.02), (capi.ACC_COMPENSATED, SMALL)):
+        with capi.Context(softening=0, eps=synth.kernel_eps(0, cells / 9), accumulation=acc,
+                          kernel_variant=0) as ctx:
+            db = ctx.box(box)
+            alone = [db.forces(s, s + 1) for s in range(9)]
+            srv = capi.Server(ctx)
+            outs = [np.full_like(a, np.nan) for a in alone]
+            tickets = [srv.submit(db, s, outs[s]) for s in (4, 0, 8, 1, 2, 7, 3, 5, 6)]
+            for t in tickets:
+                srv.wait(t)
+            assert ctx.last_engine() == capi.ENGINE_ONE_SIDED
+            srv.close()
+            db.close()
+        for a, b in zip(alone, outs):
+            assert np.array_equal(a.view(np.uint32), b.view(np.uint32))

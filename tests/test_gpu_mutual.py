@@ -98,17 +98,19 @@ def test_slab_ranges(capi, oracle, synth, R):
 
 def test_softening_below_the_fixed_point_range(capi, oracle, synth):
     """A softening so small that fixed point would not resolve ordinary pairs
-    takes the one-sided sweep: the results are as good."""
+    takes the one-sided sweep: the results are as good.  2e-4 and 3e-6 lie on
+    either side of the limit of this box for every softening (a pencil meets at
+    least 2000 sources: see nf_last_engine in the header)."""
     box = synth.uniform_box(6000, 7, seed=72)
     for soft in (0, 1, 2, 3):
-        for length in (1e-3 / 18, 1e-9):
+        for length, want in ((2e-4, capi.ENGINE_MUTUAL), (3e-6, capi.ENGINE_ONE_SIDED),
+                             (4e-7, capi.ENGINE_ONE_SIDED)):
             eps = synth.kernel_eps(soft, length)
             with capi.Context(softening=soft, eps=eps) as ctx:
                 db = ctx.box(box)
                 a = db.forces()
+                assert ctx.last_engine() == want
                 db.close()
-            if soft == 3 and length < 1e-8:
-                continue  # eps^3 is below the reference's own TAU2 floor
             _check(oracle, box, soft, eps, a, step=3)
 
 
