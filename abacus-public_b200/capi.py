@@ -208,6 +208,7 @@ EXPORTS = {
     "nf_box_update": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p,
                                      ctypes.c_void_p, ctypes.c_void_p]),
     "nf_box_destroy": (None, [ctypes.c_void_p, ctypes.c_void_p]),
+    "nf_trim": (None, []),
     "nf_box_device_bytes": (ctypes.c_size_t, [ctypes.c_void_p]),
     "nf_box_set_eps": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_float]),
     "nf_box_forces": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int,

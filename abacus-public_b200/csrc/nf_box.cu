@@ -1174,7 +1174,7 @@ extern "C" nf_status nf_box_create(nf_ctx *ctx, int cpd, int64_t np, const int64
     box->cpd = cpd;
     box->np = np;
     box->cell_start.assign(cell_start, cell_start + ncell + 1);
-    std::unique_lock<std::mutex> lk(ctx->mu);  // the context's stream and pool
+    std::unique_lock<std::mutex> lk(ctx->mu);  // the context's stream
     if (pool_alloc(ctx, &box->d_pos, (size_t)std::max<int64_t>(np, 1) * sizeof(float4)) != cudaSuccess ||
         pool_alloc(ctx, &box->d_cs, (size_t)(ncell + 1) * sizeof(int64_t)) != cudaSuccess) {
         pool_free(ctx, box->d_pos);
@@ -1259,7 +1259,9 @@ static nf_status upload_scratch(nf_ctx *ctx, nf_box *box, OrderScratch &o) {
     const size_t kb = ((size_t)n * 8 + 255) & ~(size_t)255, vb = ((size_t)n * 4 + 255) & ~(size_t)255;
     const size_t need = 2 * kb + vb + o.temp_bytes;
     if (box->sort_bytes < need) {
+        NF_CUDA(cudaDeviceSynchronize());
         pool_free(ctx, box->d_sort);
+        box->d_sort = nullptr;
         box->sort_bytes = 0;
         if (pool_alloc(ctx, &box->d_sort, need) != cudaSuccess) {
             set_error("nf_box_update: device allocation failed (ordering scratch)");
@@ -1408,7 +1410,8 @@ static nf_status ensure_scratch(nf_ctx *ctx, nf_box *box, const Plan &pl) {
         pl.mutual ? mutual_scratch_bytes(pl.n_range, nc)
                   : (size_t)(2 * ctx->cfg.near_field_radius + 1) * nc * (size_t)pl.n_range * sizeof(Partial);
     if (need <= box->part_bytes) return NF_OK;
-    pool_free(ctx, box->d_part);  // no call is in flight on it: each waits for its own work
+    NF_CUDA(cudaDeviceSynchronize());  // a call that failed may have left work behind
+    pool_free(ctx, box->d_part);
     box->d_part = nullptr;
     box->part_bytes = 0;
     for (auto &kv : box->plans)
@@ -1715,6 +1718,7 @@ extern "C" nf_status nf_box_step(nf_ctx *ctx, nf_box *box, const float *x, const
     bool two = true;
     for (Plan *pl : pls) two = two && pl->mutual;
     if (two && box->part2_bytes < box->part_bytes) {
+        NF_CUDA(cudaDeviceSynchronize());
         pool_free(ctx, box->d_part2);
         box->d_part2 = nullptr;
         box->part2_bytes = 0;

@@ -26,12 +26,94 @@ nf_status cuda_fail(cudaError_t e, const char *what) {
 
 using namespace nf;
 
-// On the library's own stream, whatever stream the caller has set: it lives as
-// long as the context.  A block is handed out once it is usable on any stream,
-// and every call waits for its own work before it frees one.
-cudaError_t nf::pool_alloc(nf_ctx *ctx, void **p, size_t bytes) {
-    cudaError_t e = cudaMallocFromPoolAsync(p, bytes ? bytes : 16, ctx->pool, ctx->own_stream);
-    if (e == cudaSuccess && ctx->stream != ctx->own_stream) e = cudaStreamSynchronize(ctx->own_stream);
+// Every cache of the process, for trim_all().
+static std::mutex g_caches_mu;
+static std::vector<DeviceCache *> g_caches;
+
+DeviceCache::DeviceCache() {
+    std::lock_guard<std::mutex> lk(g_caches_mu);
+    g_caches.push_back(this);
+}
+
+DeviceCache::~DeviceCache() {
+    {
+        std::lock_guard<std::mutex> lk(g_caches_mu);
+        g_caches.erase(std::find(g_caches.begin(), g_caches.end(), this));
+    }
+    trim();
+}
+
+void DeviceCache::trim() {
+    std::lock_guard<std::mutex> lk(mu);
+    for (const Block &b : kept) cudaFree(b.p);
+    kept.clear();
+    kept_bytes = 0;
+}
+
+void DeviceCache::trim_all() {
+    std::lock_guard<std::mutex> lk(g_caches_mu);
+    for (DeviceCache *c : g_caches) c->trim();
+}
+
+cudaError_t DeviceCache::alloc(void **p, size_t bytes) {
+    // sixteenths of a power of two, so that a block fits the next box's list or
+    // sums too; blocks that are not kept anyway as they are
+    size_t step = 512;
+    while (step * 32 <= bytes) step *= 2;
+    if (bytes <= KEEP_BYTES) bytes = std::max((bytes + step - 1) / step, (size_t)1) * step;
+    const size_t spare = std::max(bytes / 8, (size_t)1 << 18);
+    {
+        std::lock_guard<std::mutex> lk(mu);
+        auto best = kept.end();  // the smallest that holds it without much to spare
+        for (auto it = kept.begin(); it != kept.end(); ++it)
+            if (it->bytes >= bytes && it->bytes - bytes <= spare &&
+                (best == kept.end() || it->bytes < best->bytes))
+                best = it;
+        if (best != kept.end()) {
+            *p = best->p;
+            used[best->p] = best->bytes;
+            kept_bytes -= best->bytes;
+            kept.erase(best);
+            return cudaSuccess;
+        }
+    }
+    const cudaError_t e = device_malloc(p, bytes);
+    if (e == cudaSuccess) {
+        std::lock_guard<std::mutex> lk(mu);
+        used[*p] = bytes;
+    }
+    return e;
+}
+
+void DeviceCache::free(void *p) {
+    std::vector<void *> out;
+    {
+        std::lock_guard<std::mutex> lk(mu);
+        auto it = used.find(p);
+        const size_t bytes = it == used.end() ? 0 : it->second;
+        if (it != used.end()) used.erase(it);
+        if (bytes == 0 || bytes > KEEP_BYTES) {
+            out.push_back(p);
+        } else {
+            kept.push_back(Block{p, bytes});
+            kept_bytes += bytes;
+            while (kept_bytes > KEEP_BYTES || kept.size() > KEEP_BLOCKS) {
+                out.push_back(kept.front().p);
+                kept_bytes -= kept.front().bytes;
+                kept.pop_front();
+            }
+        }
+    }
+    for (void *q : out) cudaFree(q);
+}
+
+cudaError_t nf::device_malloc(void **p, size_t bytes) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        DeviceCache::trim_all();
+        e = cudaMalloc(p, bytes);
+    }
     if (e != cudaSuccess) {
         cudaGetLastError();
         *p = nullptr;
@@ -39,9 +121,11 @@ cudaError_t nf::pool_alloc(nf_ctx *ctx, void **p, size_t bytes) {
     return e;
 }
 
+cudaError_t nf::pool_alloc(nf_ctx *ctx, void **p, size_t bytes) { return ctx->memory.alloc(p, bytes); }
+
 void nf::pool_free(nf_ctx *ctx, void *p) {
     if (!p) return;
-    if (ctx) cudaFreeAsync(p, ctx->own_stream);
+    if (ctx) ctx->memory.free(p);
     else cudaFree(p);
 }
 
@@ -160,20 +244,6 @@ extern "C" nf_status nf_init(const nf_config *cfg, nf_ctx **out) {
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->own_stream, cudaStreamNonBlocking);
     ctx->stream = ctx->own_stream;
     for (int i = 0; i < 4 && e == cudaSuccess; i++) e = cudaEventCreate(&ctx->ev[i]);
-    if (e == cudaSuccess) {
-        cudaMemPoolProps pp{};
-        pp.allocType = cudaMemAllocationTypePinned;
-        pp.location.type = cudaMemLocationTypeDevice;
-        pp.location.id = cfg->device;
-        e = cudaMemPoolCreate(&ctx->pool, &pp);
-    }
-    if (e == cudaSuccess) {
-        size_t freeb = 0, total = 0;
-        e = cudaMemGetInfo(&freeb, &total);
-        uint64_t keep = total / 32;
-        if (e == cudaSuccess)
-            e = cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep);
-    }
     if (e != cudaSuccess) {
         nf_status s2 = cuda_fail(e, "nf_init");
         nf_shutdown(ctx);
@@ -193,9 +263,10 @@ extern "C" void nf_shutdown(nf_ctx *ctx) {
     for (int i = 0; i < 4; i++)
         if (ctx->ev[i]) cudaEventDestroy(ctx->ev[i]);
     if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
-    if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
     delete ctx;
 }
+
+extern "C" void nf_trim(void) { DeviceCache::trim_all(); }
 
 extern "C" nf_status nf_set_stream(nf_ctx *ctx, void *stream) {
     if (!ctx) {
@@ -240,7 +311,7 @@ extern "C" nf_status nf_measure_fp32_peak(nf_ctx *ctx, double seconds_sustained,
     NF_CUDA(cudaSetDevice(ctx->device));
     const int threads = 256, blocks = ctx->sms * 8, iters = 4096;
     float *out = nullptr;
-    NF_CUDA(cudaMalloc(&out, (size_t)blocks * threads * sizeof(float)));
+    NF_CUDA(device_malloc(&out, (size_t)blocks * threads * sizeof(float)));
     // FMA = 2 flops, two FMAs per paired instruction
     const double flops = 2.0 * 2.0 * PEAK_CHAINS * PEAK_UNROLL * (double)iters * blocks * threads;
     cudaStream_t s = ctx->stream;

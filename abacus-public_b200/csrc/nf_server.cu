@@ -214,9 +214,19 @@ static nf_status apply_booking(nf_server *s, Booking &bk) {
     sl.out = nullptr;
     sl.counters = nullptr;
     void *p = nullptr, *o = nullptr, *c = nullptr;
-    cudaError_t e = cudaMallocFromPoolAsync(&p, bk.part, s->pool, st);
-    if (e == cudaSuccess) e = cudaMallocFromPoolAsync(&o, bk.out, s->pool, st);
-    if (e == cudaSuccess) e = cudaMallocFromPoolAsync(&c, 256, s->pool, st);
+    auto get = [&](void **q, size_t bytes) {
+        cudaError_t e = cudaMallocFromPoolAsync(q, bytes, s->pool, st);
+        if (e == cudaErrorMemoryAllocation) {
+            cudaGetLastError();
+            DeviceCache::trim_all();
+            e = cudaMallocFromPoolAsync(q, bytes, s->pool, st);
+        }
+        if (e != cudaSuccess) *q = nullptr;
+        return e;
+    };
+    cudaError_t e = get(&p, bk.part);
+    if (e == cudaSuccess) e = get(&o, bk.out);
+    if (e == cudaSuccess) e = get(&c, 256);
     if (e != cudaSuccess) {
         cudaGetLastError();
         for (void *q : {p, o, c})
@@ -374,10 +384,7 @@ extern "C" nf_status nf_server_start(nf_ctx *ctx, const nf_server_config *cfg, n
         set_error("nf_server_start: max_inflight above 256");
         return NF_EINVAL;
     }
-    {
-        std::lock_guard<std::mutex> lk(ctx->mu);
-        NF_CUDA(cudaMemPoolTrimTo(ctx->pool, 0));  // what the context keeps but does not use
-    }
+    DeviceCache::trim_all();  // what contexts keep but do not use
     size_t freeb = 0, total = 0;
     NF_CUDA(cudaMemGetInfo(&freeb, &total));
     s->budget = s->cfg.hbm_budget_bytes ? s->cfg.hbm_budget_bytes : (size_t)(0.9 * (double)freeb);

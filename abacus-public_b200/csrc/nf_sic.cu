@@ -130,7 +130,7 @@ static nf_status grow(nf_ctx *ctx, SicBuffer &b, size_t particles, size_t sinks,
         cudaFree(b.d_pos);
         b.d_pos = nullptr;
         b.cap_pos = 0;
-        NF_CUDA(cudaMalloc(&b.d_pos, c * sizeof(float4)));
+        NF_CUDA(device_malloc(&b.d_pos, c * sizeof(float4)));
         b.cap_pos = c;
     }
     if (block > b.cap_block) {
@@ -139,7 +139,7 @@ static nf_status grow(nf_ctx *ctx, SicBuffer &b, size_t particles, size_t sinks,
         host_free(b.h_block, b.pinned);
         b.d_block = b.h_block = nullptr;
         b.cap_block = 0;
-        NF_CUDA(cudaMalloc(&b.d_block, c));
+        NF_CUDA(device_malloc(&b.d_block, c));
         NF_CUDA(host_alloc(&b.h_block, c, b.pinned, true));
         b.cap_block = c;
     }
@@ -150,7 +150,7 @@ static nf_status grow(nf_ctx *ctx, SicBuffer &b, size_t particles, size_t sinks,
         b.d_raw = nullptr;
         b.h_raw = nullptr;
         b.cap_particles = 0;
-        NF_CUDA(cudaMalloc(&b.d_raw, 3 * c * sizeof(float)));
+        NF_CUDA(device_malloc(&b.d_raw, 3 * c * sizeof(float)));
         NF_CUDA(host_alloc((void **)&b.h_raw, 3 * c * sizeof(float), b.pinned, true));
         b.cap_particles = c;
     }
@@ -163,8 +163,8 @@ static nf_status grow(nf_ctx *ctx, SicBuffer &b, size_t particles, size_t sinks,
         b.d_out = nullptr;
         b.h_out = nullptr;
         b.cap_sinks = 0;
-        NF_CUDA(cudaMalloc(&b.d_part, (size_t)W * nc * c * sizeof(Partial)));
-        NF_CUDA(cudaMalloc(&b.d_out, c * rec));
+        NF_CUDA(device_malloc(&b.d_part, (size_t)W * nc * c * sizeof(Partial)));
+        NF_CUDA(device_malloc(&b.d_out, c * rec));
         NF_CUDA(host_alloc(&b.h_out, c * rec, b.pinned, false));
         b.cap_sinks = c;
     }
@@ -175,7 +175,7 @@ static nf_status grow(nf_ctx *ctx, SicBuffer &b, size_t particles, size_t sinks,
         b.d_items = nullptr;
         b.h_items = nullptr;
         b.cap_items = 0;
-        NF_CUDA(cudaMalloc(&b.d_items, c * sizeof(Item)));
+        NF_CUDA(device_malloc(&b.d_items, c * sizeof(Item)));
         NF_CUDA(host_alloc((void **)&b.h_items, c * sizeof(Item), b.pinned, true));
         b.cap_items = c;
     }
@@ -186,11 +186,11 @@ static nf_status grow(nf_ctx *ctx, SicBuffer &b, size_t particles, size_t sinks,
         b.d_cs = nullptr;
         b.h_cs = nullptr;
         b.cap_cells = 0;
-        NF_CUDA(cudaMalloc(&b.d_cs, c * sizeof(int64_t)));
+        NF_CUDA(device_malloc(&b.d_cs, c * sizeof(int64_t)));
         NF_CUDA(host_alloc((void **)&b.h_cs, c * sizeof(int64_t), b.pinned, true));
         b.cap_cells = c;
     }
-    if (!b.d_counters) NF_CUDA(cudaMalloc(&b.d_counters, 2 * sizeof(int)));
+    if (!b.d_counters) NF_CUDA(device_malloc(&b.d_counters, 2 * sizeof(int)));
     return NF_OK;
 }
 

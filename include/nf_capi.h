@@ -321,6 +321,12 @@ nf_status nf_box_create(nf_ctx *ctx, int cpd, int64_t np, const int64_t *cell_st
 nf_status nf_box_update(nf_ctx *ctx, nf_box *box, const float *x, const float *y,
                         const float *z);
 void nf_box_destroy(nf_ctx *ctx, nf_box *box);
+/* Device memory of destroyed boxes stays with the context for its next ones:
+ * at most 2 GiB, until nf_shutdown, nf_server_start, nf_trim, or an
+ * allocation of this library that would otherwise fail. */
+/* Give back to the device what every context of the process keeps unused (for
+ * other users of the device in the process). */
+void nf_trim(void);
 /* One whole step end to end, pipelined: upload new positions (host or
  * device x, y, z, same cell counts), sweep every slab, and copy the
  * records of all particles to out (host or device), as nf_box_update +

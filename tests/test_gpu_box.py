@@ -244,3 +244,41 @@ def test_box_rejects_cpd_beyond_32_bit_pencil_ids(capi):
                                       None, None, None, ctypes.byref(h))
         assert rc == capi.NF_EINVAL and not h.value
         assert "1290" in capi.last_error()
+
+
+def test_memory_of_destroyed_boxes(capi, synth):
+    """A context without boxes holds no device memory of its own; destroyed
+    boxes leave at most 2 GiB with it, which nf_trim and nf_shutdown give back,
+    and which the next box takes over."""
+    import torch
+    mib = 1 << 20
+
+    def free():
+        return torch.cuda.mem_get_info()[0]
+
+    box = synth.uniform_box(1_500_000, 29, seed=31)
+    with capi.Context(softening=0, eps=1e-6) as ctx:  # kernels loaded before anything is counted
+        db = ctx.box(box)
+        db.forces()
+        db.close()
+    capi.lib().nf_trim()
+    base = free()
+    ctx = capi.Context(softening=0, eps=1e-6, kernel_variant=0)
+    assert base - free() < 4 * mib
+    db = ctx.box(box)
+    want = db.forces()
+    held = base - free()
+    assert held > 64 * mib
+    db.close()
+    assert 0 < base - free() <= held <= 2 << 30
+    db = ctx.box(box)  # out of what was kept
+    assert np.array_equal(db.forces(), want)
+    assert base - free() <= held + 4 * mib
+    db.close()
+    capi.lib().nf_trim()
+    assert base - free() < 4 * mib
+    db = ctx.box(box)
+    assert np.array_equal(db.forces(), want)
+    db.close()
+    ctx.close()
+    assert base - free() < 4 * mib
