@@ -1716,13 +1716,17 @@ extern "C" nf_status nf_box_step(nf_ctx *ctx, nf_box *box, const float *x, const
     // Chunks are swept on the context's stream and a second one in turn, each
     // with its own sums: a chunk's CTAs start as the chunk before it drains
     bool two = true;
-    for (Plan *pl : pls) two = two && pl->mutual;
-    if (two && box->part2_bytes < box->part_bytes) {
+    size_t need2 = 0;  // of the largest chunk
+    for (Plan *pl : pls) {
+        two = two && pl->mutual;
+        need2 = std::max(need2, mutual_scratch_bytes(pl->n_range, ctx->cfg.b2 > 0.f ? 4 : 3));
+    }
+    if (two && box->part2_bytes < need2) {
         NF_CUDA(cudaDeviceSynchronize());
         pool_free(ctx, box->d_part2);
         box->d_part2 = nullptr;
         box->part2_bytes = 0;
-        if (pool_alloc(ctx, &box->d_part2, box->part_bytes) == cudaSuccess) box->part2_bytes = box->part_bytes;
+        if (pool_alloc(ctx, &box->d_part2, need2) == cudaSuccess) box->part2_bytes = need2;
         else two = false;
     }
     if (two && !box->s_sweep) NF_CUDA(cudaStreamCreateWithFlags(&box->s_sweep, cudaStreamNonBlocking));

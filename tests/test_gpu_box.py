@@ -282,3 +282,21 @@ def test_memory_of_destroyed_boxes(capi, synth):
     db.close()
     ctx.close()
     assert base - free() < 4 * mib
+
+
+def test_step_scratch_is_a_chunks(capi, synth):
+    """The pipelined step after a sweep of the whole box: positions staged
+    (12 bytes a particle), a record buffer per chunk (16), work lists, and a
+    second set of sums for the largest chunk only (25 bytes a particle would be
+    the whole box again; a chunk of 3 of 17 slabs holds a sixth)."""
+    box = synth.uniform_box(64 ** 3, 17, seed=32)
+    with capi.Context(softening=0, eps=1e-6, kernel_variant=0) as ctx:
+        db = ctx.box(box)
+        db.forces()
+        before = db.device_bytes()
+        out = np.empty((box.n, 4), np.float32)
+        db.step(box.x, box.y, box.z, out)
+        assert db.device_bytes() - before < (12 + 16 + 15) * box.n
+        want = db.forces()
+        db.close()
+    np.testing.assert_allclose(out, want, rtol=0, atol=2e-6 * np.abs(want).max())
