@@ -2,11 +2,10 @@
 // admission.
 //
 // A dispatcher thread admits queued requests oldest first whenever a slot is
-// free and the request's device memory (pencil partials, counters, output)
-// fits the HBM budget, and launches each admitted request on its slot's own
-// stream: the box's cached slab plan (built and autotuned on first use)
-// drives one persistent pencil-kernel launch, the co-add and the copy to the
-// caller's buffer.  Requests admitted while others run overlap with them on
+// free and the request's device memory (sums, counters, output) fits the HBM
+// budget, and launches each admitted request on its slot's own stream: the
+// box's cached slab plan (built and autotuned on first use) drives one
+// persistent sweep launch, the co-add and the copy to the caller's buffer.  Requests admitted while others run overlap with them on
 // the device (a persistent grid's tail is filled by the next request's
 // CTAs; copies overlap kernels).  A host callback after the copy marks the
 // request complete and frees its slot; latency is submit -> that callback.
@@ -33,7 +32,7 @@ struct Req;
 struct Slot {
     int index = 0;
     cudaStream_t stream = nullptr;
-    Partial *part = nullptr;
+    void *part = nullptr;  // the sums
     void *out = nullptr;
     int *counters = nullptr;
     size_t part_cap = 0, out_cap = 0;  // bytes
@@ -137,12 +136,13 @@ struct Booking {
     std::vector<void *> release_ptrs;  // their buffers, taken at booking time
 };
 
-// Device bytes of a slab request: partials (one record of nc (hi, lo) pairs per
-// sink and pencil slot) and the output records.
-static void request_bytes(const nf_server *s, int64_t nsink, size_t *part, size_t *out) {
+// Device bytes of a slab request: the sums (mutual: fixed point; one-sided:
+// one record of nc (hi, lo) pairs per sink and pencil slot) and the output
+// records.
+static void request_bytes(const nf_server *s, bool mutual, int64_t nsink, size_t *part, size_t *out) {
     const int W = 2 * s->ctx->cfg.near_field_radius + 1;
     const int nc = s->ctx->cfg.b2 > 0.f ? 4 : 3;
-    *part = (size_t)W * nc * (size_t)nsink * sizeof(Partial) + 16;
+    *part = (mutual ? mutual_scratch_bytes(nsink, nc) : (size_t)W * nc * (size_t)nsink * sizeof(Partial)) + 16;
     *out = (size_t)nsink * rec_bytes(s->ctx) + 16;
 }
 
@@ -183,14 +183,14 @@ static bool try_book(nf_server *s, Slot &sl, size_t gp, size_t go, Booking &bk) 
     return true;
 }
 
-static bool book_slot(nf_server *s, Slot &sl, const nf_box *box, size_t part_need,
+static bool book_slot(nf_server *s, Slot &sl, const nf_box *box, bool mutual, size_t part_need,
                       size_t out_need, Booking &bk) {
     bk = Booking{};
     bk.slot = &sl;
     if (sl.part_cap >= part_need && sl.out_cap >= out_need && sl.counters) return true;
     // grow to the box's largest slab if the budget allows, else to this request
     size_t pm, om;
-    request_bytes(s, largest_slab(box), &pm, &om);
+    request_bytes(s, mutual, largest_slab(box), &pm, &om);
     pm = std::max({pm, part_need, sl.part_cap});
     om = std::max({om, out_need, sl.out_cap});
     if (try_book(s, sl, pm, om, bk)) return true;
@@ -234,7 +234,7 @@ static nf_status apply_booking(nf_server *s, Booking &bk) {
         set_error("nf_server: device allocation failed within the HBM budget");
         return NF_ENOMEM;
     }
-    sl.part = (Partial *)p;
+    sl.part = p;
     sl.out = o;
     sl.counters = (int *)c;
     return NF_OK;
@@ -263,7 +263,7 @@ static nf_status launch_request(nf_server *s, Req *r, Slot &sl, const Plan *pl) 
         L.light = pl->d_light;
         L.n_light = pl->n_light;
         L.counters = sl.counters;
-        L.part = sl.part;
+        L.part = (Partial *)sl.part;
         L.p0 = pl->p0;
         L.n_range = pl->n_range;
         L.variant = pl->variant;
@@ -329,13 +329,13 @@ static void dispatcher_main(nf_server *s) {
             continue;
         }
         size_t part_need, out_need;
-        request_bytes(s, pl->n_range, &part_need, &out_need);
+        request_bytes(s, pl->mutual, pl->n_range, &part_need, &out_need);
         Slot *pick = nullptr;  // a free slot, preferring one already large enough
         for (auto &sl : s->slots)
             if (!sl.req && (!pick || (sl.part_cap >= part_need && pick->part_cap < part_need)))
                 pick = &sl;
         Booking bk;
-        if (!pick || !book_slot(s, *pick, r->box, part_need, out_need, bk)) {
+        if (!pick || !book_slot(s, *pick, r->box, pl->mutual, part_need, out_need, bk)) {
             if (s->running == 0) {  // nothing in flight will free memory
                 s->pending.pop_front();
                 r->state = -1;
@@ -421,8 +421,9 @@ extern "C" nf_status nf_server_submit(nf_server *s, nf_box *box, int slab, void 
         return NF_EINVAL;
     }
     int64_t c2 = (int64_t)box->cpd * box->cpd;
+    // refused here only if it might not fit: on the engine that takes more
     size_t pb, ob;
-    request_bytes(s, box->cell_start[(slab + 1) * c2] - box->cell_start[slab * c2], &pb, &ob);
+    request_bytes(s, false, box->cell_start[(slab + 1) * c2] - box->cell_start[slab * c2], &pb, &ob);
     size_t need = pb + ob + 256;
     std::lock_guard<std::mutex> lk(s->mu);
     s->submitted++;
@@ -618,7 +619,7 @@ extern "C" void nf_server_stop(nf_server *s) {
     cudaSetDevice(s->ctx->device);
     for (auto &sl : s->slots) {
         if (!sl.stream) continue;
-        for (void *q : {(void *)sl.part, sl.out, (void *)sl.counters})
+        for (void *q : {sl.part, sl.out, (void *)sl.counters})
             if (q) cudaFreeAsync(q, sl.stream);
         cudaStreamSynchronize(sl.stream);
         cudaStreamDestroy(sl.stream);

@@ -175,3 +175,21 @@ def test_per_box_softening(capi, synth, two_boxes):
     served = np.concatenate(outs)
     assert np.array_equal(served.view(np.uint32), want_slabs.view(np.uint32))
     np.testing.assert_allclose(served, want, rtol=0, atol=2e-6 * np.abs(want).max())
+
+
+def test_requests_book_what_their_engine_uses(capi, synth, two_boxes):
+    """Two slots of one box hold the sums (25 bytes a sink in fixed point, 120
+    as pencil partials) and the records (16) of its largest slab, no more."""
+    boxa, _ = two_boxes
+    nmax = max(boxa.slab_range(s)[1] - boxa.slab_range(s)[0] for s in range(boxa.cpd))
+    for acc, per_sink in ((capi.ACC_COMPENSATED, 25), (capi.ACC_PLAIN, 120)):
+        with capi.Context(softening=0, eps=synth.kernel_eps(0, synth.plummer_eps(40)),
+                          accumulation=acc) as ctx:
+            da = ctx.box(boxa)
+            with capi.Server(ctx, max_inflight=2) as srv:
+                outs = [_slab_out(da, s) for s in range(boxa.cpd)]
+                for t in [srv.submit(da, s, outs[s]) for s in range(boxa.cpd)]:
+                    srv.wait(t)
+                peak = srv.stats().hbm_peak_bytes
+                assert (per_sink + 16) * nmax <= peak <= 2 * ((per_sink + 16) * nmax + 1024)
+            da.close()
