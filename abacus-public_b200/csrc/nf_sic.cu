@@ -50,14 +50,14 @@ struct SicBuffer {
     float4 *d_pos = nullptr;
     int64_t *d_cs = nullptr;
     Item *d_items = nullptr;
-    Partial *d_part = nullptr;
+    void *d_part = nullptr;  // the sums: fixed point, or pencil partials
     void *d_out = nullptr;
     int *d_counters = nullptr;
     float *h_raw = nullptr;
     void *h_out = nullptr;
     int64_t *h_cs = nullptr;
     Item *h_items = nullptr;
-    size_t cap_particles = 0, cap_sinks = 0, cap_items = 0, cap_cells = 0;
+    size_t cap_particles = 0, cap_sinks = 0, cap_part = 0, cap_items = 0, cap_cells = 0;
     // mutual form: cell table, work list and positions in one block, one copy
     void *h_block = nullptr, *d_block = nullptr;
     size_t cap_block = 0, cap_pos = 0;
@@ -114,7 +114,7 @@ static void release(SicBuffer &b) {
     b.h_cs = nullptr;
     b.h_items = nullptr;
     b.stream = nullptr;
-    b.cap_particles = b.cap_sinks = b.cap_items = b.cap_cells = 0;
+    b.cap_particles = b.cap_sinks = b.cap_part = b.cap_items = b.cap_cells = 0;
 }
 
 // Grow a buffer's arrays to hold a task (1.25x headroom; never shrinks).
@@ -154,16 +154,22 @@ static nf_status grow(nf_ctx *ctx, SicBuffer &b, size_t particles, size_t sinks,
         NF_CUDA(host_alloc((void **)&b.h_raw, 3 * c * sizeof(float), b.pinned, true));
         b.cap_particles = c;
     }
+    const size_t part = block ? mutual_scratch_bytes((int64_t)sinks, nc) : (size_t)W * nc * sinks * sizeof(Partial);
+    if (part > b.cap_part) {
+        size_t c = up(part);
+        cudaFree(b.d_part);
+        b.d_part = nullptr;
+        b.cap_part = 0;
+        NF_CUDA(device_malloc(&b.d_part, c));
+        b.cap_part = c;
+    }
     if (sinks > b.cap_sinks) {
         size_t c = up(sinks);
-        cudaFree(b.d_part);
         cudaFree(b.d_out);
         host_free(b.h_out, b.pinned);
-        b.d_part = nullptr;
         b.d_out = nullptr;
         b.h_out = nullptr;
         b.cap_sinks = 0;
-        NF_CUDA(device_malloc(&b.d_part, (size_t)W * nc * c * sizeof(Partial)));
         NF_CUDA(device_malloc(&b.d_out, c * rec));
         NF_CUDA(host_alloc(&b.h_out, c * rec, b.pinned, false));
         b.cap_sinks = c;
@@ -467,7 +473,7 @@ static nf_status launch_tiles(nf_ctx *ctx, SicBuffer &b, const SicTask &t, int64
     L.light = b.d_items + (size_t)n_split * ENGINE_WARPS_PER_CTA;
     L.n_light = (int)nitems - n_split * ENGINE_WARPS_PER_CTA;
     L.counters = b.d_counters;
-    L.part = b.d_part;
+    L.part = (Partial *)b.d_part;
     L.p0 = p0;
     L.n_range = n_sinks;
     L.variant = engine_plain_variant();
@@ -476,7 +482,7 @@ static nf_status launch_tiles(nf_ctx *ctx, SicBuffer &b, const SicTask &t, int64
     if (st != NF_OK) return st;
     NF_CUDA(cudaEventRecord(b.ev1, sm));
     *bytes_to_device = 3 * pb + cs_b + nitems * sizeof(Item);
-    return engine_coadd(ctx, b.d_part, n_sinks, b.d_out, sm);
+    return engine_coadd(ctx, (const Partial *)b.d_part, n_sinks, b.d_out, sm);
 }
 
 static nf_status run_task(nf_ctx *ctx, SicBuffer &b, const SicTask &t) {

@@ -181,3 +181,24 @@ def test_sic_timing_counts_every_sic(capi, synth, oracle):
         assert n2 == n and pairs2 == pairs and ms2 > 0.0
     finally:
         drv.close()
+
+
+def test_sic_buffers_hold_what_their_engine_uses(capi, synth):
+    """Device memory of a driver's one buffer after a sweep: positions twice (12
+    and 16 bytes a source), sums (25) and records (16) of a slab's sinks, a
+    quarter more as headroom; partials of the other engine would be 120."""
+    import torch
+    box = synth.uniform_box(2_000_000, 9, seed=46)
+    length = synth.plummer_eps(126)
+    drv = capi.Driver(synth.uniform_box(3000, 9, seed=1), softening=0, softening_length=length)
+    drv.run_all()  # kernels loaded
+    drv.close()
+    sinks = max(box.slab_range(s)[1] - box.slab_range(s)[0] for s in range(9))
+    base = torch.cuda.mem_get_info()[0]
+    drv = capi.Driver(box, softening=0, softening_length=length, direct_bpd=1)
+    try:
+        drv.run_all()
+        held = base - torch.cuda.mem_get_info()[0]
+    finally:
+        drv.close()
+    assert held <= 1.25 * sinks * (5 * 28 + 25 + 16) + (12 << 20), held
