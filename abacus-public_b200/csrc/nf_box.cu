@@ -1,9 +1,8 @@
 // nf_box.cu -- batched near-field form: positions resident in HBM, one
 // persistent launch per slab range, deterministic co-add; and the one-sided
-// pencil engine.  Boxes are swept by the mutual engine (nf_mutual.cu) except
-// with plain accumulation or a softening below its fixed-point range; the
-// one-sided engine below serves those, the plain drop-in and the
-// allocation-free entry point.
+// pencil engine.  Boxes, drop-in SICs and the allocation-free call run on the
+// mutual engine (nf_mutual.cu); the one-sided engine below serves all three
+// with plain accumulation and where a softening is below the fixed-point range.
 //
 // Work decomposition (the reference's pencil-on-pencil scheme,
 // singlestep/Direct/SetInteractionCollection.hh:4-35 and
@@ -73,7 +72,6 @@ struct KParams {
     float zshift[MAXW];   // (a-R) h, sink cell a of the pencil
     float xyshift[MAXW];  // n h, n = -R .. R
     signed char odx[MAXSRC], ody[MAXSRC];  // source cell order: outer ring first
-    int n_outer;                           // cells with max(|dx|,|dy|) == 2
     // single spline: a source can be closer than eps to one of a tile's
     // sinks only if it lies within near_w (eps plus a rounding allowance) of
     // the tile's sink bounding box
@@ -95,10 +93,6 @@ struct WarpSmem {
     int64_t sstart[MAXW];
     int32_t spre[MAXW + 1];
 };
-
-__device__ __forceinline__ int wrapc(int i, int cpd) {
-    return i < 0 ? i + cpd : (i >= cpd ? i - cpd : i);
-}
 
 __device__ __forceinline__ int warp_incl_scan(int v, int lane) {
 #pragma unroll
@@ -154,13 +148,7 @@ __device__ __forceinline__ float4 load_src(const KParams &kp, const WarpSmem &ws
     float4 t = __ldg(&kp.pos[p]);
     t.x += ws.csx[k];
     t.y += ws.csy[k];
-    if (FLAG) {
-        const float4 bb = ws.tbb;
-        t.w = (t.x >= bb.x && t.x <= bb.y && t.y >= bb.z && t.y <= bb.w && t.z >= zlo &&
-               t.z <= zhi)
-                  ? 1.f
-                  : 0.f;
-    }
+    if (FLAG) t.w = inside(t, ws.tbb, zlo, zhi);
     return t;
 }
 
@@ -730,7 +718,7 @@ static inline int wrap_h(int i, int cpd) {
 
 // Source cell order: outer ring (max(|dx|,|dy|) == R >= 2) first, so that the
 // chunks that can hold pairs closer than one cell width come last.
-static void source_order(int R, signed char *odx, signed char *ody, int *n_outer) {
+static void source_order(int R, signed char *odx, signed char *ody) {
     int n = 0;
     for (int pass = 0; pass < 2; pass++)
         for (int dx = -R; dx <= R; dx++)
@@ -742,11 +730,6 @@ static void source_order(int R, signed char *odx, signed char *ody, int *n_outer
                     n++;
                 }
             }
-    int no = 0;
-    for (int dx = -R; dx <= R; dx++)
-        for (int dy = -R; dy <= R; dy++)
-            if (std::max(std::abs(dx), std::abs(dy)) >= 2) no++;
-    *n_outer = no;
 }
 
 struct HostTile {
@@ -924,7 +907,7 @@ static KParams params_from(nf_ctx *ctx, const EngineLaunch &L) {
         kp.zshift[a] = (float)((a - R) * h);
         kp.xyshift[a] = (float)((a - R) * h);
     }
-    source_order(R, kp.odx, kp.ody, &kp.n_outer);
+    source_order(R, kp.odx, kp.ody);
     return kp;
 }
 

@@ -110,10 +110,6 @@ __host__ __device__ __forceinline__ bool segment(const Stream &s, int R, int i, 
     return g.mask != 0 && g.e > g.b;
 }
 
-__host__ __device__ __forceinline__ int wrapc(int i, int cpd) {
-    return i < 0 ? i + cpd : (i >= cpd ? i - cpd : i);
-}
-
 // Cells, and the slabs [lo, hi) that hold the sinks.  onesided: no pair is met
 // mutually (a drop-in SIC: a sink's sum then has the same order whatever rows
 // and z cells the SIC holds).
@@ -440,13 +436,7 @@ __device__ __forceinline__ float4 load_src(const MParams &kp, const WarpSmem &ws
     float4 t = __ldg(&kp.pos[p]);
     t.x += ws.csx[k];
     t.y += ws.csy[k];
-    if (FLAG) {
-        const float4 bb = ws.tbb;
-        t.w = (t.x >= bb.x && t.x <= bb.y && t.y >= bb.z && t.y <= bb.w && t.z >= zlo &&
-               t.z <= zhi)
-                  ? 1.f
-                  : 0.f;
-    }
+    if (FLAG) t.w = inside(t, ws.tbb, zlo, zhi);
     return t;
 }
 
@@ -803,7 +793,7 @@ __global__ void __launch_bounds__(WPC * 32, MINB) mutual_kernel(const __grid_con
         const int nm = setup_tables(kp, it.pencil, ws, lane, s);
         if (it.S == 1)
             run_item<SOFT, DENS, 1, UNR>(kp, ws, hl, it, lane, s, nm);
-        else if (SMAX == 2 || it.S == 2)
+        else if (it.S == 2)
             run_item<SOFT, DENS, 2, UNR>(kp, ws, hl, it, lane, s, nm);
         else if (SMAX == 4 || it.S == 4)
             run_item<SOFT, DENS, 4, UNR>(kp, ws, hl, it, lane, s, nm);

@@ -226,6 +226,16 @@ __device__ __forceinline__ float2 pair_g_x2(float2 r2, const PairConst &pc) {
     }
 }
 
+__host__ __device__ __forceinline__ int wrapc(int i, int cpd) {
+    return i < 0 ? i + cpd : (i >= cpd ? i - cpd : i);
+}
+
+// 1 if source t lies inside a box: x in [b.x, b.y], y in [b.z, b.w], z in
+// [zlo, zhi]; else 0.
+__device__ __forceinline__ float inside(const float4 &t, const float4 &b, float zlo, float zhi) {
+    return (t.x >= b.x && t.x <= b.y && t.y >= b.z && t.y <= b.w && t.z >= zlo && t.z <= zhi) ? 1.f : 0.f;
+}
+
 // Fold a partial p into the running compensated sum (h, l) and clear it
 // (plain: one FP32 running sum).  Kahan's compensated summation with the
 // correction kept as the low part to add (the sum is h + l):
