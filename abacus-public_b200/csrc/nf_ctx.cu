@@ -26,92 +26,85 @@ nf_status cuda_fail(cudaError_t e, const char *what) {
 
 using namespace nf;
 
-// Every cache of the process, for trim_all().
-static std::mutex g_caches_mu;
-static std::vector<DeviceCache *> g_caches;
+// Every context's, for trim_all().
+static std::mutex g_memories_mu;
+static std::vector<DeviceMemory *> g_memories;
 
-DeviceCache::DeviceCache() {
-    std::lock_guard<std::mutex> lk(g_caches_mu);
-    g_caches.push_back(this);
+DeviceMemory::DeviceMemory() {
+    std::lock_guard<std::mutex> lk(g_memories_mu);
+    g_memories.push_back(this);
 }
 
-DeviceCache::~DeviceCache() {
+DeviceMemory::~DeviceMemory() {
     {
-        std::lock_guard<std::mutex> lk(g_caches_mu);
-        g_caches.erase(std::find(g_caches.begin(), g_caches.end(), this));
+        std::lock_guard<std::mutex> lk(g_memories_mu);
+        g_memories.erase(std::find(g_memories.begin(), g_memories.end(), this));
     }
-    trim();
+    close();
 }
 
-void DeviceCache::trim() {
+void DeviceMemory::close() {
     std::lock_guard<std::mutex> lk(mu);
-    for (const Block &b : kept) cudaFree(b.p);
-    kept.clear();
-    kept_bytes = 0;
+    if (!pool) return;
+    cudaStreamSynchronize(stream);
+    cudaMemPoolDestroy(pool);  // blocks still out stay valid until they are freed
+    pool = nullptr;
 }
 
-void DeviceCache::trim_all() {
-    std::lock_guard<std::mutex> lk(g_caches_mu);
-    for (DeviceCache *c : g_caches) c->trim();
+void DeviceMemory::trim() {
+    std::lock_guard<std::mutex> lk(mu);
+    if (!pool) return;
+    cudaStreamSynchronize(stream);  // frees that are still queued
+    cudaMemPoolTrimTo(pool, 0);
 }
 
-cudaError_t DeviceCache::alloc(void **p, size_t bytes) {
-    // sixteenths of a power of two, so that a block fits the next box's list or
-    // sums too; blocks that are not kept anyway as they are
-    size_t step = 512;
-    while (step * 32 <= bytes) step *= 2;
-    if (bytes <= KEEP_BYTES) bytes = std::max((bytes + step - 1) / step, (size_t)1) * step;
-    const size_t spare = std::max(bytes / 8, (size_t)1 << 18);
+void DeviceMemory::trim_all() {
+    std::lock_guard<std::mutex> lk(g_memories_mu);
+    for (DeviceMemory *m : g_memories) m->trim();
+}
+
+cudaError_t DeviceMemory::alloc(int device, cudaStream_t own, void **p, size_t bytes) {
+    *p = nullptr;
+    cudaError_t e = cudaSuccess;
+    cudaMemPool_t from;
     {
         std::lock_guard<std::mutex> lk(mu);
-        auto best = kept.end();  // the smallest that holds it without much to spare
-        for (auto it = kept.begin(); it != kept.end(); ++it)
-            if (it->bytes >= bytes && it->bytes - bytes <= spare &&
-                (best == kept.end() || it->bytes < best->bytes))
-                best = it;
-        if (best != kept.end()) {
-            *p = best->p;
-            used[best->p] = best->bytes;
-            kept_bytes -= best->bytes;
-            kept.erase(best);
-            return cudaSuccess;
+        if (!pool) {
+            cudaMemPoolProps pp{};
+            pp.allocType = cudaMemAllocationTypePinned;
+            pp.location.type = cudaMemLocationTypeDevice;
+            pp.location.id = device;
+            e = cudaMemPoolCreate(&pool, &pp);
+            uint64_t keep = KEEP_BYTES;
+            if (e == cudaSuccess) e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+            if (e != cudaSuccess) {
+                if (pool) cudaMemPoolDestroy(pool);
+                pool = nullptr;
+                cudaGetLastError();
+                return e;
+            }
+            stream = own;
         }
+        from = pool;
     }
-    const cudaError_t e = device_malloc(p, bytes);
-    if (e == cudaSuccess) {
-        std::lock_guard<std::mutex> lk(mu);
-        used[*p] = bytes;
+    e = cudaMallocFromPoolAsync(p, bytes ? bytes : 16, from, own);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        trim_all();
+        e = cudaMallocFromPoolAsync(p, bytes ? bytes : 16, from, own);
+    }
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        *p = nullptr;
     }
     return e;
-}
-
-void DeviceCache::free(void *p) {
-    std::vector<void *> out;
-    {
-        std::lock_guard<std::mutex> lk(mu);
-        auto it = used.find(p);
-        const size_t bytes = it == used.end() ? 0 : it->second;
-        if (it != used.end()) used.erase(it);
-        if (bytes == 0 || bytes > KEEP_BYTES) {
-            out.push_back(p);
-        } else {
-            kept.push_back(Block{p, bytes});
-            kept_bytes += bytes;
-            while (kept_bytes > KEEP_BYTES || kept.size() > KEEP_BLOCKS) {
-                out.push_back(kept.front().p);
-                kept_bytes -= kept.front().bytes;
-                kept.pop_front();
-            }
-        }
-    }
-    for (void *q : out) cudaFree(q);
 }
 
 cudaError_t nf::device_malloc(void **p, size_t bytes) {
     cudaError_t e = cudaMalloc(p, bytes);
     if (e == cudaErrorMemoryAllocation) {
         cudaGetLastError();
-        DeviceCache::trim_all();
+        DeviceMemory::trim_all();
         e = cudaMalloc(p, bytes);
     }
     if (e != cudaSuccess) {
@@ -121,11 +114,17 @@ cudaError_t nf::device_malloc(void **p, size_t bytes) {
     return e;
 }
 
-cudaError_t nf::pool_alloc(nf_ctx *ctx, void **p, size_t bytes) { return ctx->memory.alloc(p, bytes); }
+// A block is handed out once it is usable on any stream: it is allocated on the
+// library's own stream, whatever stream the caller has set.
+cudaError_t nf::pool_alloc(nf_ctx *ctx, void **p, size_t bytes) {
+    cudaError_t e = ctx->memory.alloc(ctx->device, ctx->own_stream, p, bytes);
+    if (e == cudaSuccess && ctx->stream != ctx->own_stream) e = cudaStreamSynchronize(ctx->own_stream);
+    return e;
+}
 
 void nf::pool_free(nf_ctx *ctx, void *p) {
     if (!p) return;
-    if (ctx) ctx->memory.free(p);
+    if (ctx) cudaFreeAsync(p, ctx->own_stream);
     else cudaFree(p);
 }
 
@@ -262,11 +261,12 @@ extern "C" void nf_shutdown(nf_ctx *ctx) {
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
     for (int i = 0; i < 4; i++)
         if (ctx->ev[i]) cudaEventDestroy(ctx->ev[i]);
+    ctx->memory.close();
     if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
     delete ctx;
 }
 
-extern "C" void nf_trim(void) { DeviceCache::trim_all(); }
+extern "C" void nf_trim(void) { DeviceMemory::trim_all(); }
 
 extern "C" nf_status nf_set_stream(nf_ctx *ctx, void *stream) {
     if (!ctx) {

@@ -7,13 +7,11 @@
 #include <condition_variable>
 #include <cstdint>
 #include <deque>
-#include <list>
 #include <map>
 #include <memory>
 #include <mutex>
 #include <string>
 #include <thread>
-#include <unordered_map>
 #include <vector>
 
 #include "nf_capi.h"
@@ -150,34 +148,32 @@ bool mutual_sic_list(const nf_config &cfg, int cpd, const std::vector<SicPencil>
                      int warps, Plan &pl, std::vector<MutualItem> &items);
 nf_status mutual_plan(nf_ctx *ctx, const nf_box *box, int lo, int hi, int variant, Plan &pl);
 nf_status mutual_launch(nf_ctx *ctx, const MutualLaunch &L, cudaStream_t st);
-// Device memory of a context's boxes and plans: cudaMalloc, with blocks that
-// come back kept for the next box, up to KEEP_BYTES and oldest out first.  A
+// Device memory of a context's boxes and plans: a memory pool of its own, made
+// when the first block is asked for (a context without boxes, as a driver's,
+// makes none).  What is freed stays for the next box, up to KEEP_BYTES: a
 // simulation that makes a box each step asks for the same blocks again (1.2 GB
-// for 256^3 particles: 55 ms a step, 60 ms with half of it kept; on larger
-// boxes cudaMalloc is a smaller part still).  Nothing is made or asked of the device before the first block, so a
-// context without boxes (a driver's) costs nothing.  Kept blocks go back to
-// the device at nf_shutdown, when a server starts, and when any allocation of
-// this library runs out (device_malloc).  A block handed to free() is idle:
-// no work that uses it is in flight.
-class DeviceCache {
+// for 256^3 particles: 55.5 ms a step, 60 ms with half of it kept).  It goes
+// back to the device at nf_shutdown, when a server starts, by nf_trim, and when
+// any allocation of this library runs out.  Against blocks from cudaMalloc kept
+// in a list: context + box + shutdown 3.2 ms beside 5.0 (128^3), and the first
+// pass of a server, whose 90 slab plans allocate while requests run, 95 ms
+// beside 107-167.  A block handed to free() is idle: no work that uses it is in
+// flight.
+class DeviceMemory {
   public:
-    static constexpr size_t KEEP_BYTES = (size_t)2 << 30, KEEP_BLOCKS = 256;
-    DeviceCache();
-    ~DeviceCache();
-    cudaError_t alloc(void **p, size_t bytes);
-    void free(void *p);
-    void trim();
+    static constexpr uint64_t KEEP_BYTES = (uint64_t)2 << 30;
+    DeviceMemory();
+    ~DeviceMemory();
+    // own: the context's own stream, on which blocks are handed out and freed
+    cudaError_t alloc(int device, cudaStream_t own, void **p, size_t bytes);
+    void trim();   // gives back what is unused
+    void close();  // before the stream goes
     static void trim_all();  // of every context of the process
 
   private:
-    struct Block {
-        void *p;
-        size_t bytes;
-    };
     std::mutex mu;
-    std::list<Block> kept;  // oldest first
-    size_t kept_bytes = 0;
-    std::unordered_map<void *, size_t> used;
+    cudaMemPool_t pool = nullptr;
+    cudaStream_t stream = nullptr;
 };
 // cudaMalloc that takes back what contexts keep before it gives up.
 cudaError_t device_malloc(void **p, size_t bytes);
@@ -247,7 +243,7 @@ struct nf_ctx {
     nf_timing last{};
     std::atomic<int> engine{-1};  // of the last sweep (NF_ENGINE_*)
     std::mutex mu;  // serialises nf_box_forces on one context
-    nf::DeviceCache memory;  // of boxes and plans
+    nf::DeviceMemory memory;  // of boxes and plans
     std::map<nf::TuneKey, nf::Tuned> tuned;  // shapes chosen so far
     // plain drop-in GPU control (nf_sic.cu)
     struct Sic;

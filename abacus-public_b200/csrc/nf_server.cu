@@ -218,7 +218,7 @@ static nf_status apply_booking(nf_server *s, Booking &bk) {
         cudaError_t e = cudaMallocFromPoolAsync(q, bytes, s->pool, st);
         if (e == cudaErrorMemoryAllocation) {
             cudaGetLastError();
-            DeviceCache::trim_all();
+            DeviceMemory::trim_all();
             e = cudaMallocFromPoolAsync(q, bytes, s->pool, st);
         }
         if (e != cudaSuccess) *q = nullptr;
@@ -384,7 +384,7 @@ extern "C" nf_status nf_server_start(nf_ctx *ctx, const nf_server_config *cfg, n
         set_error("nf_server_start: max_inflight above 256");
         return NF_EINVAL;
     }
-    DeviceCache::trim_all();  // what contexts keep but do not use
+    DeviceMemory::trim_all();  // what contexts keep but do not use
     size_t freeb = 0, total = 0;
     NF_CUDA(cudaMemGetInfo(&freeb, &total));
     s->budget = s->cfg.hbm_budget_bytes ? s->cfg.hbm_budget_bytes : (size_t)(0.9 * (double)freeb);

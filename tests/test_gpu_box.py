@@ -271,9 +271,9 @@ def test_memory_of_destroyed_boxes(capi, synth):
     assert held > 64 * mib
     db.close()
     assert 0 < base - free() <= held <= 2 << 30
-    db = ctx.box(box)  # out of what was kept
+    db = ctx.box(box)  # out of what was kept, but for the gaps between its blocks
     assert np.array_equal(db.forces(), want)
-    assert base - free() <= held + 4 * mib
+    assert base - free() <= 1.5 * held
     db.close()
     capi.lib().nf_trim()
     assert base - free() < 4 * mib
