@@ -1330,6 +1330,7 @@ extern "C" void nf_box_destroy(nf_ctx *ctx, nf_box *box) {
     for (void *p : {(void *)box->d_pos, (void *)box->d_cs, (void *)box->d_part, (void *)box->d_stage,
                     (void *)box->d_perm, box->d_sort, box->d_part2})
         pool_free(ctx, p);
+    if (ctx) cudaStreamSynchronize(ctx->own_stream);  // the memory can be given back from here on
     if (box->s_in) cudaStreamDestroy(box->s_in);
     if (box->s_out) cudaStreamDestroy(box->s_out);
     if (box->s_sweep) cudaStreamDestroy(box->s_sweep);

@@ -53,9 +53,9 @@ void DeviceMemory::close() {
 
 void DeviceMemory::trim() {
     std::lock_guard<std::mutex> lk(mu);
-    if (!pool) return;
-    cudaStreamSynchronize(stream);  // frees that are still queued
-    cudaMemPoolTrimTo(pool, 0);
+    // no wait for the stream: another thread may be capturing on it, which a
+    // wait would break (nf_box_destroy waits for its own frees)
+    if (pool) cudaMemPoolTrimTo(pool, 0);
 }
 
 void DeviceMemory::trim_all() {

@@ -300,3 +300,31 @@ def test_step_scratch_is_a_chunks(capi, synth):
         want = db.forces()
         db.close()
     np.testing.assert_allclose(out, want, rtol=0, atol=2e-6 * np.abs(want).max())
+
+
+def test_trim_beside_a_running_context(capi, synth):
+    """nf_trim from one thread while another sweeps, captures its graphs and
+    makes boxes: no call fails and no result changes."""
+    import threading
+    box = synth.uniform_box(20000, 11, seed=33)
+    stop = threading.Event()
+
+    def trim():
+        while not stop.is_set():
+            capi.lib().nf_trim()
+
+    t = threading.Thread(target=trim)
+    with capi.Context(softening=0, eps=1e-6, kernel_variant=0) as ctx:
+        db = ctx.box(box)
+        want = db.forces()
+        db.close()
+        t.start()
+        try:
+            for _ in range(100):
+                db = ctx.box(box)
+                for _ in range(3):  # launched, captured, replayed
+                    assert np.array_equal(db.forces(), want)
+                db.close()
+        finally:
+            stop.set()
+            t.join()
