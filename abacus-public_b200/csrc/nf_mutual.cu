@@ -462,7 +462,10 @@ __device__ __forceinline__ void meet(const float4 &t, const float2 &tz, Sinks<S>
     // density terms b2 - |d|^2: from r^2 where its r2_add is below the rounding
     // of b2 (mutual_bits); Plummer's eps^2 is not, and would leave its own
     // rounding in every term, so there |d|^2 is formed for itself (uniform
-    // n = 6000, b2 = 32 eps^2: density error 1.6e-7 from r^2, 1.4e-7 so)
+    // n = 6000, b2 = 32 eps^2: density error 1.6e-7 from r^2, 1.4e-7 so).  The
+    // sum rounds to b2, but as a register: read from the parameters each time,
+    // density 100^3 took 4.17 ms instead of 4.10
+    const float b2 = SOFT == SOFT_PLUMMER ? pc.b2 : pc.b2 + r2_add<SOFT>(pc);
 #pragma unroll
     for (int q = 0; q < Sinks<S>::N; q++) {
         if constexpr (S == 1) {
@@ -478,7 +481,7 @@ __device__ __forceinline__ void meet(const float4 &t, const float2 &tz, Sinks<S>
                 r.z.x = fmaf(g, dz, r.z.x);
             }
             if (DENS) {
-                const float d = SOFT == SOFT_PLUMMER ? dens_term(dx, dy, dz, pc.b2) : fmaxf(pc.b2 - r2, 0.f);
+                const float d = SOFT == SOFT_PLUMMER ? dens_term(dx, dy, dz, pc.b2) : fmaxf(b2 - r2, 0.f);
                 k.w[0].x += d;
                 if (MUTUAL) r.w.x += d;
             }
@@ -496,7 +499,7 @@ __device__ __forceinline__ void meet(const float4 &t, const float2 &tz, Sinks<S>
             }
             if (DENS) {
                 const float2 s2 = SOFT == SOFT_PLUMMER ? fma2(dz, dz, fma2(dy, dy, mul2(dx, dx))) : r2;
-                const float2 e = fma2(s2, dup2(-1.f), dup2(pc.b2));
+                const float2 e = fma2(s2, dup2(-1.f), dup2(b2));
                 const float2 d = make_float2(fmaxf(e.x, 0.f), fmaxf(e.y, 0.f));
                 k.w[q] = add2(k.w[q], d);
                 if (MUTUAL) r.w = add2(r.w, d);
