@@ -43,7 +43,70 @@ import numpy as np
 ROOT = pathlib.Path(__file__).resolve().parent
 sys.path.insert(0, str(ROOT))
 
-FLOPS_PER_PAIR = {0: 23, 1: 24, 2: 24, 3: 24}  # counted flops (FFMA=2, rsqrt=1, Newton incl.)
+# Flops of one interaction as the literature counts them (FFMA=2, rsqrt=1,
+# Newton included): what `interaction_tflops` of a line is made of.
+FLOPS_PER_PAIR = {0: 23, 1: 24, 2: 24, 3: 24}
+# Flops a kernel executes (far branch): separation 3, r^2 6, rsqrt 1, the cube
+# with its Newton step 5 (mutual engine) or 7 (one-sided), and 6 for the sum of
+# each particle the pair is added to.
+EVAL_FLOPS = {"mutual": 15, "one-sided": 17}
+SUM_FLOPS = 6
+DENSE_CELL = 192  # particles of a cell from which its column is met mutually (nf_mutual.cu)
+
+
+class OneSidedShare:
+    """Share of the interactions of slabs [lo, hi) that the mutual engine meets
+    one-sided: those in a sink cell's own column unless one of the two cells is
+    dense, and those with columns outside the range.  (A dense cell meets itself
+    in a triangle; the blocks on its diagonal are counted as mutual.)"""
+
+    def __init__(self, box, R=2):
+        self.R = R
+        n = np.asarray(box.counts).reshape((box.cpd,) * 3).astype(np.float64)
+        z = sum(np.roll(n, k, 2) for k in range(-R, R + 1))
+        self.n, self.yz = n, sum(np.roll(z, k, 1) for k in range(-R, R + 1))
+        self.own = np.zeros(box.cpd)  # per slab
+        for k in range(-R, R + 1):
+            m = np.roll(n, k, 2)
+            self.own += (n * np.where(np.maximum(n, m) < DENSE_CELL, m, 0.0)).sum((1, 2))
+
+    def __call__(self, lo, hi):
+        total, one = 0.0, self.own[lo:hi].sum()
+        for dx in range(-self.R, self.R + 1):
+            at = (np.arange(lo, hi) + dx) % len(self.own)
+            per = (self.n[lo:hi] * self.yz[at]).sum((1, 2))
+            total += per.sum()
+            one += per[(at < lo) | (at >= hi)].sum()
+        return float(one / total) if total else 1.0
+
+
+def roofline_work(share_of, lo, hi, pairs, kernel_ms, peak, soft, engine):
+    """The FP32 roofline of a sweep: flops executed for the pairs it has to
+    evaluate (no padding) over the kernel time; beside it the same time's
+    interactions at FLOPS_PER_PAIR each, more than is executed on the mutual
+    engine, which evaluates a pair once for both particles."""
+    secs = kernel_ms / 1e3
+    if engine == "mutual":
+        share = share_of(lo, hi)
+        flops = EVAL_FLOPS["mutual"] * (share + (1 - share) / 2) + SUM_FLOPS
+    else:
+        share, flops = 1.0, EVAL_FLOPS["one-sided"] + SUM_FLOPS
+    achieved = pairs * flops / secs / 1e12
+    inter = pairs * FLOPS_PER_PAIR[soft] / secs / 1e12
+    return {"achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
+            "engine": engine, "executed_flops_per_interaction": flops,
+            "one_sided_share": share, "interaction_tflops": inter,
+            "interaction_frac_of_peak": inter / peak, "flops_per_interaction": FLOPS_PER_PAIR[soft],
+            "counted": "achieved and frac: flops executed, no padding; interaction_*: every "
+                       "interaction at flops_per_interaction"}
+
+
+def kernel_name(engine):
+    return "mutual_kernel" if engine == "mutual" else "pencil_kernel"
+
+
+def engine_name(ctx):
+    return "mutual" if ctx.last_engine() == 0 else "one-sided"
 
 
 def _pkg():
@@ -330,10 +393,10 @@ def workload_config(args, w, box, pairs, world=1):
     """The `config` of the bench line: the workload alone, identical in both
     arms at N = 1."""
     l2_bytes = 126 * 2 ** 20
-    big = 136 * int(box.n) > l2_bytes  # 16 B positions + 120 B partials per particle
+    big = 41 * int(box.n) > l2_bytes  # 16 B positions + 25 B sums per particle
     return {"workload": args.workload, "desc": w["desc"], "particles_per_gpu": int(box.n),
             "cpd": int(box.cpd), "pairs_per_step_per_gpu": int(pairs),
-            "l2": ("inputs larger than L2 (positions 16 B x N + 120 B x N partials)" if big
+            "l2": ("inputs larger than L2 (positions 16 B x N + sums 25 B x N)" if big
                    else "inputs fit in L2 and are not flushed between steps (a small box)"),
             "parallelism": f"independent boxes x{world}"}
 
@@ -611,10 +674,11 @@ def serving_phase(capi, ctx, w, args, rank, seed=7):
 
 def precision_study(capi, box, w, device, stream, steps, comp_out, variant, frac=1e-3, seed=11):
     """Compensated vs plain FP32 accumulation on the same box: the plain
-    form's sweep rate (device time, positions resident, the compensated
-    sweep's kernel shape) and both results' RMS / max fractional error against
+    form's sweep rate (device time, positions resident, kernel shape `variant`
+    of the engine it takes) and both results' RMS / max fractional error against
     the FP64 oracle on a seeded subsample of `frac` of the sinks.  `comp_out`
-    is the compensated sweep's result."""
+    is the compensated sweep's result.  Plain accumulation runs on the one-sided
+    engine: the rates differ by the engine more than by the accumulation."""
     import torch
     soft, eps = w["softening"], kernel_eps(w)
     ctx = capi.Context(softening=soft, eps=eps, device=device, accumulation=capi.ACC_PLAIN,
@@ -632,6 +696,7 @@ def precision_study(capi, box, w, device, stream, steps, comp_out, variant, frac
     torch.cuda.synchronize()
     ms = e0.elapsed_time(e1) / steps
     pairs = db.pair_count()
+    engine = engine_name(ctx)
     plain_out = out.cpu().numpy()
     del out
     db.close()
@@ -645,7 +710,8 @@ def precision_study(capi, box, w, device, stream, steps, comp_out, variant, frac
     ref = oracle.fp64_sinks(box, soft, eps, sinks)
     t_ref = time.perf_counter() - t0
     res = {"sinks": k, "fraction": k / box.n, "seed": seed, "fp64_oracle_s": t_ref,
-           "plain_pairs_per_s": pairs / (ms / 1e3), "plain_ms_per_step": ms, "plain_steps": steps}
+           "plain_pairs_per_s": pairs / (ms / 1e3), "plain_ms_per_step": ms, "plain_steps": steps,
+           "plain_engine": engine}
     mag = np.linalg.norm(ref, axis=1)
     res["small_force_sinks"] = int((mag < 1e-3 * np.median(mag)).sum())  # |a64| < 1e-3 median
     for name, a in (("compensated", comp_out), ("plain", plain_out)):
@@ -746,6 +812,7 @@ def our_arm(args, w):
     total_pairs = all_sum(float(pairs), world)
     value = total_pairs / (ms_per_step / 1e3)
     launches = args.steps * t.launches
+    engine = engine_name(ctx)
 
     if args.profile:
         if rank == 0:
@@ -808,9 +875,7 @@ def our_arm(args, w):
     tune_info = {"variant": tv, "shape": lib.nf_kernel_variant_name(tv).decode(),
                  "candidates_ms": {lib.nf_kernel_variant_name(i).decode(): round(m, 3)
                                    for i, m in enumerate(tms) if m > 0}}
-    flops = FLOPS_PER_PAIR[soft]
     k_ms = float(np.mean(kernel_ms))
-    achieved = pairs * flops / (k_ms / 1e3) / 1e12
     traffic = None
     prof = ROOT / "profiles" / f"mutual_kernel_{args.workload}.json"
     if prof.exists():
@@ -837,12 +902,9 @@ def our_arm(args, w):
         "precision": precision,
         "plain_dropin": plain,
         "ref_gpu_kernel": refk,
-        "roofline": {"bound": "fp32", "achieved": achieved, "peak": peaks["peak"],
-                     "unit": "TFLOP/s", "frac": achieved / peaks["peak"], "traffic": traffic,
-                     "kernel": "mutual_kernel", "kernel_ms": k_ms,
-                     "flops_per_pair": flops,
-                     "counted": "flops of every interaction; the kernel evaluates each pair "
-                                "once for both particles",
+        "roofline": {"bound": "fp32",
+                     **roofline_work(OneSidedShare(box), 0, box.cpd, pairs, k_ms, peaks["peak"], soft, engine),
+                     "traffic": traffic, "kernel": kernel_name(engine), "kernel_ms": k_ms,
                      "peak_source": peaks["peak_source"],
                      "peak_probe_sustained": peaks["peak_probe_sustained"],
                      "peak_probe_burst": peaks["peak_probe_burst"],
@@ -932,8 +994,7 @@ def big_arm(args, w):
     k_ms = float(np.mean(kms))
     clocks = clk.summary()
     peak, derived = peak_from(peak_s, clocks, torch.cuda.get_device_properties(0).multi_processor_count)
-    flops = FLOPS_PER_PAIR[w["softening"]]
-    achieved = pairs * flops / (k_ms / 1e3) / 1e12
+    engine = engine_name(ctx)
     res = out.cpu().numpy()
     sys.path.insert(0, str(ROOT / "oracle"))
     import oracle
@@ -949,9 +1010,9 @@ def big_arm(args, w):
                    "slabs": [lo, hi], "particles_in_slabs": p1 - p0, "pairs_per_step": pairs,
                    "padded_pairs_per_step": int(t.padded_pairs),
                    "max_particles_per_cell": int(counts.max()), "kernel_shape": 0},
-        "roofline": {"bound": "fp32", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
-                     "frac": achieved / peak, "traffic": None, "kernel": "mutual_kernel",
-                     "kernel_ms": k_ms, "flops_per_pair": flops,
+        "roofline": {"bound": "fp32",
+                     **roofline_work(OneSidedShare(hbox), lo, hi, pairs, k_ms, peak, w["softening"], engine),
+                     "traffic": None, "kernel": kernel_name(engine), "kernel_ms": k_ms,
                      "peak_probe_sustained": peak_s, "peak_clock_derived": derived,
                      "staging_hbm": staging_hbm(p1 - p0, box_nc(w), k_ms, None)},
         "accuracy_vs_fp64": {"rms_frac": rms, "max_frac": mx, "sinks": 2000},
@@ -967,9 +1028,10 @@ def big_arm(args, w):
 
 def big_full_sweep(args, w, capi, ctx, db, hbox, eps, peak_s, stream):
     """The whole 1024^3 box, compensated and then plain FP32 accumulation:
-    one persistent launch per range of --slabs slabs (the partials of the
-    whole box would not fit beside the positions), device time summed over
-    the ranges; FP64 oracle on 2000 seeded sinks for each mode."""
+    one persistent launch per range of --slabs slabs (the sums of the whole
+    box would not fit beside the positions), device time summed over the
+    ranges; FP64 oracle on 2000 seeded sinks for each mode.  Plain
+    accumulation runs on the one-sided engine (`engine` of each mode)."""
     import torch
     sys.path.insert(0, str(ROOT / "oracle"))
     import oracle
@@ -977,7 +1039,7 @@ def big_full_sweep(args, w, capi, ctx, db, hbox, eps, peak_s, stream):
     ranges = [(lo, min(cpd, lo + args.slabs)) for lo in range(0, cpd, args.slabs)]
     sinks = np.sort(np.random.default_rng(5).choice(hbox.n, 2000, replace=False))
     a64 = oracle.fp64_sinks(hbox, soft, eps, sinks)
-    flops = FLOPS_PER_PAIR[soft]
+    share_of = OneSidedShare(hbox)
     modes = {}
     for name, acc in (("compensated", capi.ACC_COMPENSATED), ("plain", capi.ACC_PLAIN)):
         if db is None:
@@ -985,7 +1047,7 @@ def big_full_sweep(args, w, capi, ctx, db, hbox, eps, peak_s, stream):
             ctx.set_stream(stream.cuda_stream)
             db = ctx.box(hbox)
         got = np.zeros((sinks.size, 3), np.float32)
-        tot_ms = k_ms = 0.0
+        tot_ms = k_ms = executed = 0.0
         pairs = 0
         with ClockSampler(0) as clk:
             for lo, hi in ranges:
@@ -996,17 +1058,20 @@ def big_full_sweep(args, w, capi, ctx, db, hbox, eps, peak_s, stream):
                 tot_ms += t.total_ms
                 k_ms += t.kernel_ms
                 pairs += int(t.pairs)
+                executed += roofline_work(share_of, lo, hi, int(t.pairs), t.kernel_ms, 1.0, soft,
+                                          engine_name(ctx))["achieved"] * t.kernel_ms
                 sel = (sinks >= p0) & (sinks < p1)
                 if sel.any():
                     got[sel] = out[torch.from_numpy(sinks[sel] - p0).cuda(), :3].cpu().numpy()
                 del out
         rms, mx, _ = oracle.frac_errors(got, a64)
-        achieved = pairs * flops / (k_ms / 1e3) / 1e12
         clocks = clk.summary()
         peak, derived = peak_from(peak_s, clocks,
                                   torch.cuda.get_device_properties(0).multi_processor_count)
         modes[name] = {"pairs": pairs, "device_ms": tot_ms, "kernel_ms": k_ms,
-                       "pairs_per_s": pairs / (tot_ms / 1e3), "frac_of_fp32_peak": achieved / peak,
+                       "pairs_per_s": pairs / (tot_ms / 1e3), "engine": engine_name(ctx),
+                       "executed_tflops": executed / k_ms, "frac_of_fp32_peak": executed / k_ms / peak,
+                       "interaction_tflops": pairs * FLOPS_PER_PAIR[soft] / (k_ms / 1e3) / 1e12,
                        "peak": peak, "peak_clock_derived": derived, "peak_probe_sustained": peak_s,
                        "rms_frac": rms, "max_frac": mx, "clocks": clocks}
         db.close()
@@ -1023,10 +1088,12 @@ def big_full_sweep(args, w, capi, ctx, db, hbox, eps, peak_s, stream):
                    "full_sweep": True, "slabs_per_launch": args.slabs, "launches": len(ranges),
                    "kernel_shape": 0,
                    "max_particles_per_cell": int(np.diff(hbox.cell_start).max())},
-        "roofline": {"bound": "fp32", "achieved": c["pairs"] * flops / (c["kernel_ms"] / 1e3) / 1e12,
+        "roofline": {"bound": "fp32", "achieved": c["executed_tflops"],
                      "peak": c["peak"], "unit": "TFLOP/s", "frac": c["frac_of_fp32_peak"],
-                     "traffic": None, "kernel": "mutual_kernel", "kernel_ms": c["kernel_ms"],
-                     "flops_per_pair": flops,
+                     "interaction_tflops": c["interaction_tflops"],
+                     "flops_per_interaction": FLOPS_PER_PAIR[soft], "engine": c["engine"],
+                     "traffic": None, "kernel": kernel_name(c["engine"]),
+                     "kernel_ms": c["kernel_ms"],
                      "staging_hbm": staging_hbm(hbox.n, box_nc(w), c["kernel_ms"], None)},
         "modes": modes,
         "accuracy_vs_fp64": {"rms_frac": c["rms_frac"], "max_frac": c["max_frac"], "sinks": 2000},
@@ -1110,11 +1177,10 @@ def shard_arm(args, w):
     torch.cuda.synchronize()
     e2e_ms = barrier_max(e0.elapsed_time(e1) / args.steps, world)
     nbytes = all_sum(float(sum(v.numel() * 4 for v in host.values())), world)
-    flops = FLOPS_PER_PAIR[w["softening"]]
+    engine = engine_name(ctx)
     clocks = clk.summary()
     peaks = fp32_peaks(ctx, clocks, torch.cuda.get_device_properties(local).multi_processor_count)
     peak_s = peaks["peak"]
-    achieved = pairs * flops / (k_ms / 1e3) / 1e12
     result = {
         "metric": "pair_interactions_per_s", "value": total_pairs / (ms / 1e3), "unit": "pairs/s",
         "n_gpus": world, "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms,
@@ -1123,8 +1189,9 @@ def shard_arm(args, w):
         "config": {"workload": args.workload, "desc": w["desc"], "pairs_per_step": total_pairs,
                    "parallelism": f"slab-sharded x{world} (2-slab halo over NCCL)",
                    "slabs": parts, "l2": "inputs larger than L2"},
-        "roofline": {"bound": "fp32", "achieved": achieved, "peak": peak_s, "unit": "TFLOP/s",
-                     "frac": achieved / peak_s, "traffic": None, "kernel": "mutual_kernel",
+        "roofline": {"bound": "fp32",
+                     **roofline_work(OneSidedShare(wbox), lo, hi, pairs, k_ms, peak_s, w["softening"], engine),
+                     "traffic": None, "kernel": kernel_name(engine),
                      "kernel_ms": k_ms, "note": "slowest rank's kernel time, its own pairs",
                      "peak_source": peaks["peak_source"]},
         "e2e": {"value": total_pairs / (e2e_ms / 1e3), "unit": "pairs/s", "ms_per_step": e2e_ms,

@@ -95,3 +95,35 @@ def test_bench_lines_are_strict_json():
     bench = _bench()
     line = bench.json_line({"a": float("nan"), "b": [1.0, float("inf")], "c": {"d": -float("inf")}})
     assert json.loads(line) == {"a": None, "b": [1.0, None], "c": {"d": None}}
+
+
+def test_roofline_counts_executed_flops(synth):
+    """The one-sided share against a walk over all cell pairs, and the line's
+    two counts: a mutual pair is 15 flops for two interactions and 6 for each."""
+    bench = _bench()
+    box = synth.clustered_box(30000, 7, seed=3, n_clumps=6)  # some cells above DENSE_CELL
+    n = box.counts.reshape(7, 7, 7)
+    assert n.max() > bench.DENSE_CELL > n.min()
+    share = bench.OneSidedShare(box)
+    for lo, hi in ((0, 7), (2, 5), (6, 7), (0, 1)):
+        total = one = 0
+        for x in range(lo, hi):
+            for y in range(7):
+                for z in range(7):
+                    for dx in range(-2, 3):
+                        for dy in range(-2, 3):
+                            for dz in range(-2, 3):
+                                m = n[(x + dx) % 7, (y + dy) % 7, (z + dz) % 7]
+                                p = int(n[x, y, z]) * int(m)
+                                total += p
+                                if dx == dy == 0:
+                                    one += p * (max(n[x, y, z], m) < bench.DENSE_CELL)
+                                else:
+                                    one += p * (not lo <= (x + dx) % 7 < hi)
+        assert abs(share(lo, hi) - one / total) < 1e-12
+    r = bench.roofline_work(lambda lo, hi: 0.25, 0, 7, 10 ** 12, 1000.0, 80.0, 0, "mutual")
+    assert abs(r["achieved"] - (15 * 0.25 + 15 * 0.75 / 2 + 6)) < 1e-9
+    assert abs(r["frac"] - r["achieved"] / 80.0) < 1e-12
+    assert r["interaction_tflops"] == 23.0 and r["interaction_tflops"] > r["achieved"]
+    r = bench.roofline_work(None, 0, 7, 10 ** 12, 1000.0, 80.0, 0, "one-sided")
+    assert r["achieved"] == 23.0
