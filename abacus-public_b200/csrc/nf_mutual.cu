@@ -1,16 +1,17 @@
 // nf_mutual.cu -- the mutual pencil engine: each pair of particles of a slab
 // range is evaluated once and its force added to both.
 //
-// What bounds the one-sided sweep (nf_box.cu) is the FP32 pipe: 13 paired
-// instructions per two interactions.  Of these only the three accumulations
-// belong to one particle; separation, r^2 and g are the same for the pair
-// seen from the other side.  Evaluating a pair once and accumulating it twice
-// costs 16 instructions for four interactions: 8 per two instead of 13.
+// What bounds the one-sided sweep (nf_box.cu) is the FP32 pipe: 14 paired
+// instructions per two interactions (13 with the Newton step of this engine).
+// Of these only the three accumulations belong to one particle; separation,
+// r^2 and g are the same for the pair seen from the other side.  Evaluating a
+// pair once and accumulating it twice costs 16 instructions for four
+// interactions: 8 per two.
 // Sweep times, one-sided -> mutual (with the list ordered as below): uniform
 // 64^3 0.922 -> 0.768 ms, clustered 128^3 8.96 -> 6.87, clustered 256^3 119.1
-// -> 88.0 (2.8e12 pairs/s), density 100^3 6.46 -> 4.17; 3.2e12 pairs/s where
-// pencils hold thousands of sinks.
-// On clustered 256^3 the FMA pipe is busy 69 % (one instruction in three
+// -> 88.0 (2.8e12 pairs/s; 89.9 on another GPU), density 100^3 6.46 -> 4.10;
+// 3.2e12 pairs/s where pencils hold thousands of sinks.
+// On clustered 256^3 the FMA pipe is busy 67 % (one instruction in three
 // reads three distinct register pairs and issues at 2/3 rate).  Of a warp's
 // time on uniform 160^3, 79 % is the mutual loop, 7 % the centre column
 // one-sided, 8 % staging, 6 % the rest; padding of tiles and groups is 11 %.
@@ -37,8 +38,11 @@
 //
 // Where sums go.  Reactions arrive at a particle from many warps in no fixed
 // order, so all sums meet in 64-bit fixed point, added with integer atomics:
-// associative, hence bit-identical in any order and for any split of the
-// work.  The unit is 2^-fbits of the kernel's force unit, with fbits set from
+// associative, so the same work list gives the same bits in whatever order it
+// runs.  Another list -- another kernel shape, slab range or GPU size, other
+// SICs -- cuts tiles and streams elsewhere: the groups of FP32 partials below
+// and the rounding of each piece to the unit differ, and results agree to
+// rounding.  The unit is 2^-fbits of the kernel's force unit, with fbits set from
 // a strict bound on a sink's sum (largest possible pair force x most sources
 // a sink can meet) so that it cannot overflow; see mutual_bits() for the
 // condition under which its resolution is below FP32's own noise.  FP32
@@ -111,8 +115,10 @@ __host__ __device__ __forceinline__ bool segment(const Stream &s, int R, int i, 
 }
 
 // Cells, and the slabs [lo, hi) that hold the sinks.  onesided: no pair is met
-// mutually (a drop-in SIC: a sink's sum then has the same order whatever rows
-// and z cells the SIC holds).
+// mutually (a drop-in SIC: a sink's sum then runs over its sources in the same
+// order whatever rows and z cells the SIC holds, and differs between SICs only
+// by where pieces are cut and by the fixed-point unit: nodes of a z-split agree
+// with the one domain to 2e-6 of |a| instead of 7.5e-6).
 struct Geometry {
     const int64_t *__restrict__ cs;
     int cpd, R, lo, hi;

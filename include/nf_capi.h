@@ -390,9 +390,10 @@ nf_status nf_last_timing(nf_ctx *ctx, nf_timing *t);
  * softening length in box units) and M the most sources a pencil of the slab
  * range meets, it is taken where F (2R+1) M is above 2^36 to 2^37 cpd^2 --
  * a softening below 4e-4 (Plummer) to 9e-4 (single spline) cells at R 2 and
- * M = 10^4, in proportion to the root of M -- and where the density radius is tiny (b2 < 3.4e-9 with the cubic
- * Plummer softening, < 3.4e-18 with a spline).  nf_forces_noalloc follows the
- * same rule with M (2R+1) the number of particles of the box.
+ * M = 10^4, in proportion to the root of M -- and where the density radius is
+ * tiny (b2 (2R+1) M < 1.8e-12; b2 < 3.4e-9 with the cubic Plummer softening).
+ * nf_forces_noalloc follows the same rule with (2R+1) M the number of
+ * particles of the box.
  * NF_ENOTREADY before the first sweep. */
 #define NF_ENGINE_MUTUAL 0
 #define NF_ENGINE_ONE_SIDED 1

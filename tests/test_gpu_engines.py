@@ -221,3 +221,30 @@ def test_serving_on_the_one_sided_engine(capi, synth):
             db.close()
         for a, b in zip(alone, outs):
             assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
+
+
+@pytest.mark.parametrize("soft,b2,engine", [(3, 5e-9, 0), (3, 2e-9, 1), (2, 1e-12, 0), (1, 1e-13, 1),
+                                            (0, 1e-12, 0), (0, 1e-13, 1)])
+def test_tiny_density_radii(capi, oracle, synth, soft, b2, engine):
+    """The mutual engine takes the density from r^2 only where what r^2 carries
+    on top (1e-16 with the cubic Plummer softening) is below the rounding of b2,
+    and only while the scale of its sums is a float.  Pairs at half the
+    radius."""
+    cpd = 11
+    rng = np.random.default_rng(11)
+    n = np.zeros((cpd,) * 3, int)
+    n[::4, ::4, ::4] = 2
+    cs = np.zeros(cpd ** 3 + 1, np.int64)
+    cs[1:] = np.cumsum(n.ravel())
+    m = int(cs[-1])
+    d = rng.normal(size=(3, m // 2))
+    d *= 0.5 * np.sqrt(b2) / np.linalg.norm(d, axis=0)
+    p = np.stack([d / 2, -d / 2], 2).reshape(3, m).astype(np.float32)  # about the cell centre: exact enough
+    box = synth.Box(cpd=cpd, x=p[0].copy(), y=p[1].copy(), z=p[2].copy(), cell_start=cs)
+    with capi.Context(softening=soft, eps=synth.kernel_eps(soft, 0.02 / cpd), b2=b2) as ctx:
+        db = ctx.box(box)
+        a = db.forces()
+        assert ctx.last_engine() == engine
+        db.close()
+    want = oracle.fp64_density(box, b2, np.arange(m))
+    np.testing.assert_allclose(a[:, 3], want, rtol=1e-6)
