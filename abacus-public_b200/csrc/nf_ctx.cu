@@ -44,6 +44,7 @@ DeviceMemory::~DeviceMemory() {
 }
 
 void DeviceMemory::close() {
+    trim();
     std::lock_guard<std::mutex> lk(mu);
     if (!pool) return;
     cudaStreamSynchronize(stream);
@@ -53,6 +54,9 @@ void DeviceMemory::close() {
 
 void DeviceMemory::trim() {
     std::lock_guard<std::mutex> lk(mu);
+    for (const Block &b : kept) cudaFree(b.p);
+    kept.clear();
+    kept_bytes = 0;
     // no wait for the stream: another thread may be capturing on it, which a
     // wait would break (nf_box_destroy waits for its own frees)
     if (pool) cudaMemPoolTrimTo(pool, 0);
@@ -63,7 +67,58 @@ void DeviceMemory::trim_all() {
     for (DeviceMemory *m : g_memories) m->trim();
 }
 
+cudaError_t DeviceMemory::alloc_big(void **p, size_t bytes) {
+    // sixteenths of a power of two, so that a block fits the next box's list or
+    // sums too; blocks that are not kept anyway as they are
+    size_t step = 512;
+    while (step * 32 <= bytes) step *= 2;
+    if (bytes <= KEEP_BYTES) bytes = (bytes + step - 1) / step * step;
+    {
+        std::lock_guard<std::mutex> lk(mu);
+        auto best = kept.end();  // the smallest that holds it with an eighth to spare at most
+        for (auto it = kept.begin(); it != kept.end(); ++it)
+            if (it->bytes >= bytes && it->bytes - bytes <= bytes / 8 &&
+                (best == kept.end() || it->bytes < best->bytes))
+                best = it;
+        if (best != kept.end()) {
+            *p = best->p;
+            big[best->p] = best->bytes;
+            kept_bytes -= best->bytes;
+            kept.erase(best);
+            return cudaSuccess;
+        }
+    }
+    const cudaError_t e = device_malloc(p, bytes);
+    if (e == cudaSuccess) {
+        std::lock_guard<std::mutex> lk(mu);
+        big[*p] = bytes;
+    }
+    return e;
+}
+
+void DeviceMemory::free(cudaStream_t own, void *p) {
+    std::vector<void *> out;
+    {
+        std::lock_guard<std::mutex> lk(mu);
+        auto it = big.find(p);
+        if (it == big.end()) {
+            cudaFreeAsync(p, own);
+            return;
+        }
+        kept.push_back(Block{p, it->second});
+        kept_bytes += it->second;
+        big.erase(it);
+        while (kept_bytes > KEEP_BYTES) {
+            out.push_back(kept.front().p);
+            kept_bytes -= kept.front().bytes;
+            kept.pop_front();
+        }
+    }
+    for (void *q : out) cudaFree(q);
+}
+
 cudaError_t DeviceMemory::alloc(int device, cudaStream_t own, void **p, size_t bytes) {
+    if (bytes >= BIG) return alloc_big(p, bytes);
     *p = nullptr;
     cudaError_t e = cudaSuccess;
     cudaMemPool_t from;
@@ -75,7 +130,7 @@ cudaError_t DeviceMemory::alloc(int device, cudaStream_t own, void **p, size_t b
             pp.location.type = cudaMemLocationTypeDevice;
             pp.location.id = device;
             e = cudaMemPoolCreate(&pool, &pp);
-            uint64_t keep = KEEP_BYTES;
+            uint64_t keep = KEEP_POOL_BYTES;
             if (e == cudaSuccess) e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
             if (e != cudaSuccess) {
                 if (pool) cudaMemPoolDestroy(pool);
@@ -118,13 +173,13 @@ cudaError_t nf::device_malloc(void **p, size_t bytes) {
 // library's own stream, whatever stream the caller has set.
 cudaError_t nf::pool_alloc(nf_ctx *ctx, void **p, size_t bytes) {
     cudaError_t e = ctx->memory.alloc(ctx->device, ctx->own_stream, p, bytes);
-    if (e == cudaSuccess && ctx->stream != ctx->own_stream) e = cudaStreamSynchronize(ctx->own_stream);
+    if (e == cudaSuccess && bytes < DeviceMemory::BIG && ctx->stream != ctx->own_stream) e = cudaStreamSynchronize(ctx->own_stream);
     return e;
 }
 
 void nf::pool_free(nf_ctx *ctx, void *p) {
     if (!p) return;
-    if (ctx) cudaFreeAsync(p, ctx->own_stream);
+    if (ctx) ctx->memory.free(ctx->own_stream, p);
     else cudaFree(p);
 }
 

@@ -7,11 +7,13 @@
 #include <condition_variable>
 #include <cstdint>
 #include <deque>
+#include <list>
 #include <map>
 #include <memory>
 #include <mutex>
 #include <string>
 #include <thread>
+#include <unordered_map>
 #include <vector>
 
 #include "nf_capi.h"
@@ -148,32 +150,46 @@ bool mutual_sic_list(const nf_config &cfg, int cpd, const std::vector<SicPencil>
                      int warps, Plan &pl, std::vector<MutualItem> &items);
 nf_status mutual_plan(nf_ctx *ctx, const nf_box *box, int lo, int hi, int variant, Plan &pl);
 nf_status mutual_launch(nf_ctx *ctx, const MutualLaunch &L, cudaStream_t st);
-// Device memory of a context's boxes and plans: a memory pool of its own, made
-// when the first block is asked for (a context without boxes, as a driver's,
-// makes none).  What is freed stays for the next box, up to KEEP_BYTES: a
-// simulation that makes a box each step asks for the same blocks again (1.2 GB
-// for 256^3 particles: 55.5 ms a step, 60 ms with half of it kept).  It goes
-// back to the device at nf_shutdown, when a server starts, by nf_trim, and when
-// any allocation of this library runs out.  Against blocks from cudaMalloc kept
-// in a list: context + box + shutdown 3.2 ms beside 5.0 (128^3), and the first
-// pass of a server, whose 90 slab plans allocate while requests run, 95 ms
-// beside 107-167.  A block handed to free() is idle: no work that uses it is in
-// flight.
+// Device memory of a context's boxes and plans.  What is freed stays for the
+// next box, up to KEEP_BYTES + KEEP_POOL_BYTES: a simulation that makes a box
+// each step asks for the same blocks again (1.2 GB for 256^3 particles: 55.5 ms
+// a step, 60 ms with half of it kept).  It goes back to the device at
+// nf_shutdown, when a server starts, by nf_trim, and when any allocation of
+// this library runs out.
+// Blocks below BIG come from a memory pool, made when the first is asked for (a
+// context without boxes, as a driver's, makes none); others from cudaMalloc,
+// kept in a list.  New memory costs a pool 6 ms a GB (a block of 256 MB 1.5
+// ms) and cudaMalloc 0.35 ms whatever the size, so boxes of 256^3 take 8.5 ms to
+// make from the pool and 4.5 so; and cudaMalloc waits for the device, which
+// the work lists of a server's 90 slabs, made while requests run, cannot afford
+// (first pass of serving 95 ms, with cudaMalloc for all 107-167).
+// A block handed to free() is idle: no work that uses it is in flight.
 class DeviceMemory {
   public:
-    static constexpr uint64_t KEEP_BYTES = (uint64_t)2 << 30;
+    static constexpr size_t BIG = (size_t)32 << 20;
+    static constexpr size_t KEEP_BYTES = (size_t)1792 << 20, KEEP_POOL_BYTES = (size_t)256 << 20;
     DeviceMemory();
     ~DeviceMemory();
-    // own: the context's own stream, on which blocks are handed out and freed
+    // own: the context's own stream, on which the pool's blocks are handed out
+    // and freed
     cudaError_t alloc(int device, cudaStream_t own, void **p, size_t bytes);
+    void free(cudaStream_t own, void *p);
     void trim();   // gives back what is unused
     void close();  // before the stream goes
     static void trim_all();  // of every context of the process
 
   private:
+    cudaError_t alloc_big(void **p, size_t bytes);
+    struct Block {
+        void *p;
+        size_t bytes;
+    };
     std::mutex mu;
     cudaMemPool_t pool = nullptr;
     cudaStream_t stream = nullptr;
+    std::list<Block> kept;  // oldest first
+    size_t kept_bytes = 0;
+    std::unordered_map<void *, size_t> big;  // handed out
 };
 // cudaMalloc that takes back what contexts keep before it gives up.
 cudaError_t device_malloc(void **p, size_t bytes);
