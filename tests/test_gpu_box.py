@@ -328,3 +328,52 @@ def test_trim_beside_a_running_context(capi, synth):
         finally:
             stop.set()
             t.join()
+
+
+@pytest.mark.parametrize("n,cpd,rounds", [(20000, 11, 60), (2_500_000, 51, 8)])
+def test_contexts_side_by_side(capi, synth, n, cpd, rounds):
+    """Two threads, each with a context of its own, make boxes, sweep them
+    (launched, captured as a graph, replayed), change their softening, step them
+    and drop them, while a third trims: no call fails and no result changes.
+    (The larger box's blocks come from cudaMalloc, the smaller one's from the
+    pool.)"""
+    import threading
+    box = synth.uniform_box(n, cpd, seed=34)
+    errors, stop = [], threading.Event()
+    with capi.Context(softening=0, eps=1e-6, kernel_variant=0) as ctx:
+        db = ctx.box(box)
+        want = db.forces()
+        stepped = np.empty_like(want)
+        db.step(box.x, box.y, box.z, stepped)
+        db.close()
+
+    def work():
+        try:
+            with capi.Context(softening=0, eps=1e-6, kernel_variant=0) as ctx:
+                out = np.empty_like(want)
+                for _ in range(rounds):
+                    db = ctx.box(box)
+                    for _ in range(3):
+                        assert np.array_equal(db.forces(), want)
+                    db.step(box.x, box.y, box.z, out)
+                    assert np.array_equal(out, stepped)
+                    db.set_eps(2e-6)
+                    db.set_eps(0.0)
+                    assert np.array_equal(db.forces(), want)
+                    db.close()
+        except Exception as e:  # noqa: BLE001 -- reported by the main thread
+            errors.append(e)
+
+    def trim():
+        while not stop.is_set():
+            capi.lib().nf_trim()
+
+    threads = [threading.Thread(target=work) for _ in range(2)]
+    trimmer = threading.Thread(target=trim)
+    for t in threads + [trimmer]:
+        t.start()
+    for t in threads:
+        t.join()
+    stop.set()
+    trimmer.join()
+    assert not errors, errors
