@@ -38,6 +38,7 @@
 // by whole CTAs first); the CTA sums its warps' partials in warp order.  The
 // rest are taken one warp at a time from an atomic counter.
 #include <algorithm>
+#include <chrono>
 #include <cmath>
 #include <cstring>
 #include <numeric>
@@ -1112,6 +1113,20 @@ static bool on_device(const nf_ctx *ctx, const void *p, size_t bytes) {
 
 using namespace nf;
 
+// Waits for what a call may have left on the context's and the box's streams
+// (when it failed; a call that succeeds has waited).  With ctx->mu held, so that
+// none of them is being captured, and not for the whole device:
+// that is an error while another thread captures a graph, and breaks its
+// capture.
+static void wait_streams(nf_ctx *ctx, nf_box *box) {
+    if (ctx) {
+        cudaStreamSynchronize(ctx->stream);
+        if (ctx->stream != ctx->own_stream) cudaStreamSynchronize(ctx->own_stream);
+    }
+    for (cudaStream_t s : {box->s_in, box->s_out, box->s_sweep})
+        if (s) cudaStreamSynchronize(s);
+}
+
 size_t nf_box::device_bytes() const {
     size_t b = (size_t)np * sizeof(float4) + cell_start.size() * sizeof(int64_t) + part_bytes +
                part2_bytes +
@@ -1242,7 +1257,7 @@ static nf_status upload_scratch(nf_ctx *ctx, nf_box *box, OrderScratch &o) {
     const size_t kb = ((size_t)n * 8 + 255) & ~(size_t)255, vb = ((size_t)n * 4 + 255) & ~(size_t)255;
     const size_t need = 2 * kb + vb + o.temp_bytes;
     if (box->sort_bytes < need) {
-        NF_CUDA(cudaDeviceSynchronize());
+        wait_streams(ctx, box);
         pool_free(ctx, box->d_sort);
         box->d_sort = nullptr;
         box->sort_bytes = 0;
@@ -1320,12 +1335,18 @@ static nf_status nf::box_upload(nf_ctx *ctx, nf_box *box, const float *x, const 
     return NF_OK;
 }
 
+// Waits for the box's admitted requests.
+static void wait_requests(nf_box *box) {
+    while (box->serving.load() > 0) std::this_thread::sleep_for(std::chrono::microseconds(20));
+}
+
 extern "C" void nf_box_destroy(nf_ctx *ctx, nf_box *box) {
     if (!box) return;
     if (ctx) cudaSetDevice(ctx->device);
-    cudaDeviceSynchronize();  // whatever still reads the box, on any stream
+    wait_requests(box);
     std::unique_lock<std::mutex> lk;
     if (ctx) lk = std::unique_lock<std::mutex>(ctx->mu);
+    wait_streams(ctx, box);
     for (auto &kv : box->plans) free_plan(ctx, *kv.second);
     for (void *p : {(void *)box->d_pos, (void *)box->d_cs, (void *)box->d_part, (void *)box->d_stage,
                     (void *)box->d_perm, box->d_sort, box->d_part2})
@@ -1348,7 +1369,8 @@ extern "C" nf_status nf_box_set_eps(nf_ctx *ctx, nf_box *box, float eps) {
     if (eps == box->eps) return NF_OK;
     // cached plans hold graphs with the old constants: wait for every launch
     // that may use them, then drop them (the kernel-shape choice is kept)
-    NF_CUDA(cudaDeviceSynchronize());
+    wait_requests(box);
+    wait_streams(ctx, box);
     for (auto &kv : box->plans) free_plan(ctx, *kv.second);
     box->plans.clear();
     box->eps = eps;
@@ -1394,7 +1416,7 @@ static nf_status ensure_scratch(nf_ctx *ctx, nf_box *box, const Plan &pl) {
         pl.mutual ? mutual_scratch_bytes(pl.n_range, nc)
                   : (size_t)(2 * ctx->cfg.near_field_radius + 1) * nc * (size_t)pl.n_range * sizeof(Partial);
     if (need <= box->part_bytes) return NF_OK;
-    NF_CUDA(cudaDeviceSynchronize());  // a call that failed may have left work behind
+    wait_streams(ctx, box);  // a call that failed may have left work behind
     pool_free(ctx, box->d_part);
     box->d_part = nullptr;
     box->part_bytes = 0;
@@ -1706,7 +1728,7 @@ extern "C" nf_status nf_box_step(nf_ctx *ctx, nf_box *box, const float *x, const
         need2 = std::max(need2, mutual_scratch_bytes(pl->n_range, ctx->cfg.b2 > 0.f ? 4 : 3));
     }
     if (two && box->part2_bytes < need2) {
-        NF_CUDA(cudaDeviceSynchronize());
+        wait_streams(ctx, box);
         pool_free(ctx, box->d_part2);
         box->d_part2 = nullptr;
         box->part2_bytes = 0;

@@ -245,6 +245,7 @@ struct nf_box {
     std::map<std::pair<int, int>, std::unique_ptr<nf::Plan>> plans;
     nf::Tuned tuned[2];  // kernel shape by engine (NF_ENGINE_*), as chosen by the autotuner
     int engine = 0;      // of the plan built last
+    std::atomic<int> serving{0};  // admitted requests whose work may still read the box
     float eps = 0.f;        // the box's own softening parameter (0: the context's)
     size_t device_bytes() const;
 };

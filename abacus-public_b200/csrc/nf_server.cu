@@ -114,6 +114,7 @@ static void CUDART_CB on_done(void *arg) {
         r->slot_index = r->slot->index;
         r->slot->req = nullptr;
         r->slot = nullptr;
+        r->box->serving--;
         s->completed++;
         s->pairs += r->pairs;
         s->lat_ms.push_back(std::chrono::duration<double, std::milli>(r->t_done - r->t_submit).count());
@@ -290,6 +291,7 @@ static void fail_admitted(nf_server *s, Req *r, Slot *sl, nf_status st) {
         sl->part_cap = sl->out_cap = 0;
         sl->req = nullptr;
     }
+    r->box->serving--;
     r->slot = nullptr;
     r->state = -1;
     r->status = st;
@@ -354,12 +356,14 @@ static void dispatcher_main(nf_server *s) {
         r->pairs = pl->pairs;
         r->t_admit = sclock::now();
         pick->req = r;
+        r->box->serving++;
         s->admitted++;
         if (s->running++ == 0) s->busy_since = r->t_admit;
         s->max_running = std::max(s->max_running, s->running);
         lk.unlock();
         st = apply_booking(s, bk);
         if (st == NF_OK) st = launch_request(s, r, *pick, pl);
+        if (st != NF_OK) cudaStreamSynchronize(pick->stream);  // what was launched before it failed
         lk.lock();
         if (st != NF_OK) fail_admitted(s, r, pick, st);
     }

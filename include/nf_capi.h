@@ -348,8 +348,8 @@ nf_status nf_box_update_aos(nf_ctx *ctx, nf_box *box, const float *xyz);
 /* Give the box its own softening parameter (same convention as
  * nf_config.eps for the context's softening; 0 = the context's), so that
  * boxes of different particle spacing share one context and one server.
- * Waits for the device and drops the box's cached plans: call it while no
- * sweep or request of this box is in flight. */
+ * Waits for the box's work and drops its cached plans: call it while no sweep
+ * or request of this box is in flight. */
 nf_status nf_box_set_eps(nf_ctx *ctx, nf_box *box, float eps);
 /* Device bytes held by the box (positions + plans + partial buffers). */
 size_t nf_box_device_bytes(const nf_box *box);

@@ -377,3 +377,50 @@ def test_contexts_side_by_side(capi, synth, n, cpd, rounds):
     stop.set()
     trimmer.join()
     assert not errors, errors
+
+
+def test_calls_beside_a_graph_capture(capi, synth):
+    """While one thread captures a CUDA graph (thread-local mode), another makes
+    a box, sweeps, steps, changes the softening, serves and destroys it: neither
+    fails.  (A wait for the whole device in any of these calls is an error during
+    a capture, and breaks it.)"""
+    import threading
+
+    import torch
+    box = synth.uniform_box(20000, 11, seed=35)
+    errors = []
+
+    def work(ctx):
+        try:
+            db = ctx.box(box)
+            want = db.forces()
+            for _ in range(3):
+                assert np.array_equal(db.forces(), want)
+            out = np.empty_like(want)
+            db.step(box.x, box.y, box.z, out)
+            db.forces(2, 4)
+            db.set_eps(2e-6)
+            db.forces()
+            with capi.Server(ctx) as srv:
+                p0, p1 = db.slab_particles(3, 4)
+                part = np.empty((p1 - p0, 4), np.float32)
+                srv.wait(srv.submit(db, 3, part))
+            capi.lib().nf_trim()
+            db.close()
+        except Exception as e:  # noqa: BLE001 -- reported by the main thread
+            errors.append(e)
+
+    x = torch.zeros(1000, device="cuda")
+    with capi.Context(softening=0, eps=1e-6, kernel_variant=0) as ctx:
+        work(ctx)  # everything loaded
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, capture_error_mode="thread_local"):
+            x.add_(1)
+            t = threading.Thread(target=work, args=(ctx,))
+            t.start()
+            t.join()
+            x.add_(1)
+        g.replay()
+        torch.cuda.synchronize()
+        assert x[0].item() == 2.0
+    assert not errors, errors
