@@ -26,16 +26,12 @@ nf_status cuda_fail(cudaError_t e, const char *what) {
 
 using namespace nf;
 
-// Every context's, for trim_all().
+// Every context's that holds blocks, for trim_all().
 static std::mutex g_memories_mu;
 static std::vector<DeviceMemory *> g_memories;
 
-DeviceMemory::DeviceMemory() {
-    std::lock_guard<std::mutex> lk(g_memories_mu);
-    g_memories.push_back(this);
-}
-
 DeviceMemory::~DeviceMemory() {
+    if (!known) return;
     {
         std::lock_guard<std::mutex> lk(g_memories_mu);
         g_memories.erase(std::find(g_memories.begin(), g_memories.end(), this));
@@ -118,6 +114,11 @@ void DeviceMemory::free(cudaStream_t own, void *p) {
 }
 
 cudaError_t DeviceMemory::alloc(int device, cudaStream_t own, void **p, size_t bytes) {
+    if (!known) {  // (allocations of one context are serialised by its mutex)
+        std::lock_guard<std::mutex> lk(g_memories_mu);
+        g_memories.push_back(this);
+        known = true;
+    }
     if (bytes >= BIG) return alloc_big(p, bytes);
     *p = nullptr;
     cudaError_t e = cudaSuccess;

@@ -168,7 +168,6 @@ class DeviceMemory {
   public:
     static constexpr size_t BIG = (size_t)32 << 20;
     static constexpr size_t KEEP_BYTES = (size_t)1792 << 20, KEEP_POOL_BYTES = (size_t)256 << 20;
-    DeviceMemory();
     ~DeviceMemory();
     // own: the context's own stream, on which the pool's blocks are handed out
     // and freed
@@ -185,6 +184,8 @@ class DeviceMemory {
         size_t bytes;
     };
     std::mutex mu;
+    bool known = false;  // to trim_all(): from the first block on, so that the
+                         // allocation-free call's context costs nothing
     cudaMemPool_t pool = nullptr;
     cudaStream_t stream = nullptr;
     std::list<Block> kept;  // oldest first
